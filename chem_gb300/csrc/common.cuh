@@ -21,7 +21,8 @@ struct GemmGroup {
   int lda, ldb, ldc;
   int flags;
 };
-enum : int { kTransB = 1, kLowerA = 2, kAccum = 4 };
+// kUpperC: only the outputs on and above the diagonal are needed.
+enum : int { kTransB = 1, kLowerA = 2, kAccum = 4, kUpperC = 8 };
 
 // One output tile of a group (64 rows x 64 or 16 columns), over the k range
 // [k0, k1); the tile is written at C + coff (split-K partial buffers).

@@ -150,7 +150,6 @@ struct gbjk_ctx {
   double *d_Linv = nullptr, *d_Vinv = nullptr;
   bool have_B = false, have_metric = false;
   bool fitted = false;  // the uploaded tensor already is L^-1 B (no metric)
-  bool colsum_smem_set = false;
   // J workspace
   double *d_P = nullptr, *d_Pg = nullptr, *d_part = nullptr, *d_g = nullptr, *d_h = nullptr,
          *d_y = nullptr, *d_J = nullptr, *d_jpart = nullptr;
@@ -337,9 +336,13 @@ gbjk_status fp64_plan(int nbf, int naux, int nocc, const gbjk_tunables& req, Fp6
   if (t == 0) {
     pl->elem_ht = (long long)nbf * naux * nocc <= kElemOutputs;
     pl->narrow = !pl->elem_ht && nocc <= kNarrowN;
-    // occupied widths just above a multiple of 32 (e.g. 81) pad less with
-    // 64 x 32 tiles than with 64 x 64 ones
-    const bool mid = !pl->elem_ht && !pl->narrow && cdiv(nocc, 32) * 32 < cdiv(nocc, 64) * 64;
+    // the kernel computes whole patches of TN/4 columns, so the width that
+    // pads nocc least wins; narrower tiles load A more often and have to save
+    // 5 % of the columns (C8H18 fit, nocc 33: 11.8 ms at 36 columns of 64 x 16
+    // tiles, 13.5 at 40 of 64 x 32, 15.3 at 48 of 64 x 64)
+    const auto pad = [&](int w) { return cdiv(nocc, w) * w; };
+    if (!pl->elem_ht && 100 * pad(4) <= 95 * std::min(pad(8), pad(16))) pl->narrow = true;
+    const bool mid = !pl->elem_ht && !pl->narrow && pad(8) < pad(16);
     pl->ht_tn = pl->elem_ht || pl->narrow ? 16 : (mid ? 32 : 64);
   } else {
     pl->elem_ht = t == 1;
@@ -356,8 +359,11 @@ gbjk_status fp64_plan(int nbf, int naux, int nocc, const gbjk_tunables& req, Fp6
   }
   pl->ks = ks;
   pl->kc = kc;
-  pl->elem_k = req.fp64_k_tile == 0 ? (long long)nbf * nbf * ks <= kElemOutputs
-                                    : req.fp64_k_tile == 1;
+  // the exchange in 16 x 16 tiles: they follow the diagonal and the matrix
+  // edge closest, and their staged operands keep the FP64 pipe as busy as 64 x
+  // 64 tiles do (exchange of C20H42: 39.6 ms against 48.1; nbf 800, naux 2400,
+  // nocc 120: 152.6 against 193.6; water, nbf 24: 10 us against 31)
+  pl->elem_k = req.fp64_k_tile != 64;
   return GBJK_OK;
 }
 
@@ -477,7 +483,7 @@ gbjk_status ensure_k_workspace(gbjk_ctx* ctx, int nocc) {
     g.lda = (int)kdim;
     g.ldb = (int)kdim;
     g.ldc = (int)nbf;
-    g.flags = kTransB;
+    g.flags = kTransB | kUpperC;
     ctx->syrk_group = (int)groups.size();
     groups.push_back(g);
     ctx->syrk_tile0 = (int)tiles.size();
@@ -594,7 +600,7 @@ gbjk_status ensure_k_batched(gbjk_ctx* ctx, int nocc) {
     g.lda = xbc * nocc;
     g.ldb = xbc * nocc;
     g.ldc = nbf;
-    g.flags = kTransB;
+    g.flags = kTransB | kUpperC;
     groups.push_back(g);  // group ng_ht + v
     const long long kd = (long long)xbc * nocc;
     const int kt = pl.elem_k ? 16 : 64;
@@ -730,7 +736,8 @@ gbjk_status ensure_k_occ_batched(gbjk_ctx* ctx, int nocc) {
                             obc, 0};
     }
     const int kd = naux * obc;
-    g[nblk + 2 * nbf] = {ob.d_H2, ob.d_H2, ob.d_Kpart, nbf, nbf, kd, kd, kd, nbf, kTransB};
+    g[nblk + 2 * nbf] = {ob.d_H2, ob.d_H2, ob.d_Kpart, nbf, nbf, kd, kd, kd, nbf,
+                         kTransB | kUpperC};
     // DF-LMO: K_nm = -sum Hfit[n] H[m]
     g[nblk + 2 * nbf + 1] = {ob.d_H2, ob.d_H, ob.d_Kpart, nbf, nbf, kd, kd, kd, nbf, kTransB};
   }
@@ -914,7 +921,7 @@ gbjk_status run_j(gbjk_ctx* ctx, const double* dP, double* dJ) {
   }
   {
     PhaseScope ps(ctx, PH_J_REDUCE);
-    k_reduce_rows<<<cdiv(naux, 128), 128, 0, ctx->stream>>>(ctx->d_part, nbf, naux, ctx->d_g);
+    k_reduce_rows<<<cdiv(naux, 32), 32, 0, ctx->stream>>>(ctx->d_part, nbf, naux, ctx->d_g);
     CKL(PH_J_REDUCE);
   }
   const double* hvec = ctx->d_h;
@@ -927,7 +934,7 @@ gbjk_status run_j(gbjk_ctx* ctx, const double* dP, double* dJ) {
       k_gemv<<<cdiv((long long)naux * 32, 256), 256, 0, ctx->stream>>>(ctx->d_Linv, ctx->d_g,
                                                                          naux, ctx->d_y);
       CKL(PH_J_METRIC);
-      k_gemv_lower_t<<<cdiv(naux, 128), 128, 0, ctx->stream>>>(ctx->d_Linv, ctx->d_y, naux,
+      k_gemv_lower_t<<<cdiv(naux, 32), 32, 0, ctx->stream>>>(ctx->d_Linv, ctx->d_y, naux,
                                                                ctx->d_h);
     } else {
       k_gemv<<<cdiv((long long)naux * 32, 256), 256, 0, ctx->stream>>>(ctx->d_Vinv, ctx->d_g,
@@ -937,13 +944,7 @@ gbjk_status run_j(gbjk_ctx* ctx, const double* dP, double* dJ) {
   }
   {
     PhaseScope ps(ctx, PH_J_COLSUM);
-    const size_t hbytes = (size_t)naux * sizeof(double);
-    if (hbytes > 48 * 1024 && !ctx->colsum_smem_set) {
-      CK(cudaFuncSetAttribute(k_j_colsum, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)hbytes));
-      ctx->colsum_smem_set = true;
-    }
-    k_j_colsum<<<dim3(cdiv(ctx->maxK, 128), nbf), 128, naux * sizeof(double), ctx->stream>>>(
+    k_j_colsum<<<dim3(cdiv(ctx->maxK, 32), nbf), 128, 0, ctx->stream>>>(
         ctx->d_B, ctx->d_panel_off, ctx->d_blk_of, ctx->d_boff, ctx->d_panelK, ctx->d_cmoff,
         ctx->d_colmap, hvec, nbf, naux, dJ);
     CKL(PH_J_COLSUM);
@@ -1654,7 +1655,6 @@ gbjk_status gbjk_autotune(gbjk_ctx* ctx, int kmethod, const double* P, const dou
       d1.push_back(t);
     }
     for (int kt : {1, 64}) {
-      if (kt == 1 && (long long)ctx->nbf * ctx->nbf * ctx->ksplit > big) continue;
       gbjk_tunables t{};
       t.fp64_k_tile = kt;
       d2.push_back(t);
@@ -2505,9 +2505,9 @@ extern "C" gbjk_status gbjk_compute_j_noalloc(const gbjk_desc* d, const int* d_c
   k_j_rowdot<<<cdiv((long long)nbf * naux * 32, 256), 256, 0, st>>>(d_B, poff, blk_of, boff,
                                                                      panelK, pgoff, Pg, nbf, naux,
                                                                      part);
-  k_reduce_rows<<<cdiv(naux, 128), 128, 0, st>>>(part, nbf, naux, g);
+  k_reduce_rows<<<cdiv(naux, 32), 32, 0, st>>>(part, nbf, naux, g);
   k_gemv<<<cdiv((long long)naux * 32, 256), 256, 0, st>>>(d_Vinv, g, naux, h);
-  k_j_colsum<<<dim3(cdiv(std::max(maxK, 1), 128), nbf), 128, naux * sizeof(double), st>>>(
+  k_j_colsum<<<dim3(cdiv(std::max(maxK, 1), 32), nbf), 128, 0, st>>>(
       d_B, poff, blk_of, boff, panelK, cmoff, d_colmap, h, nbf, naux, d_J);
   if (d->filter_eps > 0)
     k_block_filter<<<dim3(nblk, nblk), 128, 0, st>>>(d_J, nbf, boff, d->filter_eps);

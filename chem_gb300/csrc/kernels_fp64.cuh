@@ -59,13 +59,24 @@ __global__ void k_j_rowdot(const double* __restrict__ B, const long long* __rest
   if (lane == 0) part[(long long)mu * naux + X] = s;
 }
 
-// g[X] = sum_{mu} part[mu][X] (fixed order).
+// g[X] = sum_{mu} part[mu][X], in increasing mu.  One thread per X, so the
+// sum is a serial chain; what bounds it is the latency of its loads, hence
+// sixteen of them in flight and one-warp blocks that spread over the SMs.
 __global__ void k_reduce_rows(const double* __restrict__ part, int nrows, int ncols,
                               double* __restrict__ g) {
   const int X = blockIdx.x * blockDim.x + threadIdx.x;
   if (X >= ncols) return;
+  const double* p = part + X;
   double s = 0.0;
-  for (int r = 0; r < nrows; ++r) s += part[(long long)r * ncols + X];
+  int r = 0;
+  for (; r + 16 <= nrows; r += 16) {
+    double v[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = p[(long long)(r + j) * ncols];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) s += v[j];
+  }
+  for (; r < nrows; ++r) s += p[(long long)r * ncols];
   g[X] = s;
 }
 
@@ -118,56 +129,87 @@ __global__ void k_gemv(const double* __restrict__ M, const double* __restrict__ 
 }
 
 // y = L^T x for lower-triangular L (n x n row-major): y[X] = sum_{Y >= X}
-// L[Y][X] x[Y], one thread per X, in increasing Y.
+// L[Y][X] x[Y], one thread per X, in increasing Y.  A serial chain of up to n
+// fmas per thread, so its loads are what can be hidden: a warp walks the rows
+// from its first X on, sixteen rows' coalesced loads before their fmas, and a
+// thread skips the rows above its own.
 __global__ void k_gemv_lower_t(const double* __restrict__ L, const double* __restrict__ x, int n,
                                double* __restrict__ y) {
   const int X = blockIdx.x * blockDim.x + threadIdx.x;
-  if (X >= n) return;
+  const int Xc = min(X, n - 1);
   double s = 0.0;
-  for (int Y = X; Y < n; ++Y) s = fma(L[(long long)Y * n + X], x[Y], s);
-  y[X] = s;
+  int Y = X & ~31;
+  for (; Y + 16 <= n; Y += 16) {
+    double v[16], w[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      v[j] = L[(long long)(Y + j) * n + Xc];
+      w[j] = x[Y + j];
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (Y + j >= X) s = fma(v[j], w[j], s);
+  }
+  for (; Y < n; ++Y)
+    if (Y >= X) s = fma(L[(long long)Y * n + Xc], x[Y], s);
+  if (X < n) y[X] = s;
 }
 
-// J[mu][colmap[k]] = sum_X B_I[m][X][k] h[X]; grid (ceil(maxK/128), nbf).
-__global__ void k_j_colsum(const double* __restrict__ B, const long long* __restrict__ panel_off,
-                           const int* __restrict__ blk_of, const int* __restrict__ boff,
-                           const int* __restrict__ panel_K, const int* __restrict__ cmoff,
-                           const int* __restrict__ colmap, const double* __restrict__ h,
-                           int nbf, int naux, double* __restrict__ J) {
-  extern __shared__ double hs[];
-  for (int x = threadIdx.x; x < naux; x += blockDim.x) hs[x] = h[x];
-  __syncthreads();
+// J[mu][colmap[k]] = sum_X B_I[m][X][k] h[X]; grid (ceil(maxK/32), nbf),
+// block 128.  Each output is (s0 + s1) + (s2 + s3), s_a the in-order sum over
+// X = a mod 4 below 4 floor(naux / 4) and the last naux mod 4 terms in s0.
+// Warp a of a block forms s_a of 32 columns: four times the loads in flight
+// of one thread per output, which is what bounds small tensors.
+__global__ void __launch_bounds__(128)
+    k_j_colsum(const double* __restrict__ B, const long long* __restrict__ panel_off,
+               const int* __restrict__ blk_of, const int* __restrict__ boff,
+               const int* __restrict__ panel_K, const int* __restrict__ cmoff,
+               const int* __restrict__ colmap, const double* __restrict__ h, int nbf, int naux,
+               double* __restrict__ J) {
+  __shared__ double ps[4][32];
   const int mu = blockIdx.y;
   const int I = blk_of[mu];
   const int m = mu - boff[I];
   const int KI = panel_K[I];
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= KI) return;
-  const double* b = B + panel_off[I] + (long long)m * naux * KI + k;
-  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-  int X = 0;
-  // eight loads in flight per thread; accumulator X % 4, in X order
-  for (; X + 7 < naux; X += 8) {
-    double v[8];
+  if (blockIdx.x * 32 >= KI) return;
+  const int lane = threadIdx.x & 31, a = threadIdx.x >> 5;
+  const int k = blockIdx.x * 32 + lane;
+  double s = 0.0;
+  if (k < KI) {
+    const double* b = B + panel_off[I] + (long long)m * naux * KI + k;
+    const int n4 = naux & ~3;
+    int X = a;
+    for (; X + 28 < n4; X += 32) {
+      double v[8], w[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = __ldg(b + (long long)(X + j) * KI);
-    s0 = fma(v[0], hs[X], s0);
-    s1 = fma(v[1], hs[X + 1], s1);
-    s2 = fma(v[2], hs[X + 2], s2);
-    s3 = fma(v[3], hs[X + 3], s3);
-    s0 = fma(v[4], hs[X + 4], s0);
-    s1 = fma(v[5], hs[X + 5], s1);
-    s2 = fma(v[6], hs[X + 6], s2);
-    s3 = fma(v[7], hs[X + 7], s3);
+      for (int j = 0; j < 8; ++j) {
+        v[j] = __ldg(b + (long long)(X + 4 * j) * KI);
+        w[j] = __ldg(h + X + 4 * j);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s = fma(v[j], w[j], s);
+    }
+    {
+      // up to seven more, loaded together
+      double v[8], w[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const bool in = X + 4 * j < n4;
+        v[j] = in ? __ldg(b + (long long)(X + 4 * j) * KI) : 0.0;
+        w[j] = in ? __ldg(h + X + 4 * j) : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (X + 4 * j < n4) s = fma(v[j], w[j], s);
+    }
+    if (a == 0)
+      for (int Xt = n4; Xt < naux; ++Xt) s = fma(b[(long long)Xt * KI], h[Xt], s);
   }
-  for (; X + 3 < naux; X += 4) {
-    s0 = fma(b[(long long)X * KI], hs[X], s0);
-    s1 = fma(b[(long long)(X + 1) * KI], hs[X + 1], s1);
-    s2 = fma(b[(long long)(X + 2) * KI], hs[X + 2], s2);
-    s3 = fma(b[(long long)(X + 3) * KI], hs[X + 3], s3);
-  }
-  for (; X < naux; ++X) s0 = fma(b[(long long)X * KI], hs[X], s0);
-  J[(long long)mu * nbf + colmap[cmoff[I] + k]] = (s0 + s1) + (s2 + s3);
+  ps[a][lane] = s;
+  __syncthreads();
+  if (a == 0 && k < KI)
+    J[(long long)mu * nbf + colmap[cmoff[I] + k]] =
+        (ps[0][lane] + ps[1][lane]) + (ps[2][lane] + ps[3][lane]);
 }
 
 // x as hi + lo, two FP32 values built from the FP64 bit pattern with
@@ -374,6 +416,11 @@ __global__ void k_expand_panels(const double* __restrict__ P, const long long* _
 // 16 * TN / 4 threads, 4x4 outputs per thread.  Every output is one in-order
 // fma chain over its k range, whatever the tile shape.
 // TRANSA: A is stored K x M row-major, op(A)(m, k) = A[k * lda + m].
+// Bound by the FP64 pipe (about two fmas per clock and SM), so fmas of
+// outputs nobody reads are what it can save: thread (ty, tx) holds rows
+// ty + 16 r and columns tx + TN/4 c, and the 16 x TN/4 patches (r, c) that
+// lie outside the matrix, below the diagonal of an upper-triangle tile
+// (kUpperC) or beyond the diagonal of a lower-triangular A are skipped.
 template <bool TRANSB, bool TRANSA = false, int TN = 64>
 __global__ void __launch_bounds__(TN * 4)
     k_gemm_fp64(const GemmGroup* __restrict__ groups, const GemmTile* __restrict__ tiles,
@@ -390,6 +437,16 @@ __global__ void __launch_bounds__(TN * 4)
   const int m0 = t.mt * 64, n0 = t.nt * TN;
   int kend = t.k1;
   if ((g.flags & kLowerA) && kend > m0 + 64) kend = m0 + 64;  // A[m][k] = 0 for k > m
+  // active patches: bit 4 r + c
+  unsigned int act = 0;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const bool in = m0 + 16 * r < g.M && n0 + CW * c < g.N;
+      const bool below = (g.flags & kUpperC) && m0 + 16 * r > n0 + CW * c + CW - 1;
+      if (in && !below) act |= 1u << (4 * r + c);
+    }
   double acc[4][4];
 #pragma unroll
   for (int r = 0; r < 4; ++r)
@@ -423,17 +480,33 @@ __global__ void __launch_bounds__(TN * 4)
       }
     }
     __syncthreads();
+    // a lower-triangular A has no terms for the rows that end before k0
+    const unsigned int on =
+        (g.flags & kLowerA) && k0 >= m0 + 16 ? act & (0xFFFFu << (4 * ((k0 - m0) >> 4))) : act;
+    if (on == 0xFFFFu) {
 #pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      double a[4], b[4];
+      for (int kk = 0; kk < 16; ++kk) {
+        double a[4], b[4];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) a[r] = As[kk][ty + 16 * r];
+        for (int r = 0; r < 4; ++r) a[r] = As[kk][ty + 16 * r];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) b[c] = Bs[kk][tx + CW * c];
+        for (int c = 0; c < 4; ++c) b[c] = Bs[kk][tx + CW * c];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+      }
+    } else {
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+        for (int c = 0; c < 4; ++c) {
+          if (!((on >> (4 * r + c)) & 1)) continue;
+          double s = acc[r][c];
+#pragma unroll
+          for (int kk = 0; kk < 16; ++kk) s = fma(As[kk][ty + 16 * r], Bs[kk][tx + CW * c], s);
+          acc[r][c] = s;
+        }
     }
     __syncthreads();
   }
@@ -445,7 +518,7 @@ __global__ void __launch_bounds__(TN * 4)
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const int gn = n0 + tx + CW * c;
-      if (gn >= g.N) continue;
+      if (gn >= g.N || !((act >> (4 * r + c)) & 1)) continue;
       double v = alpha * acc[r][c];
       if (g.flags & kAccum) v += C[(long long)gm * g.ldc + gn];
       C[(long long)gm * g.ldc + gn] = v;
@@ -453,43 +526,89 @@ __global__ void __launch_bounds__(TN * 4)
   }
 }
 
-// Tiny problems: 16 x 16 tiles, one thread per output, each output the
-// in-order fma chain over the tile's k range read straight from global
-// memory.  A lower-triangular A stops at k = m: the terms beyond are exact
-// zeros, so every nonzero result equals the tiled kernel's bit for bit.
-// For problems so small that 64-row tiles would be mostly padding and the
-// few tiles would leave most SMs' FP64 units idle.
+// Small problems: 16 x 16 tiles, one thread per output, each output the
+// in-order fma chain over the tile's k range.  A lower-triangular A stops at
+// k = m: the terms beyond are exact zeros, so every nonzero result equals the
+// tiled kernel's bit for bit.  For problems so small that 64-row tiles would
+// be mostly padding and the few tiles would leave most SMs' FP64 units idle.
+// Bound by latency: 64 k of both operands are staged in shared memory at a
+// time, the next 64 in registers meanwhile, so the chain waits for memory
+// once per tile and not once per eight k.
 template <bool TRANSB>
 __global__ void __launch_bounds__(256)
     k_gemm_fp64_elem(const GemmGroup* __restrict__ groups, const GemmTile* __restrict__ tiles,
                      double alpha) {
+  constexpr int KC = 64;
+  __shared__ double As[16][KC + 1];
+  __shared__ double Bs[KC][17];
   const GemmTile t = tiles[blockIdx.x];
   const GemmGroup g = groups[t.group];
-  const int gm = t.mt * 16 + (threadIdx.x >> 4), gn = t.nt * 16 + (threadIdx.x & 15);
-  if (gm >= g.M || gn >= g.N) return;
-  int kend = t.k1;
-  if ((g.flags & kLowerA) && kend > gm + 1) kend = gm + 1;
-  const double* a = g.A + (long long)gm * g.lda;
-  const double* b = TRANSB ? g.B + (long long)gn * g.ldb : g.B + gn;
-  const long long bs = TRANSB ? 1 : g.ldb;
-  double acc = 0.0;
-  int k = t.k0;
-  // eight loads in flight, then their fmas in order
-  for (; k + 8 <= kend; k += 8) {
-    double av[8], bv[8];
+  const int tid = threadIdx.x;
+  const int ty = tid >> 4, tx = tid & 15;
+  const int m0 = t.mt * 16, n0 = t.nt * 16;
+  const int gm = m0 + ty, gn = n0 + tx;
+  int kblk = t.k1;  // end of the tile's k range, and of this row's
+  if ((g.flags & kLowerA) && kblk > m0 + 16) kblk = m0 + 16;
+  const int kend = (g.flags & kLowerA) ? min(kblk, gm + 1) : kblk;
+  double ra[4], rb[4];
+  auto fetch = [&](int k0) {
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      av[u] = a[k + u];
-      bv[u] = b[(long long)(k + u) * bs];
+    for (int j = 0; j < 4; ++j) {
+      const int idx = tid + 256 * j;
+      const int row = idx >> 6, ka = k0 + (idx & 63);
+      ra[j] = (m0 + row < g.M && ka < kblk) ? g.A[(long long)(m0 + row) * g.lda + ka] : 0.0;
+      if (TRANSB) {
+        rb[j] = (n0 + row < g.N && ka < kblk) ? g.B[(long long)(n0 + row) * g.ldb + ka] : 0.0;
+      } else {
+        const int kb = k0 + (idx >> 4), col = n0 + (idx & 15);
+        rb[j] = (col < g.N && kb < kblk) ? g.B[(long long)kb * g.ldb + col] : 0.0;
+      }
     }
+  };
+  double acc = 0.0;
+  fetch(t.k0);
+  for (int k0 = t.k0; k0 < kblk; k0 += KC) {
+    __syncthreads();  // the previous chunk's readers are done
 #pragma unroll
-    for (int u = 0; u < 8; ++u) acc = fma(av[u], bv[u], acc);
+    for (int j = 0; j < 4; ++j) {
+      const int idx = tid + 256 * j;
+      As[idx >> 6][idx & 63] = ra[j];
+      if (TRANSB)
+        Bs[idx & 63][idx >> 6] = rb[j];
+      else
+        Bs[idx >> 4][idx & 15] = rb[j];
+    }
+    __syncthreads();
+    if (k0 + KC < kblk) fetch(k0 + KC);
+    const int n = min(KC, kend - k0);
+    int k = 0;
+    for (; k + 8 <= n; k += 8)
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc = fma(As[ty][k + u], Bs[k + u][tx], acc);
+    for (; k < n; ++k) acc = fma(As[ty][k], Bs[k][tx], acc);
   }
-  for (; k < kend; ++k) acc = fma(a[k], b[(long long)k * bs], acc);
+  if (gm >= g.M || gn >= g.N) return;
   double* C = g.C + t.coff + (long long)gm * g.ldc + gn;
   double v = alpha * acc;
   if (g.flags & kAccum) v += *C;
   *C = v;
+}
+
+// Ordered sum of the split-K partials of one output, eight loads in flight
+// (one at a time, small matrices spend the whole launch on load latency).
+__device__ __forceinline__ double splitk_sum(const double* __restrict__ p, int nsplit,
+                                             long long stride) {
+  double s = 0.0;
+  int k = 0;
+  for (; k + 8 <= nsplit; k += 8) {
+    double v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = p[(long long)(k + j) * stride];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += v[j];
+  }
+  for (; k < nsplit; ++k) s += p[(long long)k * stride];
+  return s;
 }
 
 // out[m][n] = alpha * sum_s part[s][m][n] over the upper triangle (n >= m)
@@ -500,8 +619,7 @@ __global__ void k_splitk_reduce(const double* __restrict__ part, int nsplit, int
   if (idx >= (long long)n * n) return;
   const int m = (int)(idx / n), c = (int)(idx % n);
   if (symmetric && c < m) return;
-  double s = 0.0;
-  for (int k = 0; k < nsplit; ++k) s += part[(long long)k * n * n + idx];
+  double s = splitk_sum(part + idx, nsplit, (long long)n * n);
   s *= alpha;
   out[idx] = s;
   if (symmetric && c != m) out[(long long)c * n + m] = s;
@@ -580,8 +698,7 @@ __global__ void k_splitk_reduce_acc(const double* __restrict__ part, int nsplit,
   if (idx >= (long long)n * n) return;
   const int m = (int)(idx / n), c = (int)(idx % n);
   if (symmetric && c < m) return;
-  double s = 0.0;
-  for (int k = 0; k < nsplit; ++k) s += part[(long long)k * n * n + idx];
+  double s = splitk_sum(part + idx, nsplit, (long long)n * n);
   s *= alpha;
   if (accumulate) s += out[idx];
   out[idx] = s;

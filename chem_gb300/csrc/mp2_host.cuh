@@ -269,7 +269,7 @@ struct Mp2State {
       g.lda = (int)kw;
       g.ldb = (int)kw;
       g.ldc = naux;
-      g.flags = kTransB;
+      g.flags = kTransB | kUpperC;
       add((int)groups.size(), g.M, g.N, g.K, true);
       groups.push_back(g);
     }

@@ -191,9 +191,11 @@ struct ScfState {
   }
 
   static int cd(long long a, long long b) { return (int)((a + b - 1) / b); }
+  // 16 x 16 tiles: the nbf x nbf products are too small for 64 x 64 ones to
+  // reach every SM
   static void tiles_for(std::vector<GemmTile>& t, int g, int M, int N, int K) {
-    for (int mt = 0; mt < cd(M, 64); ++mt)
-      for (int nt = 0; nt < cd(N, 64); ++nt) t.push_back({g, mt, nt, 0, K, 0});
+    for (int mt = 0; mt < cd(M, 16); ++mt)
+      for (int nt = 0; nt < cd(N, 16); ++nt) t.push_back({g, mt, nt, 0, K, 0});
   }
 
   // buffers and GEMM plans; H, S, X: host nbf x nbf
@@ -260,9 +262,9 @@ struct ScfState {
 
   void gemm(cudaStream_t st, int t0, int nt, bool transB, double alpha) {
     if (transB)
-      k_gemm_fp64<true><<<nt, 256, 0, st>>>(dgroups, dtiles + t0, alpha);
+      k_gemm_fp64_elem<true><<<nt, 256, 0, st>>>(dgroups, dtiles + t0, alpha);
     else
-      k_gemm_fp64<false><<<nt, 256, 0, st>>>(dgroups, dtiles + t0, alpha);
+      k_gemm_fp64_elem<false><<<nt, 256, 0, st>>>(dgroups, dtiles + t0, alpha);
   }
   // the part of graph A before the Fock build
   int64_t launch_pre(cudaStream_t st) {

@@ -36,8 +36,8 @@ using namespace gbjk;
 // SMs the mixed-path exchange GEMM leaves to the concurrent J column sums
 // unless gbjk_set_overlap says otherwise: 0, the exchange takes every SM and
 // the J blocks fill the registers and shared memory its CTAs leave free
-// (C20H42: 2.051 against 2.077 ms per build in order; forking the J sums
-// only before the exchange: 2.125 ms).
+// (a build through the host call: C20H42 1.89 ms against 1.92 in order, C10H22
+// 0.403 against 0.422, five waters 0.164 against 0.182).
 constexpr int kDefaultOverlapSms = 0;
 
 enum Phase {
@@ -152,7 +152,7 @@ struct gbjk_ctx {
   bool fitted = false;  // the uploaded tensor already is L^-1 B (no metric)
   // J workspace
   double *d_P = nullptr, *d_Pg = nullptr, *d_part = nullptr, *d_g = nullptr, *d_h = nullptr,
-         *d_y = nullptr, *d_J = nullptr, *d_jpart = nullptr;
+         *d_y = nullptr, *d_J = nullptr;
   int jmode = GBJK_J_VINV;
   // K workspace (per nocc)
   int ws_nocc = -1;
@@ -296,11 +296,6 @@ void resolve_profile(gbjk_ctx* ctx) {
 }
 
 int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
-// auxiliary rows per block of the mixed-path J column sums
-// auxiliary rows per chunk of the mixed-path J column sums (one warp of 128
-// columns per block: more, shorter blocks keep the grid several waves deep)
-constexpr int kColsumChunk = 256;
-
 // Tiles of tm rows x tn columns: 64 x 64, 64 x 16 (narrow kernel) or
 // 16 x 16 (one thread per output).
 void add_tiles(std::vector<GemmTile>& tiles, int group, int M, int N, int k0, int k1,
@@ -863,9 +858,6 @@ gbjk_status ensure_j_workspace(gbjk_ctx* ctx) {
   if ((s = dalloc(ctx, &ctx->d_y, naux))) return s;
   if ((s = dalloc(ctx, &ctx->d_J, nbf * nbf))) return s;
   if ((s = dalloc(ctx, &ctx->d_K, nbf * nbf))) return s;
-  if ((s = dalloc(ctx, &ctx->d_jpart,
-                  (size_t)cdiv(naux, kColsumChunk) * nbf * std::max(1, ctx->maxK))))
-    return s;
   return GBJK_OK;
 }
 
@@ -1086,7 +1078,7 @@ gbjk_status gbjk_create(gbjk_ctx** out, const gbjk_desc* d) {
     return s;
   }
   ctx->split.init(ctx->nbf, ctx->naux, ctx->nblk, ctx->bsize, ctx->boff, ctx->panelK, ctx->cmoff,
-                  ctx->panel_off);
+                  ctx->panel_off, ctx->colmap, ctx->blk_of);
   ctx->split.set_dev_layout(ctx->d_panel_off, ctx->d_blk_of, ctx->d_boff, ctx->d_panelK);
   *out = ctx;
   return GBJK_OK;
@@ -1105,7 +1097,6 @@ void gbjk_destroy(gbjk_ctx* ctx) {
   void* ptrs[] = {ctx->d_blk_of, ctx->d_boff,  ctx->d_panelK, ctx->d_cmoff, ctx->d_colmap,
                   ctx->d_panel_off, ctx->d_pg_off, ctx->d_B, ctx->d_Linv, ctx->d_Vinv,
                   ctx->d_P, ctx->d_Pg, ctx->d_part, ctx->d_g, ctx->d_h, ctx->d_y, ctx->d_J,
-                  ctx->d_jpart,
                   ctx->d_C, ctx->d_Cg, ctx->d_H, ctx->d_H2, ctx->d_Kpart, ctx->d_K,
                   ctx->d_groups, ctx->d_tiles};
   for (void* p : ptrs)
@@ -1799,16 +1790,8 @@ static gbjk_status run_jk_split(gbjk_ctx* ctx, const double* dP, const double* d
     }
     {
       PhaseScope ps(ctx, PH_J_COLSUM);
-      // over the 6-byte compact copy of L^-1 B (one warp of 128 columns per block)
-      const int xchunk = kColsumChunk, nchunk = cdiv(naux, xchunk);
-      k_j_colsum_f32i16<<<dim3(cdiv(ctx->maxK, 128), nbf, nchunk), 32, xchunk * sizeof(float2),
-                          js>>>(ctx->split.d_Bhi, ctx->split.d_Blo, ctx->split.d_cpo, ctx->d_blk_of,
-                                ctx->d_boff, ctx->d_panelK, ctx->split.d_dt, nbf, naux, xchunk,
-                                ctx->maxK, ctx->d_jpart);
-      k_j_colsum_chunks<<<dim3(cdiv(ctx->maxK, 128), nbf), 128, 0, js>>>(
-          ctx->d_jpart, nchunk, nbf, ctx->maxK, ctx->d_blk_of, ctx->d_panelK, ctx->d_cmoff,
-          ctx->d_colmap, dJ);
-      ctx->launches++;
+      ctx->split.run_j_cols(js, ctx->split.d_dt, dJ, &ctx->launches);
+      ctx->launches--;  // CKL counts one
       CKL(PH_J_COLSUM);
     }
     if (ctx->eps > 0) {

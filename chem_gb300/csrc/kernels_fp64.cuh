@@ -10,6 +10,23 @@
 
 namespace gbjk {
 
+// Ordered sum of the split-K partials of one output, eight loads in flight
+// (one at a time, small matrices spend the whole launch on load latency).
+__device__ __forceinline__ double splitk_sum(const double* __restrict__ p, int nsplit,
+                                             long long stride) {
+  double s = 0.0;
+  int k = 0;
+  for (; k + 8 <= nsplit; k += 8) {
+    double v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = p[(long long)(k + j) * stride];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += v[j];
+  }
+  for (; k < nsplit; ++k) s += p[(long long)k * stride];
+  return s;
+}
+
 // Pg[pg_off[I] + m*K_I + k] = P[(boff[I]+m)*ld + colmap[cmoff[I]+k]]
 // grid: (ceil(maxK/128), nbf); block 128.
 __global__ void k_gather_panel_rows(const double* __restrict__ P, int ld,
@@ -242,27 +259,35 @@ __device__ __forceinline__ void f64_split_f32(double x, float& hi, float& lo) {
 // hi = its sign, exponent and top 24 significand bits (FP32; 0 outside the
 // FP32 normal range) and lo = the next 29 bits rounded to 16
 // (lo16 = min(rint(m29 / 2^13), 65535)), so x = hi + lo16 2^(E-1062) to
-// about 40 significant bits in 6 bytes.  The copy has its own layout: panel
-// I's rows (m, X) with a stride of KP_I = K_I rounded up to a multiple of 8
-// (zero padding), panels at cpanel_off[I], in two planes (hi FP32, lo16), so
-// that four consecutive columns are one 16-byte and one 8-byte load.
-// grid (naux, nbf), block 128.
+// about 40 significant bits in 6 bytes.  The copy holds the columns [k0, K_I)
+// of each panel: all of them, or, for a tensor whose two copies of every
+// off-diagonal block pair agree bit for bit, those of the blocks J >= I.
+// Panel I is [naux][cp]: row X holds the ncol = b_I (K_I - k0) values (m, k)
+// side by side, padded with zeros to a multiple of 8, in two planes (hi FP32,
+// lo16), so that four consecutive values are one 16-byte and one 8-byte load
+// and a warp's 128 values lie in one row whatever the block sizes are.
+struct JPanel {
+  long long off;   // first element in the two planes
+  long long gcol;  // first column among all panels' columns
+  int cp, ncol;    // row stride, columns
+  int k0;          // first panel column
+};
+// grid (naux, nblk), block 128.
 __global__ void k_encode_f32i16(const double* __restrict__ B, const long long* __restrict__ panel_off,
-                                const long long* __restrict__ cpanel_off,
-                                const int* __restrict__ blk_of, const int* __restrict__ boff,
-                                const int* __restrict__ panel_K, int naux, float* __restrict__ hi,
-                                uint16_t* __restrict__ lo) {
-  const int X = blockIdx.x, mu = blockIdx.y;
-  const int I = blk_of[mu];
-  const int m = mu - boff[I];
-  const int KI = panel_K[I], KP = (KI + 7) & ~7;
-  const double* src = B + panel_off[I] + ((long long)m * naux + X) * KI;
-  const long long d = cpanel_off[I] + ((long long)m * naux + X) * KP;
-  for (int k = threadIdx.x; k < KP; k += blockDim.x) {
+                                const JPanel* __restrict__ jp, const int* __restrict__ panel_K,
+                                int naux, float* __restrict__ hi, uint16_t* __restrict__ lo) {
+  const int X = blockIdx.x, I = blockIdx.y;
+  const JPanel p = jp[I];
+  const int KI = panel_K[I], ks = KI - p.k0;
+  const double* src = B + panel_off[I] + (long long)X * KI + p.k0;
+  const long long d = p.off + (long long)X * p.cp;
+  for (int c = threadIdx.x; c < p.cp; c += blockDim.x) {
     float h = 0.f;
     unsigned int l = 0;
-    if (k < KI) {
-      const unsigned long long u = (unsigned long long)__double_as_longlong(src[k]);
+    if (c < p.ncol) {
+      const int m = c / ks, k = c - m * ks;
+      const unsigned long long u =
+          (unsigned long long)__double_as_longlong(src[(long long)m * naux * KI + k]);
       const int E = (int)((u >> 52) & 0x7FF);
       const unsigned int sgn = (unsigned int)(u >> 32) & 0x80000000u;
       const int ef = E - 896;
@@ -271,9 +296,33 @@ __global__ void k_encode_f32i16(const double* __restrict__ B, const long long* _
         l = min(((unsigned int)(u & 0x1FFFFFFFu) + 4096u) >> 13, 65535u);
       }
     }
-    hi[d + k] = h;
-    lo[d + k] = (uint16_t)l;
+    hi[d + c] = h;
+    lo[d + c] = (uint16_t)l;
   }
+}
+
+// Whether the two copies of every off-diagonal block pair (I, J), I < J, hold
+// the same bits: (m, X, kIJ + n) of panel I and (n, X, kJI + m) of panel J.
+// A difference sets *flag.  grid (npairs, ceil(naux / 64)), block 128.
+struct SymPair {
+  long long offI, offJ;
+  int KI, KJ, kIJ, kJI, bI, bJ;
+};
+__global__ void k_check_symmetric(const double* __restrict__ B, const SymPair* __restrict__ pairs,
+                                  int naux, int* __restrict__ flag) {
+  const SymPair p = pairs[blockIdx.x];
+  const int x0 = blockIdx.y * 64, x1 = min(naux, x0 + 64);
+  const int nn = p.bI * p.bJ;
+  bool differ = false;
+  for (int e = threadIdx.x; e < nn; e += blockDim.x) {
+    const int m = e / p.bJ, n = e - m * p.bJ;
+    const double* a = B + p.offI + (long long)m * naux * p.KI + p.kIJ + n;
+    const double* b = B + p.offJ + (long long)n * naux * p.KJ + p.kJI + m;
+    for (int X = x0; X < x1; ++X)
+      differ |= __double_as_longlong(a[(long long)X * p.KI]) !=
+                __double_as_longlong(b[(long long)X * p.KJ]);
+  }
+  if (differ) *flag = 1;
 }
 
 // The pair (hi, lo) of a compact element as FP32 values: lo = lo16 *
@@ -285,25 +334,24 @@ __device__ __forceinline__ float f32i16_lo(float hi, unsigned int lo16) {
   return es >= 1 ? sc * (float)lo16 : 0.f;
 }
 
-// Mixed-path J columns: J[mu][colmap[k]] = sum_X B_I[m][X][k] h[X] over
-// the compact copy (6 bytes per element), with the products and the sum in
+// Mixed-path J columns: J_c = sum_X B[X][c] h[X] over the columns c of the
+// compact copy (6 bytes per element), with the products and the sum in
 // FP32 pairs (hi/lo operands, exact product error by fma, TwoSum
 // accumulation), so no FP64 arithmetic runs in the loop and the pass is
 // bound by HBM rather than by GB300's FP64 rate.  The auxiliary range is cut
-// into chunks of xchunk rows (blockIdx.z) so that the grid is several waves
-// deep; chunk z writes its partial column sums to
-// part[(z * nbf + mu) * maxK + k] and k_j_colsum_chunks adds the chunks in
-// order.  Thread t of block (bx, mu, z) sums columns k = 4 (blockDim bx + t)
-// .. +3.  grid (ceil(maxK/(4 blockDim)), nbf, nchunk), dynamic smem xchunk
-// float2.
-__global__ void k_j_colsum_f32i16(const float* __restrict__ Bhi, const uint16_t* __restrict__ Blo,
-                                  const long long* __restrict__ cpanel_off,
-                                  const int* __restrict__ blk_of, const int* __restrict__ boff,
-                                  const int* __restrict__ panel_K, const double* __restrict__ h,
-                                  int nbf, int naux, int xchunk, int maxK,
-                                  double* __restrict__ part) {
+// into chunks of xchunk rows (blockIdx.y); chunk z writes its partial column
+// sums to part[z * ncols + column] and k_j_colsum_chunks adds the chunks in
+// order.  Block x takes the 128 columns from blk[x].y of panel blk[x].x, lane
+// t the columns 4 t .. 4 t + 3.  C20H42: 0.188 ms, 6.0 TB/s, for the upper
+// triangle (0.437 ms over the whole tensor in rows of one AO function).
+// grid (nblkcol, nchunk), block 32, dynamic smem xchunk float2.
+__global__ void __launch_bounds__(32)
+    k_j_colsum_f32i16(const float* __restrict__ Bhi, const uint16_t* __restrict__ Blo,
+                      const JPanel* __restrict__ jp, const int2* __restrict__ blk,
+                      const double* __restrict__ h, int naux, int xchunk, long long ncols,
+                      double* __restrict__ part) {
   extern __shared__ float2 h2[];
-  const int x0 = blockIdx.z * xchunk;
+  const int x0 = blockIdx.y * xchunk;
   const int nx = min(xchunk, naux - x0);
   for (int x = threadIdx.x; x < nx; x += blockDim.x) {
     float a, b;
@@ -311,16 +359,14 @@ __global__ void k_j_colsum_f32i16(const float* __restrict__ Bhi, const uint16_t*
     h2[x] = make_float2(a, b);
   }
   __syncthreads();
-  const int mu = blockIdx.y;
-  const int I = blk_of[mu];
-  const int m = mu - boff[I];
-  const int KI = panel_K[I], KP = (KI + 7) & ~7;
-  const int k0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-  if (k0 >= KI) return;
-  const long long off = cpanel_off[I] + ((long long)m * naux + x0) * KP + k0;
+  const int2 bk = blk[blockIdx.x];
+  const JPanel p = jp[bk.x];
+  const int k0 = bk.y + 4 * threadIdx.x;
+  if (k0 >= p.cp) return;
+  const long long off = p.off + (long long)x0 * p.cp + k0;
   const float4* bh = reinterpret_cast<const float4*>(Bhi + off);
   const uint2* bl = reinterpret_cast<const uint2*>(Blo + off);
-  const int st4 = KP / 4;  // row stride in float4 / uint2 units
+  const int st4 = p.cp / 4;  // row stride in float4 / uint2 units
   float sh[4] = {0.f, 0.f, 0.f, 0.f}, sl[4] = {0.f, 0.f, 0.f, 0.f}, se[4] = {0.f, 0.f, 0.f, 0.f};
   auto acc = [](float b_h, float b_l, float2 hh, float& s_h, float& s_l, float& s_e) {
     const float p = __fmul_rn(b_h, hh.x);
@@ -373,25 +419,26 @@ __global__ void k_j_colsum_f32i16(const float* __restrict__ Bhi, const uint16_t*
     X += 8;
   }
   for (; X < nx; ++X) row(__ldg(bh + (long long)X * st4), __ldg(bl + (long long)X * st4), h2[X]);
-  double* out = part + ((long long)blockIdx.z * nbf + mu) * maxK + k0;
+  double v[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if (k0 + j < KI) out[j] = (double)sh[j] + ((double)sl[j] + (double)se[j]);
+  for (int j = 0; j < 4; ++j) v[j] = (double)sh[j] + ((double)sl[j] + (double)se[j]);
+  double2* out = reinterpret_cast<double2*>(part + (long long)blockIdx.y * ncols + p.gcol + k0);
+  out[0] = make_double2(v[0], v[1]);
+  out[1] = make_double2(v[2], v[3]);
 }
 
-// J[mu][colmap(k)] = sum over chunks (in order) of part[z][mu][k].
-// grid (ceil(maxK/128), nbf).
-__global__ void k_j_colsum_chunks(const double* __restrict__ part, int nchunk, int nbf, int maxK,
-                                  const int* __restrict__ blk_of, const int* __restrict__ panel_K,
-                                  const int* __restrict__ cmoff, const int* __restrict__ colmap,
-                                  double* __restrict__ J) {
-  const int mu = blockIdx.y;
-  const int I = blk_of[mu];
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= panel_K[I]) return;
-  double s = 0.0;
-  for (int z = 0; z < nchunk; ++z) s += part[((long long)z * nbf + mu) * maxK + k];
-  J[(long long)mu * nbf + colmap[cmoff[I] + k]] = s;
+// J[mu][nu] = sum over chunks (in order) of part[z][c], (mu, nu) = map[c];
+// nu < 0: nu = ~nu and the column stands for (nu, mu) too.  mu < 0: padding.
+__global__ void k_j_colsum_chunks(const double* __restrict__ part, int nchunk, long long ncols,
+                                  int nbf, const int2* __restrict__ map, double* __restrict__ J) {
+  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= ncols) return;
+  const int2 mn = map[c];
+  if (mn.x < 0) return;
+  const double s = splitk_sum(part + c, nchunk, ncols);
+  const int nu = mn.y < 0 ? ~mn.y : mn.y;
+  J[(long long)mn.x * nbf + nu] = s;
+  if (mn.y < 0) J[(long long)nu * nbf + mn.x] = s;
 }
 
 // Dense expansion of the panel array: D[mu][X][colmap(k)] = P_I[m][X][k]
@@ -592,23 +639,6 @@ __global__ void __launch_bounds__(256)
   double v = alpha * acc;
   if (g.flags & kAccum) v += *C;
   *C = v;
-}
-
-// Ordered sum of the split-K partials of one output, eight loads in flight
-// (one at a time, small matrices spend the whole launch on load latency).
-__device__ __forceinline__ double splitk_sum(const double* __restrict__ p, int nsplit,
-                                             long long stride) {
-  double s = 0.0;
-  int k = 0;
-  for (; k + 8 <= nsplit; k += 8) {
-    double v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = p[(long long)(k + j) * stride];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) s += v[j];
-  }
-  for (; k < nsplit; ++k) s += p[(long long)k * stride];
-  return s;
 }
 
 // out[m][n] = alpha * sum_s part[s][m][n] over the upper triangle (n >= m)

@@ -20,6 +20,7 @@
 #pragma once
 #include <algorithm>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "kernels_fp64.cuh"
@@ -41,11 +42,16 @@ struct SplitState {
   bool bfit_owned = false;
   double* Bfit = nullptr;
   // compact copy of Bfit for the mixed-path J (k_encode_f32i16: FP32 hi and
-  // a 16-bit remainder per element, 6 bytes; rows padded to a multiple of 8,
-  // panels at d_cpo[I]), unbatched only
+  // a 16-bit remainder per element, 6 bytes), unbatched only; with jsym the
+  // upper block triangle alone
   float* d_Bhi = nullptr;
   uint16_t* d_Blo = nullptr;
-  long long* d_cpo = nullptr;
+  JPanel* d_jp = nullptr;
+  int2 *d_jblk = nullptr, *d_jmap = nullptr;
+  double* d_jpart = nullptr;
+  int n_jblk = 0, jchunk = 0, jnchunk = 0;
+  long long jcols = 0;
+  std::vector<int> colmap, blk_of;
   // the context's device copies of the panel layout (not owned)
   const long long* dd_panel_off = nullptr;
   const int *dd_blk_of = nullptr, *dd_boff = nullptr, *dd_panelK = nullptr;
@@ -113,7 +119,8 @@ struct SplitState {
   }
   void init(int nbf_, int naux_, int nblk_, const std::vector<int>& bs,
             const std::vector<int>& bo, const std::vector<int>& pk, const std::vector<int>& cmo,
-            const std::vector<long long>& po) {
+            const std::vector<long long>& po, const std::vector<int>& cm,
+            const std::vector<int>& blko) {
     nbf = nbf_;
     naux = naux_;
     nblk = nblk_;
@@ -122,6 +129,8 @@ struct SplitState {
     panelK = pk;
     cmoff = cmo;
     panel_off = po;
+    colmap = cm;
+    blk_of = blko;
   }
   template <class T>
   cudaError_t alloc(T** p, size_t n) {
@@ -163,7 +172,10 @@ struct SplitState {
     bfit_owned = false;
     free_(&d_Bhi);
     free_(&d_Blo);
-    free_(&d_cpo);
+    free_(&d_jp);
+    free_(&d_jblk);
+    free_(&d_jmap);
+    free_(&d_jpart);
     free_(&d_Aslices);
     free_(&d_bjobs);
     free_(&d_eA);
@@ -263,6 +275,129 @@ struct SplitState {
     return launch_gemm_v<false, false>(st, items, n, launches, err, leave_sms);
   }
 
+  // --- once per tensor: the compact copy the mixed-path J reads ------------
+  // Block pairs (I, J), I < J, whose columns lie side by side in both panels,
+  // and k0[I], the first column of a block J >= I.  False if a panel's columns
+  // are not whole blocks in ascending order or a pair is kept on one side only.
+  bool symmetric_pattern(std::vector<SymPair>* pairs, std::vector<int>* k0) const {
+    std::vector<std::vector<std::pair<int, int>>> cols(nblk);  // (J, first column)
+    for (int I = 0; I < nblk; ++I) {
+      (*k0)[I] = panelK[I];
+      const int* cm = colmap.data() + cmoff[I];
+      for (int k = 0; k < panelK[I];) {
+        const int J = blk_of[cm[k]];
+        if (cm[k] != boff[J] || k + bsize[J] > panelK[I]) return false;
+        for (int n = 1; n < bsize[J]; ++n)
+          if (cm[k + n] != boff[J] + n) return false;
+        if (!cols[I].empty() && cols[I].back().first >= J) return false;
+        if (J >= I) (*k0)[I] = std::min((*k0)[I], k);
+        cols[I].push_back({J, k});
+        k += bsize[J];
+      }
+    }
+    size_t lower = 0;
+    for (int I = 0; I < nblk; ++I)
+      for (const auto& c : cols[I]) {
+        const int J = c.first;
+        if (J < I) lower++;
+        if (J <= I) continue;
+        auto it = std::lower_bound(cols[J].begin(), cols[J].end(), std::make_pair(I, -1));
+        if (it == cols[J].end() || it->first != I) return false;
+        pairs->push_back({panel_off[I], panel_off[J], panelK[I], panelK[J], c.second, it->second,
+                          bsize[I], bsize[J]});
+      }
+    return lower == pairs->size();
+  }
+
+  gbjk_status prepare_j(cudaStream_t st, int64_t* launches, std::string* err) {
+    auto oom = [&]() {
+      *err = "split path: out of memory for the compact J tensor";
+      return GBJK_OOM;
+    };
+    // J is symmetric where the tensor is: a tensor that holds the same bits
+    // in both copies of every off-diagonal block pair (as the integral engines
+    // write it) is read in its upper block triangle only, and J mirrored
+    std::vector<SymPair> pairs;
+    std::vector<int> k0(nblk, 0);
+    bool sym = symmetric_pattern(&pairs, &k0);
+    if (sym && !pairs.empty()) {
+      SymPair* dp = nullptr;
+      int* df = nullptr;
+      int h = 0;
+      if (alloc(&dp, pairs.size()) != cudaSuccess || alloc(&df, 1) != cudaSuccess) {
+        free_(&dp);
+        return oom();
+      }
+      cudaMemcpy(dp, pairs.data(), pairs.size() * sizeof(SymPair), cudaMemcpyHostToDevice);
+      cudaMemsetAsync(df, 0, sizeof(int), st);
+      {
+        Scope sc(this, 3, st);
+        k_check_symmetric<<<dim3((unsigned)pairs.size(), cdiv_(naux, 64)), 128, 0, st>>>(
+            Bfit, dp, naux, df);
+        (*launches)++;
+      }
+      cudaMemcpyAsync(&h, df, sizeof(int), cudaMemcpyDeviceToHost, st);
+      const cudaError_t e = cudaStreamSynchronize(st);
+      bytes -= pairs.size() * sizeof(SymPair) + sizeof(int);
+      free_(&dp);
+      free_(&df);
+      if (e != cudaSuccess) {
+        *err = std::string("split path preparation: ") + cudaGetErrorString(e);
+        return GBJK_CUDA_ERROR;
+      }
+      sym = h == 0;
+    }
+    if (!sym) std::fill(k0.begin(), k0.end(), 0);
+    std::vector<JPanel> jp(nblk);
+    std::vector<int2> blk, map;
+    long long ncomp = 0;
+    for (int I = 0; I < nblk; ++I) {
+      const int ks = panelK[I] - k0[I], ncol = bsize[I] * ks, cp = (ncol + 7) & ~7;
+      jp[I] = {ncomp, (long long)map.size(), cp, ncol, k0[I]};
+      for (int c0 = 0; c0 < ncol; c0 += 128) blk.push_back(make_int2(I, c0));
+      for (int c = 0; c < cp; ++c) {
+        if (c >= ncol) {
+          map.push_back(make_int2(-1, 0));
+          continue;
+        }
+        const int m = c / ks, nu = colmap[cmoff[I] + k0[I] + c % ks];
+        map.push_back(make_int2(boff[I] + m, sym && blk_of[nu] != I ? ~nu : nu));
+      }
+      ncomp += (long long)naux * cp;
+    }
+    jcols = (long long)map.size();
+    n_jblk = (int)blk.size();
+    // rows per block: 128, or fewer while the blocks would not fill the SMs
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    jchunk = 128;
+    while (jchunk > 32 && (long long)n_jblk * cdiv_(naux, jchunk) < 16LL * nsm) jchunk /= 2;
+    jnchunk = cdiv_(naux, jchunk);
+    if (alloc(&d_Bhi, (size_t)ncomp) != cudaSuccess || alloc(&d_Blo, (size_t)ncomp) != cudaSuccess ||
+        alloc(&d_jp, jp.size()) != cudaSuccess || alloc(&d_jblk, blk.size()) != cudaSuccess ||
+        alloc(&d_jmap, map.size()) != cudaSuccess ||
+        alloc(&d_jpart, (size_t)jnchunk * jcols) != cudaSuccess ||
+        cudaMemcpy(d_jp, jp.data(), jp.size() * sizeof(JPanel), cudaMemcpyHostToDevice) ||
+        cudaMemcpy(d_jblk, blk.data(), blk.size() * sizeof(int2), cudaMemcpyHostToDevice) ||
+        cudaMemcpy(d_jmap, map.data(), map.size() * sizeof(int2), cudaMemcpyHostToDevice))
+      return oom();
+    Scope sc(this, 3, st);
+    k_encode_f32i16<<<dim3(naux, nblk), 128, 0, st>>>(Bfit, dd_panel_off, d_jp, dd_panelK, naux,
+                                                      d_Bhi, d_Blo);
+    (*launches)++;
+    return GBJK_OK;
+  }
+
+  // J = (L^-1 B)^T d from the compact copy into dJ (screened blocks untouched)
+  void run_j_cols(cudaStream_t st, const double* d, double* dJ, int64_t* launches) {
+    if (n_jblk == 0) return;
+    k_j_colsum_f32i16<<<dim3(n_jblk, jnchunk), 32, jchunk * sizeof(float2), st>>>(
+        d_Bhi, d_Blo, d_jp, d_jblk, d, naux, jchunk, jcols, d_jpart);
+    k_j_colsum_chunks<<<cdiv_(jcols, 128), 128, 0, st>>>(d_jpart, jnchunk, jcols, nbf, d_jmap, dJ);
+    *launches += 2;
+  }
+
   // --- once per tensor: prefit and A-operand digits -----------------------
   gbjk_status prepare_b(cudaStream_t st, const double* d_B, const double* d_Linv,
                         int64_t* launches, std::string* err) {
@@ -337,24 +472,8 @@ struct SplitState {
     }
     Bfit = d_Bfit;
     if (nbatch == 1) {
-      // the mixed-mode J reads L^-1 B once per build: a 6-byte copy
-      std::vector<long long> cpo(nblk);
-      long long ncomp = 0;
-      for (int I = 0; I < nblk; ++I) {
-        cpo[I] = ncomp;
-        ncomp += (long long)bsize[I] * naux * ((panelK[I] + 7) & ~7);
-      }
-      if (alloc(&d_Bhi, (size_t)ncomp) != cudaSuccess ||
-          alloc(&d_Blo, (size_t)ncomp) != cudaSuccess || alloc(&d_cpo, (size_t)nblk) != cudaSuccess ||
-          cudaMemcpy(d_cpo, cpo.data(), nblk * sizeof(long long), cudaMemcpyHostToDevice) !=
-              cudaSuccess) {
-        *err = "split path: out of memory for the compact J tensor";
-        return GBJK_OOM;
-      }
-      Scope sc(this, 3, st);
-      k_encode_f32i16<<<dim3(naux, nbf), 128, 0, st>>>(d_Bfit, dd_panel_off, d_cpo, dd_blk_of,
-                                                      dd_boff, dd_panelK, naux, d_Bhi, d_Blo);
-      (*launches)++;
+      gbjk_status js = prepare_j(st, launches, err);
+      if (js) return js;
     }
     // A operands: rows (m, y) of panel I, y < xb (all auxiliary rows when
     // not batched), at m * pad32(batch) + y; columns k

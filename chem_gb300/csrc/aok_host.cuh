@@ -32,8 +32,11 @@ struct AoKState {
   size_t bytes = 0;
   int precision = -1;
   bool ready = false;
-  long long kdim = 0;  // naux * nbf
+  long long kdim = 0;  // k of the exchange: naux * nbf (split path: padded)
   double *d_Pg = nullptr, *d_cbar = nullptr, *d_cd = nullptr, *d_Kpart = nullptr;
+  long long* d_cbi = nullptr;  // split: integers of L^-1 cbar (SplitItem::iout)
+  long long* d_eoff = nullptr;
+  std::vector<SplitIntJob> cjob;
   // FP64 plan
   GemmGroup* d_groups = nullptr;
   GemmTile* d_tiles = nullptr;
@@ -41,10 +44,10 @@ struct AoKState {
   // split plan
   uint16_t *d_Pdig = nullptr, *d_Cbdig = nullptr, *d_Bdig = nullptr;
   int *d_eP = nullptr, *d_eBd = nullptr;
-  unsigned int* d_eCb = nullptr;
+  int* d_eCb = nullptr;
   SplitItem* d_items = nullptr;
   SplitJob* d_jobs = nullptr;
-  int i_ht0 = 0, i_htn = 0, i_k0 = 0, i_kn = 0, j_p0 = 0, j_cb = 0;
+  int i_ht0 = 0, i_htn = 0, i_k0 = 0, i_kn = 0, j_p0 = 0;
   int p_nrb = 0, r_nrb = 0, r_nkt = 0, p_maxthr = 0;
 
   template <class T>
@@ -67,6 +70,8 @@ struct AoKState {
     free_(&d_cbar);
     free_(&d_cd);
     free_(&d_Kpart);
+    free_(&d_cbi);
+    free_(&d_eoff);
     free_(&d_groups);
     free_(&d_tiles);
     free_(&d_Pdig);
@@ -228,8 +233,11 @@ struct AoKState {
       return GBJK_INVALID_ARG;
     }
     const int nbf = L.nbf, naux = L.naux, nblk = L.nblk;
-    kdim = (long long)naux * nbf;
-    const size_t big = (size_t)nbf * naux * nbf;
+    // rows of L^-1 cbar and of the dense Bfit in the column-pair-outermost
+    // order of the half transform's integer output
+    const int ld = nbf + (nbf & 1), npad = SplitState::pad32(naux);
+    kdim = (long long)npad * ld;
+    const size_t big = (size_t)nbf * kdim;
     p_nrb = cdiv_(nbf, kTileN) * (kTileN / 32);
     std::vector<long long> p_off(nblk);
     long long ptot = 0;
@@ -250,7 +258,8 @@ struct AoKState {
     const int ks = sp.choose_ksplit(r_nkt, ntile);
     const int kt_per = cdiv_(r_nkt, ks);
     ksplit = cdiv_(r_nkt, kt_per);
-    if (alloc(&d_Pg, (size_t)L.ncols_total * nbf) || alloc(&d_cbar, big) ||
+    if (alloc(&d_Pg, (size_t)L.ncols_total * nbf) || alloc(&d_cbi, big) ||
+        alloc(&d_eoff, (size_t)2 * nbf) ||
         alloc(&d_Kpart, (size_t)ksplit * nbf * nbf) || alloc(&d_Pdig, (size_t)ptot) ||
         alloc(&d_Cbdig, (size_t)rdig) || alloc(&d_Bdig, (size_t)rdig) ||
         alloc(&d_eP, (size_t)nblk * p_nrb * 32) || alloc(&d_eBd, (size_t)r_nrb * 32) ||
@@ -259,13 +268,12 @@ struct AoKState {
         cudaMemsetAsync(d_Cbdig, 0, (size_t)rdig * 2, st) ||
         cudaMemsetAsync(d_Bdig, 0, (size_t)rdig * 2, st) ||
         cudaMemsetAsync(d_eP, 0, (size_t)nblk * p_nrb * 32 * 4, st) ||
-        cudaMemsetAsync(d_eBd, 0, (size_t)r_nrb * 32 * 4, st) ||
-        cudaMemsetAsync(d_eCb, 0, (size_t)r_nrb * 32 * 4, st)) {
+        cudaMemsetAsync(d_eBd, 0, (size_t)r_nrb * 32 * 4, st)) {
       *err = "DF-AO K: out of device memory for the split path";
       return GBJK_OOM;
     }
-    // jobs: P rows per panel, the half-transformed rows M, and (once) the
-    // dense Bfit rows N
+    // jobs: P rows per panel, and (once) the dense Bfit rows N; the digits of
+    // the half-transformed rows M are cut from their integers
     std::vector<SplitJob> jobs;
     j_p0 = 0;
     p_maxthr = 0;
@@ -278,36 +286,51 @@ struct AoKState {
       j.nrows = nbf;
       j.ncols = (*L.panelK)[I];
       j.e = d_eP + (long long)I * p_nrb * 32;
-      j.e_biased = 0;
       j.nrb = p_nrb;
       j.nkt = sp.nkt[I];
       j.dst = d_Pdig + p_off[I];
       jobs.push_back(j);
       p_maxthr = std::max(p_maxthr, (nbf / 8 + 2) * sp.nkt[I] * 32);
     }
-    j_cb = (int)jobs.size();
+    const int j_bd = (int)jobs.size();
     {
       SplitJob j;
-      j.src = d_cbar;
+      j.src = (const double*)d_cbi;  // the dense Bfit is staged there once
       j.rs = kdim;
       j.cs = 1;
       j.row0 = 0;
       j.nrows = nbf;
       j.ncols = kdim;
-      j.e = (int*)d_eCb;
-      j.e_biased = 0;
+      j.e = d_eBd;
+      j.nrb = r_nrb;
+      j.nkt = r_nkt;
+      j.dst = d_Bdig;
+      jobs.push_back(j);
+    }
+    std::vector<long long> eoff((size_t)2 * nbf);
+    for (int I = 0; I < nblk; ++I)
+      for (int m = 0; m < (*L.bsize)[I]; ++m) {
+        eoff[(*L.boff)[I] + m] = sp.eA_off[I] + (long long)m * sp.apitch;
+        eoff[(size_t)nbf + (*L.boff)[I] + m] = (long long)I * p_nrb * 32;
+      }
+    {
+      SplitIntJob j;
+      j.src = d_cbi;
+      j.rs = kdim;
+      j.ncols = kdim;
+      j.gs = 32LL * ld;
+      j.nrows = nbf;
+      j.ny = npad;
+      j.ld = ld;
+      j.e = d_eCb;
+      j.ea = sp.d_eA;
+      j.ea_off = d_eoff;
+      j.eb = d_eP;
+      j.eb_off = d_eoff + nbf;
       j.nrb = r_nrb;
       j.nkt = r_nkt;
       j.dst = d_Cbdig;
-      jobs.push_back(j);
-    }
-    const int j_bd = (int)jobs.size();
-    {
-      SplitJob j = jobs[j_cb];
-      j.src = d_cbar;  // the dense Bfit is staged in the cbar buffer once
-      j.e = d_eBd;
-      j.dst = d_Bdig;
-      jobs.push_back(j);
+      cjob.assign(1, j);
     }
     // items
     std::vector<SplitItem> items;
@@ -316,6 +339,7 @@ struct AoKState {
       w.emax = nullptr;
       w.emax_row0 = 0;
       w.emax_div = 1;
+      w.out = nullptr;
       w.out2 = nullptr;
       w.c0 = 0;
       w.ncol1 = 1 << 30;
@@ -341,9 +365,11 @@ struct AoKState {
           w.nkt = sp.nkt[I];
           w.ea = sp.d_eA + sp.eA_off[I] + (long long)mt * kTileM;
           w.eb = d_eP + (long long)I * p_nrb * 32 + (long long)nt * kTileN;
-          w.out = d_cbar + ((long long)(*L.boff)[I] * naux + (long long)mt * kTileM) * nbf +
-                  (long long)nt * kTileN;
-          w.ldr = nbf;
+          w.iout = d_cbi + (long long)(*L.boff)[I] * kdim;
+          w.ldr = ld;
+          w.perm_rs = kdim;
+          w.perm_div = naux;
+          w.c0 = nt * kTileN;
           w.m_valid = (int)std::min<long long>(kTileM, rows - (long long)mt * kTileM);
           w.n_valid = std::min(kTileN, nbf - nt * kTileN);
           // row (m, Y) of panel I is row M = boff[I] + m of cbar
@@ -368,7 +394,7 @@ struct AoKState {
           w.b_rb0 = c0 / 32;
           w.kt0 = kt0;
           w.nkt = n_kt;
-          w.ea = (const int*)d_eCb + r0;
+          w.ea = d_eCb + r0;
           w.eb = d_eBd + c0;
           w.out = d_Kpart + (long long)k * nbf * nbf + (long long)r0 * nbf + c0;
           w.ldr = nbf;
@@ -381,18 +407,28 @@ struct AoKState {
     if (alloc(&d_items, items.size()) || alloc(&d_jobs, jobs.size()) ||
         cudaMemcpy(d_items, items.data(), items.size() * sizeof(SplitItem),
                    cudaMemcpyHostToDevice) ||
-        cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(SplitJob), cudaMemcpyHostToDevice)) {
+        cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(SplitJob), cudaMemcpyHostToDevice) ||
+        cudaMemcpy(d_eoff, eoff.data(), eoff.size() * sizeof(long long), cudaMemcpyHostToDevice)) {
       *err = "DF-AO K: out of memory for the work lists";
       return GBJK_OOM;
     }
-    // once: the dense Bfit (staged in the cbar buffer), its row exponents
-    // and digits
-    gbjk_status s;
-    if ((s = expand(st, L, sp.Bfit, d_cbar, launches, err))) return s;
+    // once: the dense Bfit (staged in the buffer of cbar's integers), its row
+    // exponents and digits; then the buffer's padding is zero again
+    if (cudaMemsetAsync(d_cbi, 0, big * 8, st) != cudaSuccess) {
+      *err = "DF-AO K: memset failed";
+      return GBJK_CUDA_ERROR;
+    }
+    k_expand_panels_perm<<<dim3(cdiv_(L.maxK, 128), naux, nbf), 128, 0, st>>>(
+        sp.Bfit, L.d_panel_off, L.d_blk_of, L.d_boff, L.d_panelK, L.d_cmoff, L.d_colmap, naux, ld,
+        kdim, (double*)d_cbi);
     k_row_maxexp<<<dim3(cdiv_((long long)nbf * 32, 256), 1), 256, 0, st>>>(d_jobs + j_bd);
     const long long thr = (long long)(nbf / 8 + 2) * r_nkt * 32;
     k_split_tiles<<<dim3(cdiv_(thr, 256), 1), 256, 0, st>>>(d_jobs + j_bd);
-    *launches += 2;
+    *launches += 3;
+    if (cudaMemsetAsync(d_cbi, 0, big * 8, st) != cudaSuccess) {
+      *err = "DF-AO K: memset failed";
+      return GBJK_CUDA_ERROR;
+    }
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
       *err = std::string("DF-AO K split preparation: ") + cudaGetErrorString(e);
@@ -429,15 +465,12 @@ struct AoKState {
       k_row_maxexp<<<dim3(cdiv_((long long)nbf * 32, 256), L.nblk), 256, 0, st>>>(d_jobs + j_p0);
       k_split_tiles<<<dim3(cdiv_(p_maxthr, 256), L.nblk), 256, 0, st>>>(d_jobs + j_p0);
       *launches += 2;
-      if (cudaMemsetAsync(d_eCb, 0, (size_t)r_nrb * 32 * 4, st) != cudaSuccess) {
+      if (cudaMemsetAsync(d_eCb, kNoExpByte, (size_t)r_nrb * 32 * 4, st) != cudaSuccess) {
         *err = "DF-AO K: memset failed";
         return GBJK_CUDA_ERROR;
       }
-      if ((s = sp.launch_gemm(st, d_items + i_ht0, i_htn, launches, err))) return s;
-      k_exp_unbias<<<cdiv_((long long)r_nrb * 32, 256), 256, 0, st>>>((int*)d_eCb, r_nrb * 32);
-      const long long thr = (long long)(nbf / 8 + 2) * r_nkt * 32;
-      k_split_tiles<<<dim3(cdiv_(thr, 256), 1), 256, 0, st>>>(d_jobs + j_cb);
-      *launches += 2;
+      if ((s = sp.launch_gemm<kOutInt>(st, d_items + i_ht0, i_htn, launches, err))) return s;
+      SplitState::launch_ints<true>(st, cjob.data(), 1, launches);
       if ((s = sp.launch_gemm(st, d_items + i_k0, i_kn, launches, err))) return s;
       k_splitk_reduce<<<cdiv_(nn, 256), 256, 0, st>>>(d_Kpart, ksplit, nbf, -1.0, 1, dK);
       (*launches)++;

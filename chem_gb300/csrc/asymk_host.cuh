@@ -11,8 +11,11 @@
 // FP64 path: the reference route (grouped half transforms, V^-1 fit of the
 // v side, one non-symmetric split-K GEMM; bitwise equal to the oracle).
 // Split path, Cholesky route on the prefitted tensor Bfit = L^-1 B:
-// K = -(Bfit u)(Bfit v)^T over k = (Y, i), both half transforms as split
-// GEMMs, then the exchange over all tiles, split over k.
+// K = -(Bfit u)(Bfit v)^T over k = (Y, i): both half transforms as one split
+// GEMM over the columns [u | v] (one 96-wide tile holds up to 48 vectors of
+// each side; a tile per side computed twice the products and read the tensor's
+// digits twice: 614 us against 300 for C14H30, 37 vectors), integers out, then
+// the exchange over all tiles, split over k.
 #pragma once
 #include <algorithm>
 #include <string>
@@ -30,6 +33,9 @@ struct AsymKState {
   bool ready = false;
   double *d_U = nullptr, *d_V = nullptr, *d_Ug = nullptr, *d_Vg = nullptr;
   double *d_Hu = nullptr, *d_Hv = nullptr, *d_Hvf = nullptr, *d_Kpart = nullptr;
+  long long* d_Hi = nullptr;  // split: integers of [Bfit u | Bfit v]
+  long long* d_eoff = nullptr;
+  std::vector<SplitIntJob> hjobs;
   // FP64 plan
   GemmGroup* d_groups = nullptr;
   GemmTile* d_tiles = nullptr;
@@ -37,12 +43,12 @@ struct AsymKState {
   // split plan
   uint16_t *d_Cdig = nullptr, *d_Hdig = nullptr;
   int* d_eC = nullptr;
-  unsigned int* d_eH = nullptr;
+  int* d_eH = nullptr;
   SplitItem* d_items = nullptr;
   SplitJob* d_jobs = nullptr;
-  int i_ht0 = 0, i_htn = 0, i_k0 = 0, i_kn = 0, j_h0 = 0;
+  int i_ht0 = 0, i_htn = 0, i_k0 = 0, i_kn = 0;
   int c_nrb = 0, h_nrb = 0, h_nkt = 0, c_maxthr = 0;
-  long long cdig_side = 0, hdig_side = 0;
+  long long hdig_side = 0;
 
   template <class T>
   cudaError_t alloc(T** p, size_t n) {
@@ -61,6 +67,8 @@ struct AsymKState {
   }
   void release() {
     for (double** p : {&d_U, &d_V, &d_Ug, &d_Vg, &d_Hu, &d_Hv, &d_Hvf, &d_Kpart}) free_(p);
+    free_(&d_Hi);
+    free_(&d_eoff);
     free_(&d_groups);
     free_(&d_tiles);
     free_(&d_Cdig);
@@ -89,12 +97,10 @@ struct AsymKState {
     // the split epilogue stores FP64 pairs (even stride); the FP64 path keeps
     // the unpadded k = (X, i) order of the oracle
     hld = prec == GBJK_SPLIT_BF16 ? nocc + (nocc & 1) : nocc;
-    const size_t nbf = L.nbf, naux = L.naux;
-    const size_t hsz = nbf * naux * hld;
+    const size_t nbf = L.nbf;
     if (alloc(&d_U, nbf * nocc) || alloc(&d_V, nbf * nocc) ||
-        alloc(&d_Ug, (size_t)L.ncols_total * nocc) || alloc(&d_Vg, (size_t)L.ncols_total * nocc) ||
-        alloc(&d_Hu, hsz) || alloc(&d_Hv, hsz) || cudaMemset(d_Hu, 0, hsz * 8) ||
-        cudaMemset(d_Hv, 0, hsz * 8)) {
+        alloc(&d_Ug, (size_t)L.ncols_total * nocc) || alloc(&d_Vg, (size_t)L.ncols_total * nocc)) {
+      release();
       *err = "non-symmetric DF-LMO K: out of device memory";
       return GBJK_OOM;
     }
@@ -114,7 +120,8 @@ struct AsymKState {
     const long long kdim = (long long)naux * hld;
     long long kc = kdim;
     gbjk_k_split_plan(L.nbf, L.naux, hld, &ksplit, &kc);
-    if (alloc(&d_Hvf, nbf * naux * hld) || alloc(&d_Kpart, (size_t)ksplit * nbf * nbf)) {
+    if (alloc(&d_Hu, nbf * naux * hld) || alloc(&d_Hv, nbf * naux * hld) ||
+        alloc(&d_Hvf, nbf * naux * hld) || alloc(&d_Kpart, (size_t)ksplit * nbf * nbf)) {
       *err = "non-symmetric DF-LMO K: out of device memory";
       return GBJK_OOM;
     }
@@ -198,27 +205,30 @@ struct AsymKState {
       return GBJK_INVALID_ARG;
     }
     const int nbf = L.nbf, naux = L.naux, nblk = L.nblk;
-    c_nrb = cdiv_(nocc, kTileN) * (kTileN / 32);
+    const int lc = 2 * hld;                       // columns [u | v]
+    const int npad = SplitState::pad32(naux);     // auxiliary slots of an H row
+    const long long hrow = (long long)npad * lc;  // an H row
+    c_nrb = cdiv_(lc, kTileN) * (kTileN / 32);
     std::vector<long long> c_off(nblk);
     long long ctot = 0;
     for (int I = 0; I < nblk; ++I) {
       c_off[I] = ctot;
       ctot += (long long)c_nrb * sp.nkt[I] * kSlices * kImage;
     }
-    cdig_side = ctot;
     h_nrb = std::max(cdiv_(nbf, kTileM) * (kTileM / 32), cdiv_(nbf, kTileN) * (kTileN / 32));
-    h_nkt = cdiv_((long long)naux * hld, kTileK);
+    h_nkt = cdiv_((long long)npad * hld, kTileK);
     hdig_side = (long long)h_nrb * h_nkt * kSlices * kImage;
     const int ntile = cdiv_(nbf, kTileM) * cdiv_(nbf, kTileN);
     const int ks = sp.choose_ksplit(h_nkt, ntile);
     const int kt_per = cdiv_(h_nkt, ks);
     ksplit = cdiv_(h_nkt, kt_per);
-    if (alloc(&d_Cdig, (size_t)2 * ctot) || alloc(&d_Hdig, (size_t)2 * hdig_side) ||
-        alloc(&d_eC, (size_t)2 * nblk * c_nrb * 32) || alloc(&d_eH, (size_t)2 * h_nrb * 32) ||
+    if (alloc(&d_Cdig, (size_t)ctot) || alloc(&d_Hdig, (size_t)2 * hdig_side) ||
+        alloc(&d_eC, (size_t)nblk * c_nrb * 32) || alloc(&d_eH, (size_t)2 * h_nrb * 32) ||
+        alloc(&d_Hi, (size_t)nbf * hrow) || alloc(&d_eoff, (size_t)3 * nbf) ||
         alloc(&d_Kpart, (size_t)ksplit * nbf * nbf) ||
-        cudaMemset(d_Cdig, 0, (size_t)2 * ctot * 2) ||
+        cudaMemset(d_Cdig, 0, (size_t)ctot * 2) || cudaMemset(d_Hi, 0, (size_t)nbf * hrow * 8) ||
         cudaMemset(d_Hdig, 0, (size_t)2 * hdig_side * 2) ||
-        cudaMemset(d_eC, 0, (size_t)2 * nblk * c_nrb * 32 * 4)) {
+        cudaMemset(d_eC, 0, (size_t)nblk * c_nrb * 32 * 4)) {
       *err = "non-symmetric DF-LMO K: out of device memory for the split path";
       return GBJK_OOM;
     }
@@ -231,77 +241,91 @@ struct AsymKState {
         j.src = (side ? d_Vg : d_Ug) + (long long)(*L.cmoff)[I] * nocc;
         j.rs = 1;
         j.cs = nocc;
-        j.row0 = 0;
+        j.row0 = side * hld;
         j.nrows = nocc;
         j.ncols = (*L.panelK)[I];
-        j.e = d_eC + ((long long)side * nblk + I) * c_nrb * 32;
-        j.e_biased = 0;
+        j.e = d_eC + (long long)I * c_nrb * 32;
         j.nrb = c_nrb;
         j.nkt = sp.nkt[I];
-        j.dst = d_Cdig + side * cdig_side + c_off[I];
+        j.dst = d_Cdig + c_off[I];
         jobs.push_back(j);
         c_maxthr = std::max(c_maxthr, (nocc / 8 + 2) * sp.nkt[I] * 32);
       }
-    j_h0 = (int)jobs.size();
+    // digits of the two sides of H: exponent offsets per AO function (the
+    // tensor's rows, then the columns of u and of v)
+    std::vector<long long> eoff((size_t)3 * nbf);
+    for (int I = 0; I < nblk; ++I)
+      for (int m = 0; m < (*L.bsize)[I]; ++m) {
+        const int mu = (*L.boff)[I] + m;
+        eoff[mu] = sp.eA_off[I] + (long long)m * sp.apitch;
+        for (int side = 0; side < 2; ++side)
+          eoff[(size_t)(1 + side) * nbf + mu] = (long long)I * c_nrb * 32 + side * hld;
+      }
+    hjobs.clear();
     for (int side = 0; side < 2; ++side) {
-      SplitJob j;
-      j.src = side ? d_Hv : d_Hu;
-      j.rs = (long long)naux * hld;
-      j.cs = 1;
-      j.row0 = 0;
+      SplitIntJob j;
+      j.src = d_Hi + (long long)side * 32 * hld;
+      j.rs = hrow;
+      j.ncols = (long long)npad * hld;
+      j.gs = 32LL * lc;
       j.nrows = nbf;
-      j.ncols = (long long)naux * hld;
-      j.e = (int*)d_eH + (long long)side * h_nrb * 32;
-      j.e_biased = 0;
+      j.ny = npad;
+      j.ld = hld;
+      j.e = d_eH + (long long)side * h_nrb * 32;
+      j.ea = sp.d_eA;
+      j.ea_off = d_eoff;
+      j.eb = d_eC;
+      j.eb_off = d_eoff + (size_t)(1 + side) * nbf;
       j.nrb = h_nrb;
       j.nkt = h_nkt;
       j.dst = d_Hdig + side * hdig_side;
-      jobs.push_back(j);
+      hjobs.push_back(j);
     }
     auto base = []() {
       SplitItem w;
       w.emax = nullptr;
       w.emax_row0 = 0;
       w.emax_div = 1;
+      w.out = nullptr;
       w.out2 = nullptr;
       w.c0 = 0;
       w.ncol1 = 1 << 30;
       return w;
     };
-    // both sides' tiles of one A row tile are adjacent: its digits come
-    // from HBM once and from L2 for the other side
     i_ht0 = 0;
     for (int I = 0; I < nblk; ++I) {
       // A rows (m, Y) at m * sp.apitch + Y (SplitItem::apitch)
       const long long rows = (long long)(*L.bsize)[I] * sp.apitch;
       for (int mt = 0; mt < cdiv_(rows, kTileM); ++mt)
-        for (int side = 0; side < 2; ++side)
-          for (int nt = 0; nt < cdiv_(nocc, kTileN); ++nt) {
-            SplitItem w = base();
-            w.a = sp.d_Aslices + sp.a_off[I];
-            w.a_nrb = sp.a_nrb[I];
-            w.a_rb0 = mt * (kTileM / 32);
-            w.apitch = sp.apitch;
-            w.arow0 = mt * kTileM;
-            w.ay_valid = naux;
-            w.b = d_Cdig + side * cdig_side + c_off[I];
-            w.b_nrb = c_nrb;
-            w.b_rb0 = nt * (kTileN / 32);
-            w.kt0 = 0;
-            w.nkt = sp.nkt[I];
-            w.ea = sp.d_eA + sp.eA_off[I] + (long long)mt * kTileM;
-            w.eb = d_eC + ((long long)side * nblk + I) * c_nrb * 32 + (long long)nt * kTileN;
-            w.out = (side ? d_Hv : d_Hu) +
-                    ((long long)(*L.boff)[I] * naux + (long long)mt * kTileM) * hld +
-                    (long long)nt * kTileN;
-            w.ldr = hld;
-            w.m_valid = (int)std::min<long long>(kTileM, rows - (long long)mt * kTileM);
-            w.n_valid = std::min(kTileN, nocc - nt * kTileN);
-            w.emax = d_eH + (long long)side * h_nrb * 32 + (*L.boff)[I];
-            w.emax_row0 = mt * kTileM;
-            w.emax_div = naux;
-            items.push_back(w);
-          }
+        for (int nt = 0; nt < cdiv_(lc, kTileN); ++nt) {
+          SplitItem w = base();
+          w.a = sp.d_Aslices + sp.a_off[I];
+          w.a_nrb = sp.a_nrb[I];
+          w.a_rb0 = mt * (kTileM / 32);
+          w.apitch = sp.apitch;
+          w.arow0 = mt * kTileM;
+          w.ay_valid = naux;
+          w.b = d_Cdig + c_off[I];
+          w.b_nrb = c_nrb;
+          w.b_rb0 = nt * (kTileN / 32);
+          w.kt0 = 0;
+          w.nkt = sp.nkt[I];
+          w.ea = sp.d_eA + sp.eA_off[I] + (long long)mt * kTileM;
+          w.eb = d_eC + (long long)I * c_nrb * 32 + (long long)nt * kTileN;
+          w.iout = d_Hi + (long long)(*L.boff)[I] * hrow;
+          w.ldr = lc;
+          w.perm_rs = hrow;
+          w.perm_div = naux;
+          w.c0 = nt * kTileN;
+          w.m_valid = (int)std::min<long long>(kTileM, rows - (long long)mt * kTileM);
+          w.n_valid = std::min(kTileN, lc - nt * kTileN);
+          w.emax = d_eH + (*L.boff)[I];
+          w.emax2 = d_eH + (long long)h_nrb * 32 + (*L.boff)[I];
+          w.csplit = hld - nt * kTileN;
+          w.emax_row0 = mt * kTileM;
+          w.emax_div = naux;
+          items.push_back(w);
+        }
     }
     i_htn = (int)items.size() - i_ht0;
     i_k0 = (int)items.size();
@@ -318,8 +342,8 @@ struct AsymKState {
           w.b_rb0 = nt * (kTileN / 32);
           w.kt0 = kt0;
           w.nkt = n_kt;
-          w.ea = (const int*)d_eH + (long long)mt * kTileM;
-          w.eb = (const int*)d_eH + (long long)h_nrb * 32 + (long long)nt * kTileN;
+          w.ea = d_eH + (long long)mt * kTileM;
+          w.eb = d_eH + (long long)h_nrb * 32 + (long long)nt * kTileN;
           w.out = d_Kpart + (long long)k * nbf * nbf + (long long)mt * kTileM * nbf +
                   (long long)nt * kTileN;
           w.ldr = nbf;
@@ -332,38 +356,35 @@ struct AsymKState {
     if (alloc(&d_items, items.size()) || alloc(&d_jobs, jobs.size()) ||
         cudaMemcpy(d_items, items.data(), items.size() * sizeof(SplitItem),
                    cudaMemcpyHostToDevice) ||
-        cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(SplitJob), cudaMemcpyHostToDevice)) {
+        cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(SplitJob), cudaMemcpyHostToDevice) ||
+        cudaMemcpy(d_eoff, eoff.data(), eoff.size() * sizeof(long long), cudaMemcpyHostToDevice)) {
       *err = "non-symmetric DF-LMO K: out of memory for the work lists";
       return GBJK_OOM;
     }
     return GBJK_OK;
   }
 
-  // K from u (nbf x nocc) and v (nbf x nocc, the transpose of the
-  // reference's vt), both already in d_U / d_V.
+  // K from u (nbf x nocc, in d_U) and vt (nocc x nbf, in d_V).
   gbjk_status run(cudaStream_t st, int nbf, int naux, int nblk, int ncols_total,
                   const int* d_colmap, double* dK, SplitState& sp, int64_t* launches,
                   std::string* err) {
     const long long nn = (long long)nbf * nbf;
     const long long gtot = (long long)ncols_total * nocc;
     k_gather_cols<<<cdiv_(gtot, 256), 256, 0, st>>>(d_U, nocc, d_colmap, ncols_total, d_Ug);
-    k_gather_cols<<<cdiv_(gtot, 256), 256, 0, st>>>(d_V, nocc, d_colmap, ncols_total, d_Vg);
+    k_gather_cols_t<<<cdiv_(gtot, 256), 256, 0, st>>>(d_V, nocc, nbf, d_colmap, ncols_total,
+                                                      d_Vg);
     *launches += 2;
     if (precision == GBJK_SPLIT_BF16) {
       gbjk_status s;
       k_row_maxexp<<<dim3(cdiv_((long long)nocc * 32, 256), 2 * nblk), 256, 0, st>>>(d_jobs);
       k_split_tiles<<<dim3(cdiv_(c_maxthr, 256), 2 * nblk), 256, 0, st>>>(d_jobs);
       *launches += 2;
-      if (cudaMemsetAsync(d_eH, 0, (size_t)2 * h_nrb * 32 * 4, st) != cudaSuccess) {
+      if (cudaMemsetAsync(d_eH, kNoExpByte, (size_t)2 * h_nrb * 32 * 4, st) != cudaSuccess) {
         *err = "non-symmetric DF-LMO K: memset failed";
         return GBJK_CUDA_ERROR;
       }
-      if ((s = sp.launch_gemm(st, d_items + i_ht0, i_htn, launches, err))) return s;
-      k_exp_unbias<<<cdiv_((long long)2 * h_nrb * 32, 256), 256, 0, st>>>((int*)d_eH,
-                                                                          2 * h_nrb * 32);
-      const long long thr = (long long)(nbf / 8 + 2) * h_nkt * 32;
-      k_split_tiles<<<dim3(cdiv_(thr, 256), 2), 256, 0, st>>>(d_jobs + j_h0);
-      *launches += 2;
+      if ((s = sp.launch_gemm<kOutIntTwo>(st, d_items + i_ht0, i_htn, launches, err))) return s;
+      SplitState::launch_ints<true>(st, hjobs.data(), 2, launches);
       if ((s = sp.launch_gemm(st, d_items + i_k0, i_kn, launches, err))) return s;
     } else {
       auto gemm = [&](int t0, int n, bool transB) {

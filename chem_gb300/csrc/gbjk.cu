@@ -39,6 +39,8 @@ using namespace gbjk;
 // (a build through the host call: C20H42 1.89 ms against 1.92 in order, C10H22
 // 0.403 against 0.422, five waters 0.164 against 0.182).
 constexpr int kDefaultOverlapSms = 0;
+// ... as long as J's tensor copy is smaller than this
+constexpr size_t kOverlapJBytes = size_t(384) << 20;
 
 enum Phase {
   PH_GATHER = 0,
@@ -1769,9 +1771,14 @@ static gbjk_status run_jk_split(gbjk_ctx* ctx, const double* dP, const double* d
   }
   // J = (L^-1 B)^T dt needs only the half transform's density partials: with
   // overlap on (and no per-phase timing, whose events sit on one stream) it
-  // runs on the side stream beside the exchange
+  // runs on the side stream beside the exchange.  Where J alone fills the
+  // GPU's memory bandwidth the two only delay each other, and the phases run in
+  // order (C20H42, 1.1 GB: 1.93 ms against 1.96 side by side; C10H22, 0.2 GB:
+  // 0.414 against 0.413; five waters, 0.03 GB: 166 us against 155).
   const bool fused = dJ && ctx->split.fused_j();
-  const bool overlap = fused && ctx->overlap_sms >= 0 && !ctx->profile;
+  const bool overlap = fused && !ctx->profile &&
+                       (ctx->overlap_sms > 0 ||
+                        (ctx->overlap_sms == 0 && ctx->split.j_bytes() < kOverlapJBytes));
   ctx->split.ev_ht = overlap ? ctx->ev_fork : nullptr;
   ctx->split.k_grid = overlap ? ctx->overlap_sms : 0;
   s = ctx->split.run_k(ctx->stream, dK, &ctx->launches, &ctx->err);
@@ -2110,13 +2117,9 @@ gbjk_status gbjk_compute_k_lmo_asym(gbjk_ctx* ctx, const double* U, const double
     if ((s = a.plan(ctx->precision, nocc, L, ctx->d_B, ctx->d_Vinv, ctx->split, &ctx->err)))
       return s;
   }
-  // v = Vt^T as nbf x nocc, row-major
   const int nbf = ctx->nbf;
-  std::vector<double> v((size_t)nbf * nocc);
-  for (int i = 0; i < nocc; ++i)
-    for (int n = 0; n < nbf; ++n) v[(size_t)n * nocc + i] = Vt[(size_t)i * nbf + n];
   CK(cudaMemcpyAsync(a.d_U, U, (size_t)nbf * nocc * 8, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(a.d_V, v.data(), v.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(a.d_V, Vt, (size_t)nbf * nocc * 8, cudaMemcpyHostToDevice, ctx->stream));
   if (ctx->precision == GBJK_SPLIT_BF16 && (s = ctx->split.clear_error(ctx->stream)))
     return fail(ctx, s, "split path: memset failed");
   {

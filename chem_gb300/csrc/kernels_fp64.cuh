@@ -54,6 +54,16 @@ __global__ void k_gather_cols(const double* __restrict__ Cm, int n, const int* _
   Cg[idx] = Cm[(long long)colmap[r] * n + i];
 }
 
+// Cg[r*n + i] = Ct[i*ld + colmap[r]]: the same from the transposed matrix.
+__global__ void k_gather_cols_t(const double* __restrict__ Ct, int n, int ld,
+                                const int* __restrict__ colmap, int nrows,
+                                double* __restrict__ Cg) {
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (long long)nrows * n) return;
+  const int r = (int)(idx / n), i = (int)(idx % n);
+  Cg[idx] = Ct[(long long)i * ld + colmap[r]];
+}
+
 // part[mu][X] = sum_k B_I[m][X][k] * Pg_I[m][k]; one warp per (mu, X) row.
 __global__ void k_j_rowdot(const double* __restrict__ B, const long long* __restrict__ panel_off,
                            const int* __restrict__ blk_of, const int* __restrict__ boff,
@@ -457,6 +467,25 @@ __global__ void k_expand_panels(const double* __restrict__ P, const long long* _
   const int m = mu - boff[I];
   D[((long long)mu * naux + X) * nbf + colmap[cmoff[I] + k]] =
       P[panel_off[I] + ((long long)m * naux + X) * KI + k];
+}
+
+// The same expansion in the column-pair-outermost order of a split half
+// transform (rows of rs values, ld columns): D[mu * rs + (X / 32) * 32 ld +
+// (c / 2) * 64 + (X % 32) * 2 + c % 2], c = colmap(k).
+__global__ void k_expand_panels_perm(const double* __restrict__ P,
+                                     const long long* __restrict__ panel_off,
+                                     const int* __restrict__ blk_of, const int* __restrict__ boff,
+                                     const int* __restrict__ panel_K,
+                                     const int* __restrict__ cmoff, const int* __restrict__ colmap,
+                                     int naux, int ld, long long rs, double* __restrict__ D) {
+  const int mu = blockIdx.z, X = blockIdx.y;
+  const int I = blk_of[mu];
+  const int KI = panel_K[I];
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= KI) return;
+  const int m = mu - boff[I], c = colmap[cmoff[I] + k];
+  D[(long long)mu * rs + (long long)(X >> 5) * 32 * ld + (long long)(c >> 1) * 64 + (X & 31) * 2 +
+    (c & 1)] = P[panel_off[I] + ((long long)m * naux + X) * KI + k];
 }
 
 // Grouped FP64 GEMM over a tile list; 64 x TN tiles (TN = 64, 32 or 16),

@@ -81,14 +81,25 @@ __global__ void k_mp2_rowsq(const double* __restrict__ Z, int n, double* __restr
   if (lane == 0) rsq[(long long)t * n + w] = s;
 }
 
-// e[t] = sum_X rsq[t][X] in X order (one thread per point).
+// e[t] = sum_X rsq[t][X] in X order: a serial chain of n additions, bound by
+// their latency once thirty-two loads are in flight (one warp per point
+// passes them on by shuffles).  grid npts, block 32.
 __global__ void k_mp2_energy(const double* __restrict__ rsq, int n, int npts,
                              double* __restrict__ e) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= npts) return;
+  const int t = blockIdx.x, lane = threadIdx.x;
+  const double* p = rsq + (long long)t * n;
   double s = 0.0;
-  for (int X = 0; X < n; ++X) s += rsq[(long long)t * n + X];
-  e[t] = s;
+  double next = lane < n ? p[lane] : 0.0;
+  for (int X0 = 0; X0 < n; X0 += 32) {
+    const double v = next;
+    if (X0 + 32 + lane < n) next = p[X0 + 32 + lane];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      const double x = __shfl_sync(0xffffffffu, v, j);
+      if (X0 + j < n) s += x;
+    }
+  }
+  if (lane == 0) e[t] = s;
 }
 
 }  // namespace gbjk

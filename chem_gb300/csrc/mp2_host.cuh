@@ -46,14 +46,16 @@ struct Mp2State {
   // split plan
   uint16_t *d_Cdig = nullptr, *d_Hdig = nullptr, *d_Lvdig = nullptr, *d_Wdig = nullptr;
   int *d_eC = nullptr, *d_eH = nullptr, *d_eLv = nullptr;
-  unsigned int* d_eW = nullptr;
+  int* d_eW = nullptr;
   double* d_Zpart = nullptr;
   SplitItem* d_items = nullptr;
   SplitJob* d_jobs = nullptr;
   int i1_0 = 0, i1_n = 0, i2_0 = 0, i2_n = 0, iz_0 = 0, iz_n = 0;
-  int jc_0 = 0, jlv_0 = 0, jh_0 = 0, jw_0 = 0;
+  int jc_0 = 0, jlv_0 = 0, jh_0 = 0;
   int c_nrb = 0, h_nrb = 0, h_nkt = 0, lv_nrb = 0, w_nrb = 0, w_nkt = 0, ksplit = 1;
-  long long cdig_stride = 0, hdig_stride = 0, lvdig_stride = 0, wdig_stride = 0;
+  long long hdig_stride = 0, lvdig_stride = 0, wdig_stride = 0;
+  long long *d_cofs = nullptr, *d_eoff = nullptr;
+  std::vector<SplitIntJob> wjobs;
   int c_maxthr = 0;
   // profiling
   bool profile = false;
@@ -98,6 +100,8 @@ struct Mp2State {
     free_(&d_Zpart);
     free_(&d_items);
     free_(&d_jobs);
+    free_(&d_cofs);
+    free_(&d_eoff);
     resolve();
     bytes = 0;
     npts = 0;
@@ -294,13 +298,21 @@ struct Mp2State {
       return GBJK_INVALID_ARG;
     }
     // digit buffers
-    c_nrb = cdiv_(hld, kTileN) * (kTileN / 32);
+    // T1 columns: every point's occupied columns side by side (an even number
+    // each), so that a 96-wide tile is full whatever the ranks are
+    std::vector<int> co(npts + 1, 0);
+    for (int t = 0; t < npts; ++t) co[t + 1] = co[t] + ro[t] + (ro[t] & 1);
+    const int ncol = co[npts];
+    c_nrb = cdiv_(ncol, kTileN) * (kTileN / 32);
     std::vector<long long> cdig_off(nblk);
-    cdig_stride = 0;
+    long long cdig_tot = 0;
     for (int I = 0; I < nblk; ++I) {
-      cdig_off[I] = cdig_stride;
-      cdig_stride += (long long)c_nrb * sp.nkt[I] * kSlices * kImage;
+      cdig_off[I] = cdig_tot;
+      cdig_tot += (long long)c_nrb * sp.nkt[I] * kSlices * kImage;
     }
+    std::vector<long long> cofs((size_t)c_nrb * 32, 0);
+    for (int t = 0; t < npts; ++t)
+      for (int i = 0; i < co[t + 1] - co[t]; ++i) cofs[co[t] + i] = t * h_stride + i;
     h_nrb = cdiv_(nrho, kTileM) * (kTileM / 32);
     h_nkt = cdiv_(nbf, kTileK);
     hdig_stride = (long long)h_nrb * h_nkt * kSlices * kImage;
@@ -320,18 +332,19 @@ struct Mp2State {
     const int kt_per = cdiv_(w_nkt, ks);
     ksplit = cdiv_(w_nkt, kt_per);
     const size_t nn = (size_t)naux * naux;
-    if (alloc(&d_Cdig, (size_t)npts * cdig_stride) || alloc(&d_Hdig, (size_t)npts * hdig_stride) ||
+    if (alloc(&d_Cdig, (size_t)cdig_tot) || alloc(&d_Hdig, (size_t)npts * hdig_stride) ||
         alloc(&d_Lvdig, (size_t)npts * lvdig_stride) ||
         alloc(&d_Wdig, (size_t)npts * wdig_stride) ||
-        alloc(&d_eC, (size_t)npts * nblk * c_nrb * 32) ||
+        alloc(&d_eC, (size_t)nblk * c_nrb * 32) || alloc(&d_cofs, cofs.size()) ||
+        alloc(&d_eoff, (size_t)2 * npts * naux) ||
         alloc(&d_eH, (size_t)npts * h_nrb * 32) || alloc(&d_eLv, (size_t)npts * lv_nrb * 32) ||
         alloc(&d_eW, (size_t)npts * w_nrb * 32) ||
         alloc(&d_Zpart, (size_t)ksplit * npts * nn) ||
-        cudaMemsetAsync(d_Cdig, 0, (size_t)npts * cdig_stride * 2, st) ||
+        cudaMemsetAsync(d_Cdig, 0, (size_t)cdig_tot * 2, st) ||
         cudaMemsetAsync(d_Hdig, 0, (size_t)npts * hdig_stride * 2, st) ||
         cudaMemsetAsync(d_Lvdig, 0, (size_t)npts * lvdig_stride * 2, st) ||
         cudaMemsetAsync(d_Wdig, 0, (size_t)npts * wdig_stride * 2, st) ||
-        cudaMemsetAsync(d_eC, 0, (size_t)npts * nblk * c_nrb * 32 * 4, st) ||
+        cudaMemsetAsync(d_eC, 0, (size_t)nblk * c_nrb * 32 * 4, st) ||
         cudaMemsetAsync(d_eH, 0, (size_t)npts * h_nrb * 32 * 4, st) ||
         cudaMemsetAsync(d_eLv, 0, (size_t)npts * lv_nrb * 32 * 4, st)) {
       *err = "MP2 batch: out of device memory for the operand digits";
@@ -347,14 +360,13 @@ struct Mp2State {
         j.src = d_Cg + t * cg_stride + (long long)cmoff[I] * hld;
         j.rs = 1;
         j.cs = hld;
-        j.row0 = 0;
+        j.row0 = co[t];
         j.nrows = ro[t];
         j.ncols = panelK[I];
-        j.e = d_eC + ((long long)t * nblk + I) * c_nrb * 32;
-        j.e_biased = 0;
+        j.e = d_eC + (long long)I * c_nrb * 32;
         j.nrb = c_nrb;
         j.nkt = sp.nkt[I];
-        j.dst = d_Cdig + t * cdig_stride + cdig_off[I];
+        j.dst = d_Cdig + cdig_off[I];
         jobs.push_back(j);
         c_maxthr = std::max(c_maxthr, (ro[t] / 8 + 2) * sp.nkt[I] * 32);
       }
@@ -368,7 +380,6 @@ struct Mp2State {
       j.nrows = rv[t];
       j.ncols = nbf;
       j.e = d_eLv + (long long)t * lv_nrb * 32;
-      j.e_biased = 0;
       j.nrb = lv_nrb;
       j.nkt = h_nkt;
       j.dst = d_Lvdig + t * lvdig_stride;
@@ -384,27 +395,38 @@ struct Mp2State {
       j.nrows = (int)nrho;
       j.ncols = nbf;
       j.e = d_eH + (long long)t * h_nrb * 32;
-      j.e_biased = 0;
       j.nrb = h_nrb;
       j.nkt = h_nkt;
       j.dst = d_Hdig + t * hdig_stride;
       jobs.push_back(j);
     }
-    jw_0 = (int)jobs.size();
+    // W rows X from the integers of T2, k = (i, a) in the column-pair-outermost
+    // order of hld indices i and vld columns a
+    std::vector<long long> eoff((size_t)2 * npts * naux);
+    wjobs.clear();
     for (int t = 0; t < npts; ++t) {
-      SplitJob j;
-      j.src = d_W + t * w_stride;
+      long long* ea = eoff.data() + (size_t)2 * t * naux;
+      for (int X = 0; X < naux; ++X) {
+        ea[X] = (long long)t * h_nrb * 32 + (long long)X * hld;
+        ea[naux + X] = (long long)t * lv_nrb * 32;
+      }
+      SplitIntJob j;
+      j.src = (const long long*)d_W + t * w_stride;
       j.rs = kw;
-      j.cs = 1;
-      j.row0 = 0;
-      j.nrows = naux;
       j.ncols = kw;
-      j.e = (int*)d_eW + (long long)t * w_nrb * 32;
-      j.e_biased = 0;
+      j.gs = 32LL * vld;
+      j.nrows = naux;
+      j.ny = hld;
+      j.ld = vld;
+      j.e = d_eW + (long long)t * w_nrb * 32;
+      j.ea = d_eH;
+      j.ea_off = d_eoff + (size_t)2 * t * naux;
+      j.eb = d_eLv;
+      j.eb_off = j.ea_off + naux;
       j.nrb = w_nrb;
       j.nkt = w_nkt;
       j.dst = d_Wdig + t * wdig_stride;
-      jobs.push_back(j);
+      wjobs.push_back(j);
     }
     // items
     std::vector<SplitItem> items;
@@ -413,12 +435,13 @@ struct Mp2State {
       w.emax = nullptr;
       w.emax_row0 = 0;
       w.emax_div = 1;
+      w.out = nullptr;
       w.out2 = nullptr;
       w.c0 = 0;
       w.ncol1 = 1 << 30;
       return w;
     };
-    // T1 items: the points' tiles of one A row tile are adjacent in the list
+    // T1 items: the column tiles of one A row tile are adjacent in the list
     // (and so run at the same time on different SMs), so the L^-1 B digit
     // tile is read from HBM once for all points and then served from L2
     i1_0 = 0;
@@ -426,29 +449,28 @@ struct Mp2State {
       // A rows (m, Y) at m * sp.apitch + Y (SplitItem::apitch)
       const long long rows = (long long)bsize[I] * sp.apitch;
       for (int mt = 0; mt < cdiv_(rows, kTileM); ++mt)
-        for (int t = 0; t < npts; ++t)
-          for (int nt = 0; nt < cdiv_(ro[t], kTileN); ++nt) {
-            SplitItem w = base_item();
-            w.a = sp.d_Aslices + sp.a_off[I];
-            w.a_nrb = sp.a_nrb[I];
-            w.a_rb0 = mt * (kTileM / 32);
-            w.apitch = sp.apitch;
-            w.arow0 = mt * kTileM;
-            w.ay_valid = naux;
-            w.b = d_Cdig + t * cdig_stride + cdig_off[I];
-            w.b_nrb = c_nrb;
-            w.b_rb0 = nt * (kTileN / 32);
-            w.kt0 = 0;
-            w.nkt = sp.nkt[I];
-            w.ea = sp.d_eA + sp.eA_off[I] + (long long)mt * kTileM;
-            w.eb = d_eC + ((long long)t * nblk + I) * c_nrb * 32 + (long long)nt * kTileN;
-            w.out = d_H + t * h_stride + ((long long)boff[I] * naux + (long long)mt * kTileM) * hld +
-                    (long long)nt * kTileN;
-            w.ldr = hld;
-            w.m_valid = (int)std::min<long long>(kTileM, rows - (long long)mt * kTileM);
-            w.n_valid = std::min(kTileN, ro[t] - nt * kTileN);
-            items.push_back(w);
-          }
+        for (int nt = 0; nt < cdiv_(ncol, kTileN); ++nt) {
+          SplitItem w = base_item();
+          w.a = sp.d_Aslices + sp.a_off[I];
+          w.a_nrb = sp.a_nrb[I];
+          w.a_rb0 = mt * (kTileM / 32);
+          w.apitch = sp.apitch;
+          w.arow0 = mt * kTileM;
+          w.ay_valid = naux;
+          w.b = d_Cdig + cdig_off[I];
+          w.b_nrb = c_nrb;
+          w.b_rb0 = nt * (kTileN / 32);
+          w.kt0 = 0;
+          w.nkt = sp.nkt[I];
+          w.ea = sp.d_eA + sp.eA_off[I] + (long long)mt * kTileM;
+          w.eb = d_eC + (long long)I * c_nrb * 32 + (long long)nt * kTileN;
+          w.out = d_H + ((long long)boff[I] * naux + (long long)mt * kTileM) * hld;
+          w.ldr = hld;
+          w.cofs = d_cofs + (long long)nt * kTileN;
+          w.m_valid = (int)std::min<long long>(kTileM, rows - (long long)mt * kTileM);
+          w.n_valid = std::min(kTileN, ncol - nt * kTileN);
+          items.push_back(w);
+        }
     }
     i1_n = (int)items.size();
     i2_0 = (int)items.size();
@@ -466,8 +488,11 @@ struct Mp2State {
           w.nkt = h_nkt;
           w.ea = d_eH + (long long)t * h_nrb * 32 + (long long)mt * kTileM;
           w.eb = d_eLv + (long long)t * lv_nrb * 32 + (long long)nt * kTileN;
-          w.out = d_W + t * w_stride + (long long)mt * kTileM * vld + (long long)nt * kTileN;
+          w.iout = (long long*)d_W + t * w_stride;
           w.ldr = vld;
+          w.perm_rs = kw;
+          w.perm_div = hld;
+          w.c0 = nt * kTileN;
           w.m_valid = (int)std::min<long long>(kTileM, nrho - (long long)mt * kTileM);
           w.n_valid = std::min(kTileN, rv[t] - nt * kTileN);
           // row rho = X * hld + i of W belongs to auxiliary row X
@@ -492,7 +517,7 @@ struct Mp2State {
             w.b_rb0 = c0 / 32;
             w.kt0 = kt0;
             w.nkt = n_kt;
-            const int* eW = (const int*)d_eW + (long long)t * w_nrb * 32;
+            const int* eW = d_eW + (long long)t * w_nrb * 32;
             w.ea = eW + r0;
             w.eb = eW + c0;
             w.out = d_Zpart + ((long long)k * npts + t) * nn + (long long)r0 * naux + c0;
@@ -506,7 +531,9 @@ struct Mp2State {
     if (alloc(&d_items, items.size()) || alloc(&d_jobs, jobs.size()) ||
         cudaMemcpy(d_items, items.data(), items.size() * sizeof(SplitItem),
                    cudaMemcpyHostToDevice) ||
-        cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(SplitJob), cudaMemcpyHostToDevice)) {
+        cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(SplitJob), cudaMemcpyHostToDevice) ||
+        cudaMemcpy(d_cofs, cofs.data(), cofs.size() * sizeof(long long), cudaMemcpyHostToDevice) ||
+        cudaMemcpy(d_eoff, eoff.data(), eoff.size() * sizeof(long long), cudaMemcpyHostToDevice)) {
       *err = "MP2 batch: out of memory for the work lists";
       return GBJK_OOM;
     }
@@ -560,7 +587,7 @@ struct Mp2State {
       }
       {
         Scope sc(this, kT1, st);
-        if ((s = sp.launch_gemm(st, d_items + i1_0, i1_n, launches, err))) return s;
+        if ((s = sp.launch_gemm<kOutF64Cols>(st, d_items + i1_0, i1_n, launches, err))) return s;
       }
       {
         Scope sc(this, kOps, st);
@@ -569,22 +596,18 @@ struct Mp2State {
         const long long hthr = (nrho / 8 + 2) * (long long)h_nkt * 32;
         k_split_tiles<<<dim3(cdiv_(hthr, 256), npts), 256, 0, st>>>(d_jobs + jh_0);
         *launches += 2;
-        if (cudaMemsetAsync(d_eW, 0, (size_t)npts * w_nrb * 32 * 4, st) != cudaSuccess) {
+        if (cudaMemsetAsync(d_eW, kNoExpByte, (size_t)npts * w_nrb * 32 * 4, st) != cudaSuccess) {
           *err = "MP2 batch: memset failed";
           return GBJK_CUDA_ERROR;
         }
       }
       {
         Scope sc(this, kT2, st);
-        if ((s = sp.launch_gemm(st, d_items + i2_0, i2_n, launches, err))) return s;
+        if ((s = sp.launch_gemm<kOutIntRagged>(st, d_items + i2_0, i2_n, launches, err))) return s;
       }
       {
         Scope sc(this, kOps, st);
-        k_exp_unbias<<<cdiv_((long long)npts * w_nrb * 32, 256), 256, 0, st>>>(
-            (int*)d_eW, npts * w_nrb * 32);
-        const long long wthr = (long long)(naux / 8 + 2) * w_nkt * 32;
-        k_split_tiles<<<dim3(cdiv_(wthr, 256), npts), 256, 0, st>>>(d_jobs + jw_0);
-        *launches += 2;
+        SplitState::launch_ints<false>(st, wjobs.data(), npts, launches);
       }
       {
         Scope sc(this, kZ, st);
@@ -620,7 +643,7 @@ struct Mp2State {
     {
       Scope sc(this, kOps, st);
       k_mp2_rowsq<<<dim3(cdiv_((long long)naux * 32, 256), npts), 256, 0, st>>>(d_Z, naux, d_rsq);
-      k_mp2_energy<<<cdiv_(npts, 32), 32, 0, st>>>(d_rsq, naux, npts, d_E);
+      k_mp2_energy<<<npts, 32, 0, st>>>(d_rsq, naux, npts, d_E);
       *launches += 2;
     }
     cudaError_t e = cudaGetLastError();

@@ -58,6 +58,9 @@
 namespace gbjk {
 
 constexpr int kMaxSlices = 8;
+// exponent of a row without a nonzero element: any value <= -2000 (cudaMemset
+// with the byte 0x80 gives one)
+constexpr int kNoExpByte = 0x80;
 constexpr int kSlices = 5;        // digits per operand
 constexpr int kTileM = 128;       // rows of A per tile (TMEM lanes)
 constexpr int kTileN = 96;        // rows of B per tile (accumulator columns)
@@ -84,38 +87,48 @@ struct SplitItem {
   int kt0, nkt;
   const int* ea;  // row exponents of the tile's A rows (tile-local index)
   const int* eb;  // row exponents of the tile's B rows
-  double* out;    // out[r * ldr + c]
+  double* out;    // out[r * ldr + c], or out[r * ldr + cofs[c]] (c even: a pair)
   long long ldr;
   int m_valid, n_valid;
-  // optional: atomicMax of the biased FP64 exponent of row r's results into
-  // emax[(emax_row0 + r) / emax_div] (row exponents of the next operand)
-  unsigned int* emax;
+  // optional: atomicMax of the exponent e of row r's results (|x| < 2^e) into
+  // emax[(emax_row0 + r) / emax_div] (row exponents of the next operand; the
+  // caller fills them with kNoExpByte: all zero).  kOutIntTwo: columns from
+  // csplit on (even, tile-local) go to emax2 instead.
+  int* emax;
   int emax_row0, emax_div;
+  int* emax2 = nullptr;
+  int csplit = 1 << 30;
   // optional: columns c0 + col >= ncol1 (c0 = first column of the tile) are
   // density columns m' = c0 + col - ncol1; the value of row r goes to
   // out2[emax_row0 + r] when m' == (emax_row0 + r) / emax_div, and is neither
   // stored in `out` nor counted in emax
   double* out2;
   int c0, ncol1;
-  // Output layout.  perm_rs == 0: row-major out[r * ldr + c].  perm_rs > 0:
-  // the half-transform layout.  The tile's row r is the linear panel row
+  // Output layout.  k_split_gemm writes FP64 values row-major,
+  // out[r * ldr + c].  The integer outputs (SplitOut) write its int64
+  // results V, value = V 2^(ea[r] + eb[c] - 46), to iout in the
+  // column-pair-outermost layout: the tile's row r is the linear panel row
   // R = emax_row0 + r = m * perm_div + y (AO function m of the panel,
-  // auxiliary index y); its value in column c lands at
-  //   out[m * perm_rs + (y / 32) * 32 * ldr + (c / 2) * 64 + (y % 32) * 2 + c % 2]
-  // (ldr even, out 16-byte aligned), i.e. within each group of 32 auxiliary
+  // auxiliary index y); column c (c0 + tile-local) lands at
+  //   iout[m * perm_rs + (y / 32) * 32 * ldr + (c / 2) * 64 + (y % 32) * 2 + c % 2]
+  // (ldr even, iout 16-byte aligned), i.e. within each group of 32 auxiliary
   // indices the column pairs are outermost.  A warp holds 32 consecutive
   // rows, so each of its 16-byte column-pair stores is one contiguous
-  // 512-byte run.  Rows of out are flat k-vectors of length perm_rs; a
+  // 512-byte run.  Rows of iout are flat k-vectors of length perm_rs; a
   // consumer that contracts over the whole k range (the exchange) needs no
   // other order, provided every row uses the same one.
+  long long* iout = nullptr;
+  // kOutIntRagged: the last group holds perm_div mod 32 y (even), and is that
+  // narrow.
   long long perm_rs = 0;
   int perm_div = 1;
+  const long long* cofs = nullptr;
   // Padded A rows.  apitch > 0: the A operand holds its panel rows (m, y) at
   // R' = m * apitch + y (apitch a multiple of 32, so every 32-row block is
   // one AO function m and one group of 32 auxiliary indices); the tile's
   // row r is R' = arow0 + r, rows with y >= ay_valid are padding.  Every
   // row-indexed output then uses the unpadded row R = m * ay_valid + y: the
-  // row-major `out` points at unpadded row arow0, emax/out2/perm take R.
+  // row-major `out` points at unpadded row arow0, emax/out2/iout take R.
   int apitch = 0, arow0 = 0, ay_valid = 0;
   // Half transform with digit output (k_split_gemm<true, false>): the
   // tile's rows are (m, y) of one panel, its columns i orbitals.  Instead
@@ -123,7 +136,7 @@ struct SplitItem {
   // mu = hrow0 + m into `hdig` (h_nrb row blocks, 64-byte swizzled images,
   // k-tile g * seg_nkt + i for auxiliary group g = y / 32, k = y % 32 in it)
   // with one exponent per (mu, g), eseg[mu * es_ld + g], and the maximum
-  // over g into emax (biased, atomicMax).
+  // over g into emax (atomicMax).
   uint16_t* hdig = nullptr;
   int h_nrb = 0, hrow0 = 0;
   int* eseg = nullptr;
@@ -335,9 +348,7 @@ __device__ __forceinline__ long long shr_round(long long x, int sh) {
 // ------------------------------------------------------------ split kernels
 // A split job fills rows [row0, row0 + nrows) of one digit operand:
 // element (r, c) = src[(r - row0)*rs + c*cs] for c < ncols, zero for
-// ncols <= c < nkt*32.  Row exponents are e[r] (e_biased != 0: e holds the
-// maximum biased FP64 exponent of the row, 0 for an all-zero row).  Slice
-// images go to dst as [kt][s][rb][1024]; rows outside every job stay as
+// ncols <= c < nkt*32.  Row exponents are e[r].  Slice images go to dst as [kt][s][rb][1024]; rows outside every job stay as
 // allocated (zero).
 struct SplitJob {
   const double* src;
@@ -345,7 +356,6 @@ struct SplitJob {
   int row0, nrows;
   long long ncols;
   int* e;
-  int e_biased;
   int nrb, nkt;
   uint16_t* dst;
 };
@@ -375,16 +385,10 @@ __global__ void k_fill_int(int* __restrict__ p, long long n, int v) {
     p[i] = v;
 }
 
-// Biased FP64 exponent maxima (0 = all zero) -> row exponents in place.
-__global__ void k_exp_unbias(int* __restrict__ e, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) e[i] = e[i] == 0 ? -2000 : e[i] - 1022;
-}
-
 // Zero the auxiliary slots y0 <= y' < 32 of the last 32-index group of every
-// row of a column-pair-outermost H (SplitItem::perm_rs): rows of rs doubles,
+// row of a column-pair-outermost H (SplitItem::iout): rows of rs elements,
 // the group starting at column gbase, npairs column pairs.  Grid-stride.
-__global__ void k_zero_hpad(double* __restrict__ H, int nrows, long long rs, long long gbase,
+__global__ void k_zero_hpad(long long* __restrict__ H, int nrows, long long rs, long long gbase,
                             int y0, int npairs) {
   const int ny = 32 - y0;
   const long long per_row = (long long)npairs * ny;
@@ -394,8 +398,15 @@ __global__ void k_zero_hpad(double* __restrict__ H, int nrows, long long rs, lon
     const long long r = i / per_row, t = i - r * per_row;
     const long long p = t / ny;
     const int yy = y0 + (int)(t - p * ny);
-    *reinterpret_cast<double2*>(H + r * rs + gbase + p * 64 + yy * 2) = make_double2(0.0, 0.0);
+    *reinterpret_cast<longlong2*>(H + r * rs + gbase + p * 64 + yy * 2) = make_longlong2(0, 0);
   }
+}
+
+// x >> sh for any sh >= 0 (PTX clamps: 0 from 64 on)
+__device__ __forceinline__ unsigned long long shr_u64(unsigned long long x, int sh) {
+  unsigned long long r;
+  asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(sh));
+  return r;
 }
 
 __device__ __forceinline__ uint16_t small_int_to_bf16(int d) {
@@ -403,6 +414,40 @@ __device__ __forceinline__ uint16_t small_int_to_bf16(int d) {
   // (exact: |d| <= 128 needs at most 8 significant bits)
   const float f = __int_as_float(0x4B400000 + d) - 12582912.0f;
   return (uint16_t)(__float_as_uint(f) >> 16);
+}
+
+// The five digit slices of eight elements sign * X (X <= 2^39, one k run of
+// a row) as BF16, 16 bytes per slice at p + s * sstride.  A digit byte u of
+// X + 0x80808080 becomes the float 2^23 + u by one byte permute, d = u - 128
+// by one subtraction, and its upper half is the exact BF16; the sign is set
+// in the packed pairs (a zero digit may be -0).
+__device__ __forceinline__ void store_digits8(const unsigned long long (&X)[8], const bool (&neg)[8],
+                                              uint16_t* p, long long sstride) {
+  uint32_t lo[8], hi[8], sgn[4];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const unsigned long long T = X[j] + 0x80808080ull;
+    lo[j] = (uint32_t)T;
+    hi[j] = (uint32_t)(T >> 32);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    sgn[j] = (neg[2 * j] ? 0x8000u : 0u) | (neg[2 * j + 1] ? 0x80000000u : 0u);
+#pragma unroll
+  for (int s = 0; s < kSlices; ++s) {
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float f[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        f[h] = s == 0 ? __uint_as_float(0x4B000000u | hi[2 * j + h]) - 8388608.0f
+                      : __uint_as_float(__byte_perm(lo[2 * j + h], 0x4B000000u, 0x7440 | (4 - s))) -
+                            8388736.0f;
+      o[j] = __byte_perm(__float_as_uint(f[0]), __float_as_uint(f[1]), 0x7632) ^ sgn[j];
+    }
+    *reinterpret_cast<uint4*>(p + s * sstride) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
 }
 
 // Slice images.  One warp per (8-row group, k-tile): lane (rr, kc) =
@@ -419,53 +464,156 @@ __global__ void k_split_tiles(const SplitJob* __restrict__ jobs) {
   const int rr = lane & 7, kc = lane >> 3;
   const int r = 8 * g + rr;
   if (r < jb.row0 || r >= jb.row0 + jb.nrows) return;
-  int er = jb.e[r];
-  if (jb.e_biased) er = er == 0 ? -2000 : er - 1022;
+  const int er = jb.e[r];
   const double* src = jb.src + (long long)(r - jb.row0) * jb.rs;
-  uint16_t out[kSlices][8];
+  unsigned long long X[8];
+  bool neg[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const long long c = (long long)kt * 32 + kc * 8 + j;
     const double x = c < jb.ncols ? src[c * jb.cs] : 0.0;
     const unsigned long long u = (unsigned long long)__double_as_longlong(x);
     const int E = (int)((u >> 52) & 0x7FF);
-    unsigned long long X = 0;
-    if (E != 0 && er > -2000) {
-      const unsigned long long m = (u & ((1ull << 52) - 1)) | (1ull << 52);
-      const int sh = 1036 + er - E;  // X = rint(m / 2^sh); sh >= 14 since |x| < 2^er
-      if (sh < 64) X = (m + (1ull << (sh - 1))) >> sh;
+    const unsigned long long m = (u & ((1ull << 52) - 1)) | (1ull << 52);
+    // X = rint(m / 2^sh); sh >= 14 since |x| < 2^er
+    X[j] = E != 0 && er > -2000 ? (shr_u64(m, 1035 + er - E) + 1) >> 1 : 0;
+    neg[j] = (u >> 63) != 0;
+  }
+  store_digits8(X, neg,
+                jb.dst + ((long long)kt * kSlices * jb.nrb + (r >> 5)) * kImage +
+                    ((r & 31) >> 3) * 256 + kc * 64 + rr * 8,
+                (long long)jb.nrb * kImage);
+}
+
+// Digit slices of an operand whose elements are the integers V of a split
+// GEMM (SplitItem::iout): row r, flat k index in the column-pair-outermost
+// order of ny indices y and ld columns c, value V 2^(ea[ea_off[r] + y] +
+// eb[eb_off[r] + c] - 46).  e[r]: the row's exponent, |value| <= 2^e[r]
+// (-2000: all zero).  dst as in SplitJob; rows start at 0.
+struct SplitIntJob {
+  const long long* src;
+  long long rs, ncols;
+  long long gs;  // elements from one group of 32 y to the next in a row of src
+  int nrows, ny, ld;
+  const int* e;
+  const int* ea;
+  const long long* ea_off;
+  const int* eb;
+  const long long* eb_off;
+  int nrb, nkt;
+  uint16_t* dst;
+};
+
+// One warp per (8-row group, k-tile), lanes as in k_split_tiles.  Bound by
+// HBM (8 bytes in, 10 out per element).  kFull: ny is a multiple of 32 (every
+// group of y is whole), so a lane's eight elements are four y of one column
+// pair; otherwise ny is even and they are two runs of two y.  grid
+// (warps/8, njobs).
+constexpr int kMaxIntJobs = 16;
+struct SplitIntJobs {
+  SplitIntJob j[kMaxIntJobs];
+};
+template <bool kFull>
+__global__ void k_split_ints(const __grid_constant__ SplitIntJobs jobs) {
+  const SplitIntJob& jb = jobs.j[blockIdx.y];
+  const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  const int ng = (jb.nrows + 7) >> 3;
+  if (wid >= (long long)ng * jb.nkt) return;
+  const int g = (int)(wid % ng), kt = (int)(wid / ng);
+  const int rr = lane & 7, kc = lane >> 3;
+  const int r = 8 * g + rr;
+  if (r >= jb.nrows) return;
+  const long long k0 = (long long)kt * 32 + kc * 8;
+  const int er = jb.e[r];
+  const int base = er + 7;  // X = |V| 2^(39 - e + ea + eb - 46)
+  const long long* src = jb.src + (long long)r * jb.rs;
+  const int* ea = jb.ea + jb.ea_off[r];
+  const int* eb = jb.eb + jb.eb_off[r];
+  long long v[8];
+  int sh[8];
+  if (er <= -2000 || k0 >= jb.ncols) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = 0;
+      sh[j] = 0;
     }
-    const bool neg = (u >> 63) != 0;
-    const unsigned long long T = X + 0x80808080ull;
-    int dgt[5];
+  } else if constexpr (kFull) {
+    // ncols is a multiple of 8
+    const int per = 32 * jb.ld, k = (int)k0;
+    const int G = k / per, rem = k - G * per;
+    src += G * jb.gs + rem;
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) dgt[jj] = (int)((T >> (8 * jj)) & 255) - 128;
-    dgt[4] = (int)(T >> 32);
+    for (int j = 0; j < 4; ++j) {
+      const longlong2 t = *reinterpret_cast<const longlong2*>(src + 2 * j);
+      v[2 * j] = t.x;
+      v[2 * j + 1] = t.y;
+    }
+    const int4 y = *reinterpret_cast<const int4*>(ea + 32 * G + ((rem & 63) >> 1));
+    const int2 c = *reinterpret_cast<const int2*>(eb + 2 * (rem >> 6));
+    const int b0 = base - c.x, b1 = base - c.y;
+    sh[0] = b0 - y.x;
+    sh[1] = b1 - y.x;
+    sh[2] = b0 - y.y;
+    sh[3] = b1 - y.y;
+    sh[4] = b0 - y.z;
+    sh[5] = b1 - y.z;
+    sh[6] = b0 - y.w;
+    sh[7] = b1 - y.w;
+  } else {
+    const int per = 32 * jb.ld;
 #pragma unroll
-    for (int s = 0; s < kSlices; ++s) {
-      const int d = dgt[4 - s];
-      out[s][j] = small_int_to_bf16(neg ? -d : d);
+    for (int h = 0; h < 2; ++h) {
+      const int k = (int)k0 + 4 * h;
+      const bool in = k < jb.ncols;  // ncols is a multiple of 4
+      const int G = k / per, rem = k - G * per;
+      const int ng2 = 2 * max(2, min(32, jb.ny - 32 * G));
+      const int p = rem / ng2, s = rem - p * ng2;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v[4 * h + j] = in ? src[G * jb.gs + rem + j] : 0ll;
+        sh[4 * h + j] = in ? base - ea[32 * G + (s >> 1) + (j >> 1)] - eb[2 * p + (j & 1)] : 0;
+      }
     }
   }
-  const int rb = r >> 5;
-  const long long off_in = (long long)((r & 31) >> 3) * 256 + kc * 64 + rr * 8;
+  unsigned long long X[8];
+  bool neg[8];
+  int shmin = sh[0];
 #pragma unroll
-  for (int s = 0; s < kSlices; ++s) {
-    uint16_t* p = jb.dst + (((long long)kt * kSlices + s) * jb.nrb + rb) * kImage + off_in;
-    uint4 v;
-    v.x = (uint32_t)out[s][0] | ((uint32_t)out[s][1] << 16);
-    v.y = (uint32_t)out[s][2] | ((uint32_t)out[s][3] << 16);
-    v.z = (uint32_t)out[s][4] | ((uint32_t)out[s][5] << 16);
-    v.w = (uint32_t)out[s][6] | ((uint32_t)out[s][7] << 16);
-    *reinterpret_cast<uint4*>(p) = v;
+  for (int j = 1; j < 8; ++j) shmin = min(shmin, sh[j]);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    neg[j] = v[j] < 0;
+    X[j] = neg[j] ? (unsigned long long)(-v[j]) : (unsigned long long)v[j];
   }
+  // rint(a 2^-sh) as (a 2^-(sh-1) + 1) / 2; only results far below their
+  // operands' exponents (cancellation) shift left
+  if (shmin >= 1) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) X[j] = (shr_u64(X[j], sh[j] - 1) + 1) >> 1;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      X[j] = sh[j] >= 1 ? (shr_u64(X[j], sh[j] - 1) + 1) >> 1 : X[j] << min(-sh[j], 63);
+  }
+  store_digits8(X, neg,
+                jb.dst + ((long long)kt * kSlices * jb.nrb + (r >> 5)) * kImage +
+                    ((r & 31) >> 3) * 256 + kc * 64 + rr * 8,
+                (long long)jb.nrb * kImage);
 }
 
 // ------------------------------------------------------------ the GEMM
 // Pairs (s, t) are issued exact diagonals first (d = 0, 1, 2), then d = 3, 4;
 // the accumulator of diagonal d sits at TMEM column d * kTileN.
 //
-// Variants.  kHDigits: the half transform writes H as digit slices
+// Variants.  kOutInt*: the half transform leaves its results as the integers V
+// of the number format (SplitItem::iout); the digits of the next operand are
+// cut from them by k_split_ints.  What bounds a half transform of short k
+// ranges is the epilogue's store phase (FP64 conversions on GB300's narrow
+// FP64 pipe, exponents, selects), and V needs none of it: 1.25 -> 0.80 ms for
+// a batch of the synthetic tensor at nbf 1200, nocc 180 (four k-tiles), 158 ->
+// 149 us for C10H22; C20H42 (ten k-tiles) stays at 0.73 ms, its HBM stream.
+// kHDigits: the half transform writes H as digit slices
 // (SplitItem::hdig) with one exponent per (AO function, auxiliary group)
 // instead of FP64 values.  kSeg: the exchange over such digits; its
 // operands are 64-byte swizzled and its k range is cut into segments of
@@ -477,7 +625,15 @@ __global__ void k_split_tiles(const SplitJob* __restrict__ jobs) {
 // rounding (exact while that shift is at most 16 for a chunk, 0 for a
 // fold).  Without kSeg there is one segment per item and no shift.
 
-template <bool kHDigits, bool kSeg>
+enum SplitOut {
+  kOutF64 = 0,     // FP64, row-major
+  kOutF64Cols,     // FP64, column c at cofs[c]
+  kOutInt,         // integers (density columns in FP64 to out2)
+  kOutIntTwo,      // integers, two sets of row exponents (csplit)
+  kOutIntRagged,   // integers, the last group of 32 y as wide as what is left
+};
+
+template <bool kHDigits, bool kSeg, int kOut>
 __global__ void __launch_bounds__(kThreads, 1)
     k_split_gemm(const SplitItem* __restrict__ items, int nitems, int* __restrict__ err,
                  int stop_item, unsigned long long spin_ns) {
@@ -873,7 +1029,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int gy = yrow >> 5;
         if (third == 0 && lane == 0 && rin) {
           w.eseg[(long long)mu * w.es_ld + gy] = eg;
-          if (eg > -2000 && w.emax) atomicMax(w.emax + mloc, (unsigned int)max(1, eg + 1022));
+          if (eg > -2000 && w.emax) atomicMax(w.emax + mloc, eg);
         }
         if (rin) {
           // digit slices of X = rint(|value| 2^(39-eg)) (see the number
@@ -905,61 +1061,115 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       } else {
-        unsigned int emax_row = 0;
-        {
-          const bool perm = perm_rs != 0;
-          double* orow;
-          if (perm) {
+        constexpr int kNone = -100000;
+        int e_row = kNone;  // exponent of this thread's kept results
+        constexpr bool kInt = kOut >= kOutInt;
+        if constexpr (kInt) {
+          // columns kept by this warp; a row's exponent is that of
+          // max_c |V_c| 2^eb[c]: OR the magnitudes, each shifted to the
+          // largest column exponent (`any` keeps a nonzero row nonzero).
+          // Columns from cs on belong to the second set of exponents.
+          const int nv = min(max(nstore - cbase, 0), kEpiCols);
+          const int cs = kOut == kOutIntTwo ? min(max(w.csplit - cbase, 0), kEpiCols) : kEpiCols;
+          const int ecm0 = __reduce_max_sync(0xffffffffu, lane < min(nv, cs) ? ecl : kNone);
+          int ecm1 = kNone;
+          if constexpr (kOut == kOutIntTwo)
+            ecm1 = __reduce_max_sync(0xffffffffu, lane < nv && lane >= cs ? ecl : kNone);
+          const int shl = min((lane < cs ? ecm0 : ecm1) - ecl, 63);
+          long long* orow;
+          int pstep = 64;
+          {
             const int m = R / perm_div, y = R - m * perm_div;
-            orow = out + (long long)m * perm_rs + (long long)(y & ~31) * ldr +
-                   ((y & 31) * 2 + (cbase >> 1) * 64);
-          } else {
-            orow = out + rofs * ldr + cbase;
+            if constexpr (kOut == kOutIntRagged) pstep = 2 * min(32, perm_div - (y & ~31));
+            orow = w.iout + (long long)m * perm_rs + (long long)(y & ~31) * ldr + (y & 31) * 2 +
+                   (long long)((c0 + cbase) >> 1) * pstep;
           }
-          const bool vec = ((uintptr_t)orow & 15) == 0;
+          unsigned long long mag0 = 0, mag1 = 0;
+          unsigned int any0 = 0, any1 = 0;
+#pragma unroll
+          for (int c = 0; c < kEpiCols; c += 2) {
+            if (c >= nv) continue;  // the same for the whole warp
+            const int sh0 = __shfl_sync(0xffffffffu, shl, c);
+            const int sh1 = __shfl_sync(0xffffffffu, shl, c + 1);
+            const long long v0 = V[c];
+            // the pair's second column is the zero pad column when the
+            // number of kept columns is odd
+            const long long v1 = c + 1 < nv ? V[c + 1] : 0ll;
+            const unsigned long long m0 = (unsigned long long)(v0 ^ (v0 >> 63));
+            const unsigned long long m1 = (unsigned long long)(v1 ^ (v1 >> 63));
+            const unsigned long long mg = (m0 >> sh0) | (m1 >> (c + 1 < nv ? sh1 : 63));
+            const unsigned int an = (unsigned int)v0 | (unsigned int)(v0 >> 32) |
+                                    (unsigned int)v1 | (unsigned int)(v1 >> 32);
+            if (kOut != kOutIntTwo || c < cs) {
+              mag0 |= mg;
+              any0 |= an;
+            } else {
+              mag1 |= mg;
+              any1 |= an;
+            }
+            if (rvalid)
+              *reinterpret_cast<longlong2*>(orow + (c >> 1) * pstep) = make_longlong2(v0, v1);
+          }
+          // |x| <= 2^e, e = bit length + er + ecm - 46
+          if (rvalid && any0)
+            e_row = (mag0 ? 64 - __clzll((long long)mag0) : 1) + er + ecm0 - 46;
+          if constexpr (kOut == kOutIntTwo) {
+            // the padded A rows make a warp's 32 rows one AO function
+            const int m = __reduce_max_sync(
+                0xffffffffu,
+                rvalid && any1 ? (mag1 ? 64 - __clzll((long long)mag1) : 1) + er + ecm1 - 46
+                               : kNone);
+            if (lane == 0 && m > kNone) atomicMax(w.emax2 + R / emax_div, m);
+          }
+          // the density column of this warp's AO function, in FP64
+          const int dc = dcol - cbase;
+          if (kOut == kOutInt && dcol >= 0 && dc >= 0 && dc < kEpiCols) {
+            long long v = 0;
+#pragma unroll
+            for (int c = 0; c < kEpiCols; ++c) v = c == dc ? V[c] : v;
+            const int ec = w.eb[cbase + dc];
+            if (rvalid)
+              out2[R] = (er <= -2000 || ec <= -2000) ? 0.0 : i64_scaled_to_f64(v, er + ec - 46);
+          }
+        } else {
+          double* const rowp = out + rofs * ldr;
+          const bool vec = ((uintptr_t)rowp & 15) == 0;
 #pragma unroll
           for (int c = 0; c < kEpiCols; c += 2) {
             const int ecs0 = __shfl_sync(0xffffffffu, ecl, c);
             const int ecs1 = __shfl_sync(0xffffffffu, ecl, c + 1);
             const int col = cbase + c;
             const bool s0 = rvalid && col < nstore, s1 = rvalid && col + 1 < nstore;
-            const bool d0 = rvalid && col == dcol, d1 = rvalid && col + 1 == dcol;
-            if (!(s0 || s1 || d0 || d1)) continue;
-            const int ec0 = (s0 || d0) ? ecs0 : -2000;
-            const int ec1 = (s1 || d1) ? ecs1 : -2000;
+            if (!(s0 || s1)) continue;
+            const int ec0 = s0 ? ecs0 : -2000;
+            const int ec1 = s1 ? ecs1 : -2000;
             const double x0 =
                 (er <= -2000 || ec0 <= -2000) ? 0.0 : i64_scaled_to_f64(V[c], er + ec0 - 46);
             const double x1 =
                 (er <= -2000 || ec1 <= -2000) ? 0.0 : i64_scaled_to_f64(V[c + 1], er + ec1 - 46);
-            if (d0) out2[R] = x0;
-            if (d1) out2[R] = x1;
-            if (s0) emax_row = max(emax_row, (unsigned int)((__double_as_longlong(x0) >> 52) & 0x7FF));
-            if (s1) emax_row = max(emax_row, (unsigned int)((__double_as_longlong(x1) >> 52) & 0x7FF));
-            if (perm) {
-              // the pair's second column is the zero pad column when nstore
-              // is odd (the last orbital of an odd count)
-              if (s0)
-                *reinterpret_cast<double2*>(orow + (c >> 1) * 64) = make_double2(x0, s1 ? x1 : 0.0);
-            } else if (vec && s0 && s1) {
-              *reinterpret_cast<double2*>(orow + c) = make_double2(x0, x1);
+            const int E0 = (int)((__double_as_longlong(x0) >> 52) & 0x7FF);
+            const int E1 = (int)((__double_as_longlong(x1) >> 52) & 0x7FF);
+            if (s0 && E0) e_row = max(e_row, E0 - 1022);
+            if (s1 && E1) e_row = max(e_row, E1 - 1022);
+            double* const o =
+                rowp + (kOut == kOutF64Cols ? __ldg(w.cofs + col) : (long long)col);
+            if (vec && s0 && s1) {
+              *reinterpret_cast<double2*>(o) = make_double2(x0, x1);
             } else {
-              if (s0) orow[c] = x0;
-              if (s1) orow[c + 1] = x1;
+              if (s0) o[0] = x0;
+              if (s1) o[1] = x1;
             }
           }
         }
-        if (unsigned int* const emaxp = w.emax) {
+        if (int* const emaxp = w.emax) {
           // one atomic per warp when all its rows map to the same target row
           const int target = rvalid ? R / emax_div : -1;
           const int t0 = __shfl_sync(0xffffffffu, target, 0);
-          const bool same = __all_sync(0xffffffffu, target == t0);
-          if (same) {
-            unsigned int m = emax_row;
-#pragma unroll
-            for (int o2 = 16; o2 > 0; o2 >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o2));
-            if (lane == 0 && t0 >= 0 && m) atomicMax(emaxp + t0, m);
-          } else if (target >= 0 && emax_row) {
-            atomicMax(emaxp + target, emax_row);
+          if (__all_sync(0xffffffffu, target == t0 || target < 0)) {
+            const int m = __reduce_max_sync(0xffffffffu, e_row);
+            if (lane == 0 && t0 >= 0 && m > kNone) atomicMax(emaxp + t0, m);
+          } else if (target >= 0 && e_row > kNone) {
+            atomicMax(emaxp + target, e_row);
           }
         }
       }

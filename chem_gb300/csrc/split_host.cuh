@@ -76,7 +76,7 @@ struct SplitState {
   std::vector<long long> c_off;
   int c_nrb = 0;
   int* d_eC = nullptr;
-  double* d_H = nullptr;
+  long long* d_H = nullptr;  // integers of the half transform (SplitItem::iout)
   uint16_t* d_Hslices = nullptr;
   int h_nrb = 0, h_nkt = 0, hld = 0;
   int* d_eH = nullptr;
@@ -89,7 +89,9 @@ struct SplitState {
   int maxb = 0;
   SplitItem* d_items = nullptr;
   int ht_nitems = 0, k_nitems = 0;
-  SplitJob* d_jobs = nullptr;  // [0,nblk): C rows, [nblk,2nblk): P rows, [2nblk]: H
+  SplitJob* d_jobs = nullptr;  // [0,nblk): C rows, [nblk,2nblk): P rows
+  std::vector<SplitIntJob> hjobs;  // digits of H, one per distinct batch size
+  long long* d_eoff = nullptr;     // their exponent offsets per AO function
   int c_maxthreads = 0, c_maxrows = 0;
   long long h_threads = 0;
   int* d_err = nullptr;
@@ -162,6 +164,7 @@ struct SplitState {
     free_(&d_dt);
     free_(&d_items);
     free_(&d_jobs);
+    free_(&d_eoff);
     plans.clear();
     nocc = -1;
   }
@@ -237,21 +240,35 @@ struct SplitState {
   };
 
   static int cdiv_(long long a, long long b) { return (int)((a + b - 1) / b); }
+  // digits of operands left as integers by a split GEMM
+  template <bool kFull>
+  static void launch_ints(cudaStream_t st, const SplitIntJob* jobs, int n, int64_t* launches) {
+    for (int j0 = 0; j0 < n; j0 += kMaxIntJobs) {
+      const int m = std::min(kMaxIntJobs, n - j0);
+      SplitIntJobs p;
+      long long warps = 0;
+      for (int j = 0; j < m; ++j) {
+        p.j[j] = jobs[j0 + j];
+        warps = std::max(warps, (long long)cdiv_(p.j[j].nrows, 8) * p.j[j].nkt);
+      }
+      k_split_ints<kFull><<<dim3(cdiv_(warps, 8), m), 256, 0, st>>>(p);
+      (*launches)++;
+    }
+  }
   // H rows hold the half transform in groups of 32 auxiliary indices (the
   // column-pair-outermost layout of SplitItem::perm_rs), so a batch of xbc
   // auxiliary rows spans pad32(xbc) * hld columns of H
   static int pad32(int x) { return (x + 31) & ~31; }
 
-  // variant: 0 plain, 1 half transform with digit output, 2 segmented exchange
-  bool attr_v[3] = {false, false, false};
-  template <bool kH, bool kS>
+  bool attr_v[8] = {};
+  template <bool kH, bool kS, int kOut>
   gbjk_status launch_gemm_v(cudaStream_t st, SplitItem* items, int n, int64_t* launches,
                             std::string* err, int leave_sms) {
     if (n == 0) return GBJK_OK;
-    const int v = kH ? 1 : (kS ? 2 : 0);
+    const int v = kH ? 5 : (kS ? 6 : kOut);
     if (!attr_v[v]) {
-      if (cudaFuncSetAttribute(k_split_gemm<kH, kS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kSmemBytes) != cudaSuccess) {
+      if (cudaFuncSetAttribute(k_split_gemm<kH, kS, kOut>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess) {
         *err = "cannot reserve shared memory for the split GEMM";
         return GBJK_CUDA_ERROR;
       }
@@ -261,7 +278,8 @@ struct SplitState {
       attr_v[v] = true;
     }
     const int grid = std::min(n, std::max(1, nsm - leave_sms));
-    k_split_gemm<kH, kS><<<grid, kThreads, kSmemBytes, st>>>(items, n, d_err, stop_item, spin_ns);
+    k_split_gemm<kH, kS, kOut>
+        <<<grid, kThreads, kSmemBytes, st>>>(items, n, d_err, stop_item, spin_ns);
     (*launches)++;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -270,9 +288,10 @@ struct SplitState {
     }
     return GBJK_OK;
   }
+  template <int kOut = kOutF64>
   gbjk_status launch_gemm(cudaStream_t st, SplitItem* items, int n, int64_t* launches,
                           std::string* err, int leave_sms = 0) {
-    return launch_gemm_v<false, false>(st, items, n, launches, err, leave_sms);
+    return launch_gemm_v<false, false, kOut>(st, items, n, launches, err, leave_sms);
   }
 
   // --- once per tensor: the compact copy the mixed-path J reads ------------
@@ -397,6 +416,7 @@ struct SplitState {
     k_j_colsum_chunks<<<cdiv_(jcols, 128), 128, 0, st>>>(d_jpart, jnchunk, jcols, nbf, d_jmap, dJ);
     *launches += 2;
   }
+  size_t j_bytes() const { return (size_t)naux * jcols * 6; }
 
   // --- once per tensor: prefit and A-operand digits -----------------------
   gbjk_status prepare_b(cudaStream_t st, const double* d_B, const double* d_Linv,
@@ -511,7 +531,6 @@ struct SplitState {
           j.nrows = naux;
           j.ncols = panelK[I];
           j.e = d_eA + eA_off[I];
-          j.e_biased = 0;
           j.nrb = a_nrb[I];
           j.nkt = nkt[I];
           j.dst = d_Aslices + a_off[I];
@@ -547,7 +566,6 @@ struct SplitState {
             j.nrows = xbc;
             j.ncols = panelK[I];
             j.e = d_eA + eA_off[I];
-            j.e_biased = 0;
             j.nrb = a_nrb[I];
             j.nkt = nkt[I];
             j.dst = d_Aslices + a_off[I];
@@ -648,6 +666,7 @@ struct SplitState {
     if (alloc(&d_Cslices, (size_t)ctot) != cudaSuccess ||
         alloc(&d_eC, (size_t)nblk * c_nrb * 32) != cudaSuccess ||
         alloc(&d_H, nH) != cudaSuccess ||
+        alloc(&d_eoff, 2 * sizes.size() * nbf) != cudaSuccess ||
         alloc(&d_Hslices, (size_t)h_nrb * h_nkt * kSlices * kImage) != cudaSuccess ||
         alloc(&d_eH, (size_t)h_nrb * 32) != cudaSuccess ||
         alloc(&d_eHs, nEs) != cudaSuccess ||
@@ -669,6 +688,8 @@ struct SplitState {
         d_eHs, (long long)nEs, -2000);
     std::vector<SplitItem> items;
     std::vector<SplitJob> jobs(2 * nblk);
+    hjobs.clear();
+    std::vector<long long> eoff(2 * sizes.size() * nbf);
     plans.clear();
     for (size_t pi = 0; pi < sizes.size(); ++pi) {
       const int xbc = sizes[pi];
@@ -709,7 +730,8 @@ struct SplitState {
             } else {
               // column-pair-outermost layout: each epilogue store is one
               // contiguous 512-byte run (SplitItem::perm_rs)
-              w.out = d_H + (long long)boff[I] * pad32(xbc) * hld + (long long)nt * kTileN * 32;
+              w.out = nullptr;
+              w.iout = d_H + (long long)boff[I] * pad32(xbc) * hld;
               w.ldr = hld;
               w.perm_rs = (long long)pad32(xbc) * hld;
               w.perm_div = xbc;
@@ -717,7 +739,7 @@ struct SplitState {
             w.m_valid = (int)std::min<long long>(kTileM, rows - (long long)mt * kTileM);
             w.n_valid = std::min(kTileN, ncolI - nt * kTileN);
             // row (m, y) of panel I belongs to H row mu = boff[I] + m
-            w.emax = (unsigned int*)d_eH + boff[I];
+            w.emax = d_eH + boff[I];
             w.emax_row0 = mt * kTileM;
             w.emax_div = xbc;
             // density column m' = col - nocc: g-partial of row (m, Y) if m' == m
@@ -772,21 +794,31 @@ struct SplitState {
           }
       }
       pl.nk = (int)items.size() - pl.k0;
-      // digits of the half-transformed batch (exponents from the epilogue)
-      SplitJob hj;
+      // digits of the half-transformed batch (row exponents from the
+      // epilogue, element exponents from the two operands of the transform)
+      SplitIntJob hj;
       hj.src = d_H;
       hj.rs = (long long)pad32(xbc) * hld;
-      hj.cs = 1;
-      hj.row0 = 0;
+      hj.ncols = hj.rs;
+      hj.gs = 32LL * hld;
       hj.nrows = nbf;
-      hj.ncols = (long long)pad32(xbc) * hld;
+      hj.ny = pad32(xbc);
+      hj.ld = hld;
       hj.e = d_eH;
-      hj.e_biased = 0;
+      hj.ea = d_eA;
+      hj.ea_off = d_eoff + 2 * pi * nbf;
+      hj.eb = d_eC;
+      hj.eb_off = d_eoff + (2 * pi + 1) * nbf;
       hj.nrb = h_nrb;
       hj.nkt = nk_b;
       hj.dst = d_Hslices;
-      pl.hjob = (int)jobs.size();
-      jobs.push_back(hj);
+      for (int I = 0; I < nblk; ++I)
+        for (int m = 0; m < bsize[I]; ++m) {
+          eoff[2 * pi * nbf + boff[I] + m] = eA_off[I] + (long long)m * pad32(xbc);
+          eoff[(2 * pi + 1) * nbf + boff[I] + m] = (long long)I * c_nrb * 32;
+        }
+      pl.hjob = (int)hjobs.size();
+      hjobs.push_back(hj);
       plans.push_back(pl);
     }
     ht_nitems = plans[0].nht;
@@ -803,7 +835,6 @@ struct SplitState {
       pj.nrows = jfused ? bsize[I] : 0;
       pj.ncols = panelK[I];
       pj.e = d_eC + (long long)I * c_nrb * 32;
-      pj.e_biased = 0;
       pj.nrb = c_nrb;
       pj.nkt = nkt[I];
       pj.dst = d_Cslices + c_off[I];
@@ -815,7 +846,6 @@ struct SplitState {
       j.nrows = nocc_;
       j.ncols = panelK[I];
       j.e = d_eC + (long long)I * c_nrb * 32;
-      j.e_biased = 0;
       j.nrb = c_nrb;
       j.nkt = nkt[I];
       j.dst = d_Cslices + c_off[I];
@@ -827,6 +857,7 @@ struct SplitState {
       return GBJK_OOM;
     }
     cudaMemcpy(d_items, items.data(), items.size() * sizeof(SplitItem), cudaMemcpyHostToDevice);
+    cudaMemcpy(d_eoff, eoff.data(), eoff.size() * sizeof(long long), cudaMemcpyHostToDevice);
     host_jobs = jobs;
     jobs_cg = jobs_pg = nullptr;
     nocc = nocc_;
@@ -896,35 +927,29 @@ struct SplitState {
       {
         Scope sc(this, 0, st);
         // H row exponents are atomically maximised by the half-transform epilogue
-        if (cudaMemsetAsync(d_eH, 0, (size_t)h_nrb * 32 * sizeof(int), st) != cudaSuccess) {
+        if (cudaMemsetAsync(d_eH, kNoExpByte, (size_t)h_nrb * 32 * sizeof(int), st) !=
+            cudaSuccess) {
           *err = "split path: memset failed";
           return GBJK_CUDA_ERROR;
         }
         if (hfuse_eff)
-          s = launch_gemm_v<true, false>(st, d_items + pl.ht0, pl.nht, launches, err, 0);
+          s = launch_gemm_v<true, false, kOutF64>(st, d_items + pl.ht0, pl.nht, launches, err, 0);
         else
-          s = launch_gemm(st, d_items + pl.ht0, pl.nht, launches, err);
+          s = launch_gemm<kOutInt>(st, d_items + pl.ht0, pl.nht, launches, err);
         if (s) return s;
       }
       if (ev_ht && nbatch == 1 && cudaEventRecord(ev_ht, st) != cudaSuccess) {
         *err = "split path: event record failed";
         return GBJK_CUDA_ERROR;
       }
-      {
+      if (!hfuse_eff) {
         Scope sc(this, 2, st);
-        k_exp_unbias<<<cdiv_((long long)h_nrb * 32, 256), 256, 0, st>>>(d_eH, h_nrb * 32);
-        (*launches)++;
-        if (!hfuse_eff) {
-          const long long hthr =
-              (long long)(nbf / 8 + 2) * cdiv_((long long)pad32(pl.xbc) * hld, kTileK) * 32;
-          k_split_tiles<<<dim3(cdiv_(hthr, 256), 1), 256, 0, st>>>(d_jobs + pl.hjob);
-          (*launches)++;
-        }
+        launch_ints<true>(st, &hjobs[pl.hjob], 1, launches);
       }
       {
         Scope sc(this, 1, st);
         if (hfuse_eff)
-          s = launch_gemm_v<false, true>(st, d_items + pl.k0, pl.nk, launches, err, k_grid);
+          s = launch_gemm_v<false, true, kOutF64>(st, d_items + pl.k0, pl.nk, launches, err, k_grid);
         else
           s = launch_gemm(st, d_items + pl.k0, pl.nk, launches, err, k_grid);
         if (s) return s;

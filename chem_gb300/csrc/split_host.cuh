@@ -633,7 +633,10 @@ struct SplitState {
       ctot += (long long)c_nrb * nkt[I] * kSlices * kImage;
     }
     hld = nocc_ + (nocc_ & 1);  // even row stride: 16-byte aligned pairs
-    hfuse_eff = hfuse;
+    // one exponent per (AO function, auxiliary group) needs all of a row's
+    // columns in one tile: with more, the tiles' exponents would overwrite each
+    // other
+    hfuse_eff = hfuse && ntn == 1;
     const bool fuse = hfuse_eff;
     es_ld = apitch / 32;  // auxiliary groups of a full batch
     const long long hk = (long long)pad32(xb) * hld;

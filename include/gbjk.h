@@ -167,8 +167,9 @@ int gbjk_get_overlap(const gbjk_ctx* ctx);
 /* Mixed-precision exchange: 1 cuts the digit slices of the half transform
  * H = (L^-1 B) C in the half-transform epilogue, with one exponent per AO
  * function and group of 32 auxiliary indices, and the exchange GEMM applies
- * those exponents per k segment; 0 (default) writes H in FP64 and cuts its
- * digits in a separate pass with one exponent per AO function.  Both stay
+ * those exponents per k segment, as long as the occupied and density columns
+ * fit one 96-wide tile; 0 (default), and wider problems, leave H for a separate
+ * digit pass with one exponent per AO function.  Both stay
  * within the split path's accuracy bound; their results differ in the last
  * bits.  No counterpart in the reference. */
 gbjk_status gbjk_set_split_fuse(gbjk_ctx* ctx, int on);

@@ -2264,15 +2264,21 @@ gbjk_status gbjk_mp2_set_factors(gbjk_ctx* ctx, int npts, const int* rank_o,
     if (rank_o[t] < 1 || rank_o[t] > ctx->nbf || rank_v[t] < 1 || rank_v[t] > ctx->nbf)
       return fail(ctx, GBJK_INVALID_ARG, "gbjk_mp2_set_factors: rank out of range [1, nbf]");
   }
-  if (!ctx->split.b_ready &&
-      (s = ctx->split.prepare_b(ctx->stream, ctx->d_B, ctx->d_Linv, &ctx->launches, &ctx->err)))
-    return s;
   Mp2State& m = ctx->mp2;
+  if (ctx->precision == GBJK_FP64) {
+    if ((s = m.prefit_fp64(ctx->stream, ctx->d_B, ctx->d_Linv, ctx->nnz, ctx->split,
+                           &ctx->launches, &ctx->err)))
+      return s;
+  } else if (!ctx->split.b_ready &&
+             (s = ctx->split.prepare_b(ctx->stream, ctx->d_B, ctx->d_Linv, &ctx->launches,
+                                       &ctx->err))) {
+    return s;
+  }
   bool same = m.ready && m.precision == ctx->precision && m.npts == npts;
   for (int t = 0; same && t < npts; ++t) same = m.ro[t] == rank_o[t] && m.rv[t] == rank_v[t];
   if (!same && (s = m.plan(ctx->stream, ctx->precision, npts, rank_o, rank_v, ctx->nbf, ctx->naux,
                            ctx->nblk, ctx->ncols_total, ctx->bsize, ctx->boff, ctx->panelK,
-                           ctx->cmoff, ctx->panel_off, ctx->split, &ctx->err)))
+                           ctx->cmoff, ctx->panel_off, ctx->d_B, ctx->split, &ctx->err)))
     return s;
   return m.upload(ctx->stream, ctx->nbf, Lo, Lv, &ctx->err);
 }
@@ -2320,7 +2326,7 @@ gbjk_status gbjk_mp2_release(gbjk_ctx* ctx) {
   if (!ctx) return GBJK_INVALID_ARG;
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
-  ctx->mp2.release();
+  ctx->mp2.release_plan();
   return GBJK_OK;
 }
 

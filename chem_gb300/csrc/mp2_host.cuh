@@ -1,7 +1,8 @@
 // Host side of the SOS-AO-MP2 Laplace batch: megalochem's ll_full Z builder
 // (src/mp/z_full.cpp:427-620) for every quadrature point of the Laplace
 // loop (src/mp/mp_compute.cpp:232-382) in one pass, on the prefitted tensor
-// Bfit = L^-1 B that the J/K engine keeps resident.
+// Bfit = L^-1 B (split path: the J/K engine's; FP64 path: its own, in the
+// oracle's order).
 //
 // Per point t (occupied factor Lo_t, nbf x r_t; virtual factor Lv_t,
 // nbf x rv_t; both zero-padded to the common strides hld, vld):
@@ -39,6 +40,10 @@ struct Mp2State {
   double *d_Lo = nullptr, *d_Lv = nullptr, *d_Cg = nullptr;
   double *d_H = nullptr, *d_W = nullptr, *d_Z = nullptr, *d_rsq = nullptr, *d_E = nullptr;
   long long cg_stride = 0, h_stride = 0, w_stride = 0;
+  // FP64 path: L^-1 B in the oracle's summation order (kept over plans until
+  // the tensor or the metric changes)
+  double* d_Bfit64 = nullptr;
+  size_t bfit_bytes = 0;
   // FP64 plan
   GemmGroup* d_groups = nullptr;
   GemmTile* d_tiles = nullptr;
@@ -79,6 +84,11 @@ struct Mp2State {
     *p = nullptr;
   }
   void release() {
+    release_plan();
+    free_(&d_Bfit64);
+    bfit_bytes = bytes = 0;
+  }
+  void release_plan() {
     free_(&d_Lo);
     free_(&d_Lv);
     free_(&d_Cg);
@@ -103,7 +113,7 @@ struct Mp2State {
     free_(&d_cofs);
     free_(&d_eoff);
     resolve();
-    bytes = 0;
+    bytes = bfit_bytes;
     npts = 0;
     precision = -1;
     ready = have_result = false;
@@ -159,15 +169,36 @@ struct Mp2State {
 
   static int cdiv_(long long a, long long b) { return (int)((a + b - 1) / b); }
 
+  // --- FP64 path: the prefit, once per tensor ---------------------------------
+  gbjk_status prefit_fp64(cudaStream_t st, const double* d_B, const double* d_Linv,
+                          long long nnz, SplitState& sp, int64_t* launches, std::string* err) {
+    if (sp.fitted || d_Bfit64) return GBJK_OK;
+    double* p = nullptr;
+    const size_t b0 = bytes;
+    if (alloc(&p, (size_t)nnz) != cudaSuccess) {
+      *err = "MP2 batch: out of memory for the prefitted tensor";
+      return GBJK_OOM;
+    }
+    gbjk_status s = sp.prefit_fp64(st, d_B, d_Linv, p, launches, err);
+    if (s) {
+      free_(&p);
+      bytes = b0;
+      return s;
+    }
+    d_Bfit64 = p;
+    bfit_bytes = bytes - b0;
+    return GBJK_OK;
+  }
+
   // --- plan -------------------------------------------------------------------
-  // Layout arguments are the J/K engine's (host copies); `sp` holds the
-  // prefitted tensor and, for the split path, its A-operand digits.
+  // Layout arguments are the J/K engine's (host copies); for the split path
+  // `sp` holds the A-operand digits of the prefitted tensor.
   gbjk_status plan(cudaStream_t st, int prec, int npts_, const int* ro_, const int* rv_, int nbf,
                    int naux, int nblk, int ncols_total, const std::vector<int>& bsize,
                    const std::vector<int>& boff, const std::vector<int>& panelK,
                    const std::vector<int>& cmoff, const std::vector<long long>& panel_off,
-                   SplitState& sp, std::string* err) {
-    release();
+                   const double* d_B, SplitState& sp, std::string* err) {
+    release_plan();
     npts = npts_;
     ro.assign(ro_, ro_ + npts);
     rv.assign(rv_, rv_ + npts);
@@ -190,7 +221,7 @@ struct Mp2State {
         alloc(&d_rsq, (size_t)npts * naux) || alloc(&d_E, (size_t)npts) ||
         cudaMemsetAsync(d_H, 0, (size_t)npts * h_stride * 8, st) ||
         cudaMemsetAsync(d_W, 0, (size_t)npts * w_stride * 8, st)) {
-      release();
+      release_plan();
       *err = "MP2 batch: out of device memory for the transforms";
       return GBJK_OOM;
     }
@@ -198,13 +229,13 @@ struct Mp2State {
     gbjk_status s = prec == GBJK_SPLIT_BF16
                         ? plan_split(st, nbf, naux, nblk, bsize, boff, panelK, cmoff, sp, err)
                         : plan_fp64(nbf, naux, nblk, bsize, boff, panelK, cmoff, panel_off,
-                                    sp.Bfit, err);
+                                    sp.fitted ? d_B : d_Bfit64, err);
     if (s) {
-      release();
+      release_plan();
       return s;
     }
     if (cudaStreamSynchronize(st) != cudaSuccess) {
-      release();
+      release_plan();
       *err = "MP2 batch: plan upload failed";
       return GBJK_CUDA_ERROR;
     }

@@ -2,8 +2,8 @@
 // plans.
 //
 // Once per tensor upload:
-//   Bfit = L^-1 B per panel row block (FP64 grouped GEMM, temporary), its row
-//   exponents and slice images (the A operands of the half transform).
+//   Bfit = L^-1 B (prefit_gemm.cuh, to FP64 accuracy on the tensor cores), its
+//   row exponents and slice images (the A operands of the half transform).
 // Per nocc: buffers and the two work lists (half transform, exchange).
 // Per build (stream-ordered, no host sync):
 //   C digits (B operand of every panel) -> split GEMM Hfit = Bfit C (FP64,
@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "kernels_fp64.cuh"
+#include "prefit_gemm.cuh"
 #include "split_gemm.cuh"
 
 namespace gbjk {
@@ -294,6 +295,148 @@ struct SplitState {
     return launch_gemm_v<false, false, kOut>(st, items, n, launches, err, leave_sms);
   }
 
+  // --- once per tensor: Bfit = L^-1 B ----------------------------------------
+  // On the FP64 pipe, each element the in-order fma chain of the oracle's
+  // prefit (the FP64 MP2 batch needs that order; the mixed path takes it where
+  // the tensor-core prefit finds no room).
+  gbjk_status prefit_fp64(cudaStream_t st, const double* d_B, const double* d_Linv, double* d_Bfit,
+                          int64_t* launches, std::string* err) {
+    std::vector<GemmGroup> groups;
+    std::vector<GemmTile> tiles;
+    for (int I = 0; I < nblk; ++I) {
+      const int K = panelK[I];
+      if (K == 0) continue;
+      for (int m = 0; m < bsize[I]; ++m) {
+        GemmGroup g;
+        const long long off = panel_off[I] + (long long)m * naux * K;
+        g.A = d_Linv;
+        g.B = d_B + off;
+        g.C = d_Bfit + off;
+        g.M = naux;
+        g.N = K;
+        g.K = naux;
+        g.lda = naux;
+        g.ldb = K;
+        g.ldc = K;
+        g.flags = kLowerA;
+        for (int mt = 0; mt < cdiv_(naux, 64); ++mt)
+          for (int nt = 0; nt < cdiv_(K, 64); ++nt)
+            tiles.push_back({(int)groups.size(), mt, nt, 0, naux, 0});
+        groups.push_back(g);
+      }
+    }
+    GemmGroup* dg = nullptr;
+    GemmTile* dt = nullptr;
+    if (cudaMalloc((void**)&dg, std::max<size_t>(1, groups.size()) * sizeof(GemmGroup)) !=
+            cudaSuccess ||
+        cudaMalloc((void**)&dt, std::max<size_t>(1, tiles.size()) * sizeof(GemmTile)) !=
+            cudaSuccess) {
+      cudaGetLastError();
+      cudaFree(dg);
+      *err = "out of memory for the prefit plan";
+      return GBJK_OOM;
+    }
+    cudaMemcpy(dg, groups.data(), groups.size() * sizeof(GemmGroup), cudaMemcpyHostToDevice);
+    cudaMemcpy(dt, tiles.data(), tiles.size() * sizeof(GemmTile), cudaMemcpyHostToDevice);
+    {
+      Scope sc(this, 3, st);
+      // the grid limit is 2^31-1 blocks; launch in slices of 1M tiles
+      for (size_t t0 = 0; t0 < tiles.size(); t0 += (1u << 20)) {
+        const int n = (int)std::min<size_t>(1u << 20, tiles.size() - t0);
+        k_gemm_fp64<false><<<n, 256, 0, st>>>(dg, dt + t0, 1.0);
+        (*launches)++;
+      }
+    }
+    const cudaError_t e = cudaStreamSynchronize(st);
+    cudaFree(dg);
+    cudaFree(dt);
+    if (e != cudaSuccess) {
+      *err = std::string("prefit: ") + cudaGetErrorString(e);
+      return GBJK_CUDA_ERROR;
+    }
+    return GBJK_OK;
+  }
+
+  // On the tensor cores (prefit_gemm.cuh).  ws: device memory that may be
+  // overwritten, for the digits of as many tensor columns as it holds (at
+  // most 1 GB of them at a time); a temporary buffer where it holds too few to
+  // occupy the SMs.
+  gbjk_status prefit(cudaStream_t st, const double* d_B, const double* d_Linv, double* d_Bfit,
+                     void* ws, size_t ws_bytes, int64_t* launches, std::string* err) {
+    std::vector<PfTile> tiles;
+    for (int I = 0; I < nblk; ++I) {
+      const int ncol = bsize[I] * panelK[I];
+      for (int c0 = 0; c0 < ncol; c0 += kPfM)
+        tiles.push_back({d_B + panel_off[I], d_Bfit + panel_off[I], panelK[I], c0, ncol});
+    }
+    if (tiles.empty()) return GBJK_OK;
+    const int nkt_all = cdiv_(naux, kPfK), nxt = cdiv_(naux, kPfN);
+    const size_t tile_bytes = (size_t)nkt_all * kPfBytesA, bbytes = (size_t)nxt * nkt_all * kPfBytesB;
+    const size_t most =
+        std::min(tiles.size(), std::max<size_t>(1, (size_t(1) << 30) / tile_bytes));
+    size_t per = std::min(most, ws_bytes / tile_bytes);
+    void* own = nullptr;
+    if (per < most && per * nxt < 1024) {
+      if (cudaMalloc(&own, most * tile_bytes) == cudaSuccess) {
+        ws = own;
+        per = most;
+      } else {
+        cudaGetLastError();
+      }
+    }
+    PfTile* dt = nullptr;
+    uint16_t* db = nullptr;
+    int* de = nullptr;  // exponents of the X rows, then of the tensor columns
+    auto done = [&]() {
+      cudaFree(own);
+      cudaFree(dt);
+      cudaFree(db);
+      cudaFree(de);
+    };
+    if (per == 0 || cudaMalloc((void**)&dt, tiles.size() * sizeof(PfTile)) != cudaSuccess ||
+        cudaMalloc((void**)&db, bbytes) != cudaSuccess ||
+        cudaMalloc((void**)&de, ((size_t)nxt * kPfN + per * kPfM) * sizeof(int)) != cudaSuccess ||
+        cudaFuncSetAttribute(k_prefit_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kPfSmem) != cudaSuccess) {
+      cudaGetLastError();
+      done();
+      return prefit_fp64(st, d_B, d_Linv, d_Bfit, launches, err);
+    }
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    int *eb = de, *ea = de + (size_t)nxt * kPfN;
+    uint16_t* ad = (uint16_t*)ws;
+    cudaError_t e = cudaMemcpyAsync(dt, tiles.data(), tiles.size() * sizeof(PfTile),
+                                    cudaMemcpyHostToDevice, st);
+    if (!e) e = cudaMemsetAsync(db, 0, bbytes, st);
+    if (!e) {
+      Scope sc(this, 3, st);
+      k_pf_metric<<<cdiv_(naux, 8), 256, 0, st>>>(d_Linv, naux, nkt_all, eb, db);
+      (*launches)++;
+      for (size_t t0 = 0; t0 < tiles.size(); t0 += per) {
+        const int n = (int)std::min(per, tiles.size() - t0);
+        k_pf_colexp<<<n, dim3(128, 4), 0, st>>>(dt + t0, naux, ea);
+        k_pf_coldigits<<<dim3(n, 2 * nkt_all), 256, 0, st>>>(dt + t0, ea, naux, nkt_all, ad);
+        k_prefit_gemm<<<std::min(n * nxt, nsm), kThreads, kPfSmem, st>>>(
+            dt + t0, n * nxt, nxt, naux, nkt_all, ad, ea, db, eb, d_err, kSpinNs);
+        *launches += 3;
+      }
+      e = cudaGetLastError();
+    }
+    if (!e) e = cudaStreamSynchronize(st);
+    done();
+    if (e != cudaSuccess) {
+      *err = std::string("prefit: ") + cudaGetErrorString(e);
+      return GBJK_CUDA_ERROR;
+    }
+    if (const int code = read_error()) {
+      *err = "prefit: a pipeline wait timed out (code " + std::to_string(code) + ")";
+      return GBJK_TIMEOUT;
+    }
+    return GBJK_OK;
+  }
+
   // --- once per tensor: the compact copy the mixed-path J reads ------------
   // Block pairs (I, J), I < J, whose columns lie side by side in both panels,
   // and k0[I], the first column of a block J >= I.  False if a panel's columns
@@ -421,6 +564,12 @@ struct SplitState {
   // --- once per tensor: prefit and A-operand digits -----------------------
   gbjk_status prepare_b(cudaStream_t st, const double* d_B, const double* d_Linv,
                         int64_t* launches, std::string* err) {
+    const gbjk_status s = prepare_tensor(st, d_B, d_Linv, launches, err);
+    if (s) release();  // nothing half prepared stays behind
+    return s;
+  }
+  gbjk_status prepare_tensor(cudaStream_t st, const double* d_B, const double* d_Linv,
+                             int64_t* launches, std::string* err) {
     const long long nnz = panel_off.back() + (long long)bsize.back() * naux * panelK.back();
     if (alloc(&d_err, 1) != cudaSuccess || cudaMemsetAsync(d_err, 0, sizeof(int), st) != cudaSuccess) {
       *err = "split path: cannot allocate the error flag";
@@ -432,69 +581,6 @@ struct SplitState {
     if (xb > naux) xb = naux;
     nbatch = (naux + xb - 1) / xb;
     apitch = pad32(xb);
-    double* d_Bfit = nullptr;
-    if (fitted) {
-      d_Bfit = const_cast<double*>(d_B);
-      bfit_owned = false;
-    } else {
-      if (alloc(&d_Bfit, (size_t)nnz) != cudaSuccess) {
-        *err = "split path: out of memory for the prefitted tensor";
-        return GBJK_OOM;
-      }
-      bfit_owned = true;
-      // Bfit_I[m] = L^-1 B_I[m]  (naux x K_I per AO function m)
-      std::vector<GemmGroup> groups;
-      std::vector<GemmTile> tiles;
-      for (int I = 0; I < nblk; ++I) {
-        const int K = panelK[I];
-        if (K == 0) continue;
-        for (int m = 0; m < bsize[I]; ++m) {
-          GemmGroup g;
-          const long long off = panel_off[I] + (long long)m * naux * K;
-          g.A = d_Linv;
-          g.B = d_B + off;
-          g.C = d_Bfit + off;
-          g.M = naux;
-          g.N = K;
-          g.K = naux;
-          g.lda = naux;
-          g.ldb = K;
-          g.ldc = K;
-          g.flags = kLowerA;
-          for (int mt = 0; mt < cdiv_(naux, 64); ++mt)
-            for (int nt = 0; nt < cdiv_(K, 64); ++nt)
-              tiles.push_back({(int)groups.size(), mt, nt, 0, naux, 0});
-          groups.push_back(g);
-        }
-      }
-      GemmGroup* dg = nullptr;
-      GemmTile* dt = nullptr;
-      if (alloc(&dg, groups.size()) != cudaSuccess || alloc(&dt, tiles.size()) != cudaSuccess) {
-        free_(&dg);
-        free_(&d_Bfit);
-        *err = "split path: out of memory for the prefit plan";
-        return GBJK_OOM;
-      }
-      cudaMemcpy(dg, groups.data(), groups.size() * sizeof(GemmGroup), cudaMemcpyHostToDevice);
-      cudaMemcpy(dt, tiles.data(), tiles.size() * sizeof(GemmTile), cudaMemcpyHostToDevice);
-      {
-        Scope sc(this, 3, st);
-        // the grid limit is 2^31-1 blocks; launch in slices of 1M tiles
-        for (size_t t0 = 0; t0 < tiles.size(); t0 += (1u << 20)) {
-          const int n = (int)std::min<size_t>(1u << 20, tiles.size() - t0);
-          k_gemm_fp64<false><<<n, 256, 0, st>>>(dg, dt + t0, 1.0);
-          (*launches)++;
-        }
-      }
-      cudaStreamSynchronize(st);
-      cudaFree(dg);
-      cudaFree(dt);
-    }
-    Bfit = d_Bfit;
-    if (nbatch == 1) {
-      gbjk_status js = prepare_j(st, launches, err);
-      if (js) return js;
-    }
     // A operands: rows (m, y) of panel I, y < xb (all auxiliary rows when
     // not batched), at m * pad32(batch) + y; columns k
     a_off.assign(nblk, 0);
@@ -511,11 +597,35 @@ struct SplitState {
       atot += (long long)a_nrb[I] * nkt[I] * kSlices * kImage;
       etot += (long long)a_nrb[I] * 32;
     }
-    if (alloc(&d_Aslices, (size_t)atot) != cudaSuccess || alloc(&d_eA, (size_t)etot) != cudaSuccess ||
-        cudaMemsetAsync(d_Aslices, 0, (size_t)atot * 2, st) != cudaSuccess ||
-        cudaMemsetAsync(d_eA, 0, (size_t)etot * 4, st) != cudaSuccess) {
+    double* d_Bfit = nullptr;
+    if (fitted) {
+      d_Bfit = const_cast<double*>(d_B);
+      bfit_owned = false;
+    } else if (alloc(&d_Bfit, (size_t)nnz) != cudaSuccess) {
+      *err = "split path: out of memory for the prefitted tensor";
+      return GBJK_OOM;
+    } else {
+      bfit_owned = true;
+    }
+    Bfit = d_Bfit;
+    if (alloc(&d_Aslices, (size_t)atot) != cudaSuccess ||
+        alloc(&d_eA, (size_t)etot) != cudaSuccess) {
       *err = "split path: out of memory for the operand digits";
       return GBJK_OOM;
+    }
+    if (!fitted) {
+      // the buffer of the operand digits holds the prefit's until it is needed
+      gbjk_status ps = prefit(st, d_B, d_Linv, d_Bfit, d_Aslices, (size_t)atot * 2, launches, err);
+      if (ps) return ps;
+    }
+    if (cudaMemsetAsync(d_Aslices, 0, (size_t)atot * 2, st) != cudaSuccess ||
+        cudaMemsetAsync(d_eA, 0, (size_t)etot * 4, st) != cudaSuccess) {
+      *err = "split path: memset failed";
+      return GBJK_CUDA_ERROR;
+    }
+    if (nbatch == 1) {
+      gbjk_status js = prepare_j(st, launches, err);
+      if (js) return js;
     }
     if (nbatch == 1) {
       // one job per AO function: its naux rows (m, y) at m * apitch + y

@@ -25,6 +25,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
+
 namespace gbjk {
 
 constexpr int kEriMaxLao = 2, kEriMaxLaux = 3;
@@ -42,6 +44,7 @@ constexpr int kEriRnChunk = 64;
 // ket matrix M[mc][j] of an auxiliary primitive: j over the Hermite
 // indices of t + u + v <= l_aux (at most 20), mc over its spherical components
 constexpr int kEriNKet = (kEriMaxLaux + 1) * (kEriMaxLaux + 2) * (kEriMaxLaux + 3) / 6;  // 20
+constexpr int kEriList = 512;  // kept auxiliary shells listed at a time
 constexpr int kEriWarpDoubles = 2 * kEriNR + kEriNW * kEriMaxSph +
                                 kEriRnChunk * (kEriMaxL + 1) +
                                 kEriMaxSph * kEriNKet;  // R x2, W, rn, M
@@ -49,9 +52,8 @@ constexpr int kEriWarpDoubles = 2 * kEriNR + kEriNW * kEriMaxSph +
 __constant__ double c_eri_sph[1 + 9 + 30 + 70];
 // (t, u, v) of the compact Hermite index e (t + u + v <= 7): t | u << 8 | v << 16
 __constant__ int c_eri_tuv[kEriNR];
-// 1 / (2 j + 1) for the Boys series and recursion (no FP64 division there)
-constexpr int kEriBoysTerms = 400;
-__constant__ double c_eri_rodd[kEriMaxL + kEriBoysTerms + 1];
+// 1 / (2 j + 1) for the Boys recursion (no FP64 division there)
+__constant__ double c_eri_rodd[kEriMaxL + 1];
 
 struct EriShell {
   int l, nprim, prim0, bf_off;
@@ -82,32 +84,76 @@ __device__ __forceinline__ void eri_cart(int l, int c, int* ex) {
     }
 }
 
-// Boys function F_0..F_n at T: the host engine's algorithm (series at
-// n = nmax and downward recursion, or erf and upward recursion for large T),
-// with the divisions by odd integers taken as products with their
-// reciprocals (a rounding-level difference from the host).
-__device__ void eri_boys(int nmax, double T, double* F) {
-  if (T < 1e-15) {
-    for (int m = 0; m <= nmax; ++m) F[m] = c_eri_rodd[m];
-    return;
+// Boys function F_0..F_n at T.  Below T = kEriBoysTmax F_n comes from its
+// Taylor expansion about the nearest grid point (eight terms, |dT| <= 1/32, the
+// next one below 3e-17 of F), e^-T likewise, and the lower orders by downward
+// recursion; above, erf and upward recursion, as in the host engine.  FP64
+// instructions are what bounds this kernel, and the series this replaces took
+// two to three hundred of them per argument.
+constexpr double kEriBoysTmax = 33.0;
+constexpr int kEriBoysStep = 16;  // grid points per unit of T
+constexpr int kEriBoysRows = (int)kEriBoysTmax * kEriBoysStep + 2;
+// table row of order n at T0 = i / 16: F_{n+k}(T0) / k!, k = 0..7, at
+// tab[(n * kEriBoysRows + i) * 8]; e^-T0 at tab[kEriBoysExp + i]
+constexpr int kEriBoysExp = (kEriMaxL + 1) * kEriBoysRows * 8;
+constexpr int kEriBoysTable = kEriBoysExp + kEriBoysRows;
+
+// Host: the table, by the ascending series of F_15 and downward recursion.
+inline void eri_boys_table(double* tab) {
+  for (int i = 0; i < kEriBoysRows; ++i) {
+    const double T = (double)i / kEriBoysStep, eT = std::exp(-T);
+    double F[kEriMaxL + 8];
+    const int top = kEriMaxL + 7;
+    double term = 1.0 / (2 * top + 1), sum = term;
+    for (int k = 1; k < 400 && term > 1e-18 * sum; ++k) {
+      term *= 2.0 * T / (2 * (top + k) + 1);
+      sum += term;
+    }
+    F[top] = eT * sum;
+    for (int m = top - 1; m >= 0; --m) F[m] = (2.0 * T * F[m + 1] + eT) / (2 * m + 1);
+    for (int n = 0; n <= kEriMaxL; ++n) {
+      double fac = 1.0;
+      for (int k = 0; k < 8; ++k) {
+        if (k) fac *= k;
+        tab[((size_t)n * kEriBoysRows + i) * 8 + k] = F[n + k] / fac;
+      }
+    }
+    tab[kEriBoysExp + i] = eT;
   }
-  const double eT = exp(-T);
-  if (T > 33.0 + nmax) {
+}
+
+__device__ __forceinline__ void eri_boys(const double* __restrict__ tab, int nmax, double T,
+                                         double* F) {
+  if (T > kEriBoysTmax) {
+    const double eT = exp(-T);
     F[0] = 0.5 * sqrt(3.14159265358979323846 / T) * erf(sqrt(T));
     const double inv2T = 0.5 / T;
     for (int m = 0; m < nmax; ++m) F[m + 1] = ((2 * m + 1) * F[m] - eT) * inv2T;
     return;
   }
-  double term = c_eri_rodd[nmax];
-  double sum = term;
+  const int i = (int)((float)T * (float)kEriBoysStep + 0.5f);
+  const double x = (double)i * (1.0 / kEriBoysStep) - T;
+  const double2* c = reinterpret_cast<const double2*>(tab + ((long long)nmax * kEriBoysRows + i) * 8);
+  const double2 c0 = __ldg(c), c1 = __ldg(c + 1), c2 = __ldg(c + 2), c3 = __ldg(c + 3);
+  double f = fma(c3.y, x, c3.x);
+  f = fma(f, x, c2.y);
+  f = fma(f, x, c2.x);
+  f = fma(f, x, c1.y);
+  f = fma(f, x, c1.x);
+  f = fma(f, x, c0.y);
+  f = fma(f, x, c0.x);
+  F[nmax] = f;
+  if (nmax == 0) return;
+  double e = fma(x, 1.0 / 5040, 1.0 / 720);
+  e = fma(e, x, 1.0 / 120);
+  e = fma(e, x, 1.0 / 24);
+  e = fma(e, x, 1.0 / 6);
+  e = fma(e, x, 0.5);
+  e = fma(e, x, 1.0);
+  e = fma(e, x, 1.0);
+  const double eT = e * __ldg(tab + kEriBoysExp + i);
   const double twoT = 2.0 * T;
-  for (int k = 1; k < kEriBoysTerms; ++k) {
-    term *= twoT * c_eri_rodd[nmax + k];
-    sum += term;
-    if (term < 1e-17 * sum) break;
-  }
-  F[nmax] = eT * sum;
-  for (int m = nmax - 1; m >= 0; --m) F[m] = (twoT * F[m + 1] + eT) * c_eri_rodd[m];
+  for (int m = nmax - 1; m >= 0; --m) F[m] = fma(twoT, F[m + 1], eT) * c_eri_rodd[m];
 }
 
 // Ket matrix of an auxiliary primitive of exponent qq and angular momentum
@@ -143,6 +189,30 @@ __device__ void eri_ket_matrix(int lc, double qq, int lane, double* M) {
     }
     M[mc * kEriNKet + j] = ((t + u + v) & 1) ? -m : m;
   }
+}
+
+// The ket matrices of every auxiliary primitive, kEriKetSize doubles each: once
+// per tensor (every AO shell pair used to rebuild them).  grid ceil(nprim / 4),
+// block 128.
+constexpr int kEriKetSize = kEriMaxSph * kEriNKet;
+__global__ void k_eri_ket(const EriShell* __restrict__ ax, int nshell,
+                          const double* __restrict__ ax_alpha, int nprim, double* __restrict__ M) {
+  const int k = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (k >= nprim) return;
+  int lo = 0, hi = nshell - 1;  // the shell of primitive k
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (ax[mid].prim0 <= k)
+      lo = mid;
+    else
+      hi = mid - 1;
+  }
+  eri_ket_matrix(ax[lo].l, ax_alpha[k], lane, M + (long long)k * kEriKetSize);
+}
+// A primitive's ket matrix into the warp's shared memory.
+__device__ __forceinline__ void eri_load_ket(const double* __restrict__ Mg, int nsc, int lane,
+                                             double* M) {
+  for (int i = lane; i < nsc * kEriNKet; i += 32) M[i] = __ldg(Mg + i);
 }
 
 // E[axis][i][j][t] of one primitive pair, i <= la, j <= lb, t <= i + j, in
@@ -206,8 +276,8 @@ __host__ __device__ constexpr int eri_idx_c(int t, int u, int v) {
 template <int LC>
 __device__ void eri_ss_aux(const double* pp, int psz, int npp, const EriShell& c,
                            const double* __restrict__ ax_alpha,
-                           const double* __restrict__ ax_coef, int lane, double* M,
-                           double* acc) {
+                           const double* __restrict__ ax_coef, const double* __restrict__ Mg,
+                           const double* __restrict__ tab, int lane, double* M, double* acc) {
   constexpr int NSC = 2 * LC + 1;
   constexpr int NR = (LC + 1) * (LC + 2) * (LC + 3) / 6;
   double part[NSC];
@@ -215,19 +285,22 @@ __device__ void eri_ss_aux(const double* pp, int psz, int npp, const EriShell& c
   for (int m = 0; m < NSC; ++m) part[m] = 0.0;
   for (int k = 0; k < c.nprim; ++k) {
     const double qq = ax_alpha[c.prim0 + k];
+    const double cq = ax_coef[c.prim0 + k] / qq;
     __syncwarp();  // the previous primitive's M is no longer read
-    eri_ket_matrix(LC, qq, lane, M);
+    eri_load_ket(Mg + (long long)(c.prim0 + k) * kEriKetSize, NSC, lane, M);
     __syncwarp();
     for (int q = lane; q < npp; q += 32) {
       const double* o = pp + q * psz;
       if (o[5] == 0.0) continue;
       const double p = o[0];
-      const double alpha = p * qq / (p + qq);
-      const double pref = 2.0 * 17.493418327624862 / (p * qq * sqrt(p + qq)) * o[4] *
-                          ax_coef[c.prim0 + k];  // 2 pi^{5/2}
+      // alpha = p q / (p + q), pref = 2 pi^{5/2} / (p q sqrt(p + q)) (o[4] holds
+      // the bra's part)
+      const double rs = rsqrt(p + qq);
+      const double alpha = p * qq * (rs * rs);
+      const double pref = o[4] * cq * rs;
       const double X = o[1] - c.A[0], Y = o[2] - c.A[1], Z = o[3] - c.A[2];
       double F[LC + 1];
-      eri_boys(LC, alpha * (X * X + Y * Y + Z * Z), F);
+      eri_boys(tab, LC, alpha * (X * X + Y * Y + Z * Z), F);
       double rn[LC + 1];
       double fac = 1.0;
 #pragma unroll
@@ -282,39 +355,84 @@ __device__ void eri_ss_aux(const double* pp, int psz, int npp, const EriShell& c
   }
 }
 
+// How lane e of an R level forms R^n[e] from level n + 1: coordinate (axis)
+// times entry i1 plus fac times entry i2; packed i1 | i2 << 8 | axis << 16 |
+// fac << 20 (e = 0 is the Boys value itself).
+__device__ __forceinline__ int eri_r_step(int e) {
+  const int tuv = c_eri_tuv[e];
+  const int t = tuv & 255, u = (tuv >> 8) & 255, v = tuv >> 16;
+  const int axis = t > 0 ? 0 : (u > 0 ? 1 : 2);
+  const int n = axis == 0 ? t : (axis == 1 ? u : v);
+  if (n == 0) return 0;
+  const int i1 = eri_idx(t - (axis == 0), u - (axis == 1), v - (axis == 2));
+  const int i2 = n > 1 ? eri_idx(t - 2 * (axis == 0), u - 2 * (axis == 1), v - 2 * (axis == 2)) : 0;
+  return i1 | (i2 << 8) | (axis << 16) | ((n - 1) << 20);
+}
+
+// doubles of one bra primitive pair: p, P[3], coefficient, keep flag, E
+__host__ __device__ constexpr int eri_pair_size(int la, int lb) {
+  return 6 + 3 * (la + 1) * (lb + 1) * (la + lb + 1);
+}
+// doubles of its Hermite -> spherical (a, b) matrix (not for s-s pairs)
+__host__ __device__ constexpr int eri_sph_size(int la, int lb) {
+  return (2 * la + 1) * (2 * lb + 1) * ((la + lb + 1) * (la + lb + 2) * (la + lb + 3) / 6);
+}
+// primitive pairs whose matrices are held at a time (about 24 KB)
+__host__ __device__ constexpr int eri_sph_chunk(int la, int lb, int npp) {
+  const int fit = 3072 / eri_sph_size(la, lb);
+  const int n = fit < 1 ? 1 : fit;
+  return n < npp ? n : npp;
+}
+
+// One block per AO shell pair (a, b); its warps take the kept auxiliary shells
+// in turn.  What bounds it is the FP64 pipe, where a warp instruction costs 16
+// clocks however few lanes take part, so every phase spreads over the lanes:
+//   Boys values   lanes over the (shell, primitive pair, primitive)
+//                 combinations of up to 64 at once, several shells together
+//   R levels      one entry per lane, one fma and one product each
+//   W[e][mc]      lanes over (Hermite index e, spherical component mc)
+//   (a, b)        lanes over (spherical pair, mc), against a matrix per
+//                 primitive pair that folds E and both spherical transforms
 // SS: the launch holds only s-s shell pairs (lanes over primitive pairs),
 // else only the other pairs; two kernels with half the code each keep the
-// instruction working set of a block small.
+// instruction working set of a block small.  Six waters / jkfit: s-s 13.1 -> 4.2
+// ms, the others 34.4 -> 8.4 ms against lanes over e and over cartesian pairs.
 template <bool SS>
 __global__ void __launch_bounds__(32 * kEriWarps, 4)
     k_eri3c(const EriItem* __restrict__ items, const EriShell* __restrict__ ao,
             const EriShell* __restrict__ ax, const double* __restrict__ ao_alpha,
             const double* __restrict__ ao_coef, const double* __restrict__ ax_alpha,
-            const double* __restrict__ ax_coef, const int* __restrict__ pair_I,
+            const double* __restrict__ ax_coef, const double* __restrict__ ket,
+            const double* __restrict__ boys, const int* __restrict__ pair_I,
             const int* __restrict__ pair_J, const unsigned char* __restrict__ keep, int nablk,
             const int* __restrict__ ablk_shell_off, const int* __restrict__ blk_bf_off,
             const long long* __restrict__ panel_off, const int* __restrict__ panel_K,
             const int* __restrict__ col_IJ, const int* __restrict__ col_JI, int naux,
             double* __restrict__ B) {
   extern __shared__ double sm[];
+  __shared__ unsigned char plus[kEriNW * kEriNKet];  // index of e + j (Hermite indices)
+  __shared__ int list[kEriList];                     // kept auxiliary shells
+  __shared__ int nlist, next_A, next_s;
+  __shared__ double small[kEriMaxL];  // 0, 1, .. (a conversion is an FP64 instruction too)
   const EriItem it = items[blockIdx.x];
   const EriShell a = ao[it.a], b = ao[it.b];
   const int la = a.l, lb = b.l, Lb = la + lb;
-  const int nca = (la + 1) * (la + 2) / 2, ncb = (lb + 1) * (lb + 2) / 2;
-  const int nsa = 2 * la + 1, nsb = 2 * lb + 1;
+  const int nsa = 2 * la + 1, nsb = 2 * lb + 1, nab = nsa * nsb;
   const int npp = a.nprim * b.nprim;
-  const int esz = 3 * (la + 1) * (lb + 1) * (Lb + 1);  // E doubles per primitive pair
-  const int psz = 6 + esz;                              // p, P[3], coef, keep flag, E
-  const int nW = eri_tet(Lb + 1);                       // bra Hermite indices
-  double* pp = sm;                                      // npp * psz
-  double* wbase = sm + npp * psz + (threadIdx.x >> 5) * kEriWarpDoubles;
+  const int psz = eri_pair_size(la, lb);
+  const int nW = eri_tet(Lb + 1);  // bra Hermite indices
+  const int qcs = SS ? npp : eri_sph_chunk(la, lb, npp);
+  double* pp = sm;  // npp * psz
+  double* Es = sm + npp * psz;
+  double* wbase = Es + (SS ? 0 : qcs * nab * nW) + (threadIdx.x >> 5) * kEriWarpDoubles;
   double* R0 = wbase;
   double* R1 = wbase + kEriNR;
   double* W = wbase + 2 * kEriNR;
-  double* rnq = W + kEriNW * kEriMaxSph;  // kEriRnChunk x (kEriMaxL + 1)
+  double* rnq = W + kEriNW * kEriMaxSph;            // kEriRnChunk x (kEriMaxL + 1)
   double* Mk = rnq + kEriRnChunk * (kEriMaxL + 1);  // kEriMaxSph x kEriNKet
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
+  if (threadIdx.x < kEriMaxL) small[threadIdx.x] = threadIdx.x;
   // bra primitive pairs
   double ab2 = 0.0;
   for (int d = 0; d < 3; ++d) ab2 += (a.A[d] - b.A[d]) * (a.A[d] - b.A[d]);
@@ -335,197 +453,252 @@ __global__ void __launch_bounds__(32 * kEriWarps, 4)
     o[1] = P[0];
     o[2] = P[1];
     o[3] = P[2];
-    o[4] = coef;
+    o[4] = 2.0 * 17.493418327624862 * coef / p;  // 2 pi^{5/2}
+    if (SS) o[4] *= c_eri_sph[0] * c_eri_sph[0];  // both s functions' normalisation
     o[5] = fabs(coef * kab) < 1e-16 ? 0.0 : 1.0;
     eri_hermite_pair(la, lb, p, PA, PB, kab, o + 6);
   }
+  if (!SS)
+    for (int i = threadIdx.x; i < nW * kEriNKet; i += blockDim.x) {
+      const int x = c_eri_tuv[i / kEriNKet], y = c_eri_tuv[i % kEriNKet];
+      const int t = (x & 255) + (y & 255), u = ((x >> 8) & 255) + ((y >> 8) & 255),
+                v = (x >> 16) + (y >> 16);
+      plus[i] = t + u + v <= kEriMaxL ? (unsigned char)eri_idx(t, u, v) : 0;
+    }
   __syncthreads();
 
   const int I = pair_I[it.p], J = pair_J[it.p];
-  const int Eax = (la + 1) * (lb + 1) * (Lb + 1), Esi = (lb + 1) * (Lb + 1), Esj = Lb + 1;
-  // shells of the kept auxiliary blocks, in turn over the warps
-  int counter = 0;
-  for (int A = 0; A < nablk; ++A) {
-    if (!keep[(long long)it.p * nablk + A]) continue;
-    for (int s = ablk_shell_off[A]; s < ablk_shell_off[A + 1]; ++s, ++counter) {
-      if (counter % kEriWarps != warp) continue;
-      const EriShell c = ax[s];
-      const int lc = c.l, nsc = 2 * lc + 1;
-      const int L = Lb + lc;
-      double acc0[kEriMaxSph], acc1[kEriMaxSph];  // cartesian pairs lane, lane + 32
-      for (int m = 0; m < kEriMaxSph; ++m) acc0[m] = acc1[m] = 0.0;
-      const int nck = c.nprim;
-      const int qch = kEriRnChunk / nck > 0 ? kEriRnChunk / nck : 1;
-      if constexpr (SS) {
-        // s-s pair: lanes over the bra primitive pairs; every lane ends
-        // with the sums, lane 0 stores them as the one cartesian pair
-        if (lc == 0)
-          eri_ss_aux<0>(pp, psz, npp, c, ax_alpha, ax_coef, lane, Mk, acc0);
-        else if (lc == 1)
-          eri_ss_aux<1>(pp, psz, npp, c, ax_alpha, ax_coef, lane, Mk, acc0);
-        else if (lc == 2)
-          eri_ss_aux<2>(pp, psz, npp, c, ax_alpha, ax_coef, lane, Mk, acc0);
-        else
-          eri_ss_aux<3>(pp, psz, npp, c, ax_alpha, ax_coef, lane, Mk, acc0);
-      } else if (nck == 1) {
-        // one auxiliary primitive: its ket matrix serves every bra pair
-        eri_ket_matrix(lc, ax_alpha[c.prim0], lane, Mk);
-        __syncwarp();
-      }
-      for (int q0 = 0; q0 < (SS ? 0 : npp); q0 += qch) {
-      const int q1 = min(npp, q0 + qch);
-      // Boys functions of the chunk's (q, k) combinations, one per lane
-      for (int jq = lane; jq < (q1 - q0) * nck; jq += 32) {
-        const int q = q0 + jq / nck, k = jq % nck;
-        const double* o = pp + q * psz;
-        if (o[5] == 0.0) continue;
-        const double p = o[0], qq = ax_alpha[c.prim0 + k];
-        const double alpha = p * qq / (p + qq);
-        const double X = o[1] - c.A[0], Y = o[2] - c.A[1], Z = o[3] - c.A[2];
-        double F[kEriMaxL + 1];
-        eri_boys(L, alpha * (X * X + Y * Y + Z * Z), F);
-        double fac = 1.0;
-        double* r = rnq + jq * (kEriMaxL + 1);
-        for (int n = 0; n <= L; ++n) {
-          r[n] = fac * F[n];
-          fac *= -2.0 * alpha;
-        }
-      }
-      __syncwarp();
-      for (int q = q0; q < q1; ++q) {
-        const double* o = pp + q * psz;
-        if (o[5] == 0.0) continue;
-        const double p = o[0];
-        double w0[kEriMaxSph], w1[kEriMaxSph];  // W for bra indices lane, lane + 32
-        for (int m = 0; m < kEriMaxSph; ++m) w0[m] = w1[m] = 0.0;
-        for (int k = 0; k < c.nprim; ++k) {
-          const double qq = ax_alpha[c.prim0 + k];
-          const double pref = 2.0 * 17.493418327624862 / (p * qq * sqrt(p + qq)) * o[4] *
-                              ax_coef[c.prim0 + k];  // 2 pi^{5/2}
-          const double X = o[1] - c.A[0], Y = o[2] - c.A[1], Z = o[3] - c.A[2];
-          const double* rn = rnq + ((q - q0) * nck + k) * (kEriMaxL + 1);
-          // R^n_{tuv}, levels n = L .. 0; level 0 ends in Rc
-          double* cur = (L & 1) ? R1 : R0;
-          double* old = (L & 1) ? R0 : R1;
-          if (lane == 0) cur[0] = rn[L];
-          __syncwarp();
-          for (int n = L - 1; n >= 0; --n) {
-            double* t_ = cur;
-            cur = old;
-            old = t_;
-            const int lt = L - n, cnt = eri_tet(lt + 1);
-            for (int e = lane; e < cnt; e += 32) {
-              const int tuv = c_eri_tuv[e];
-              const int t = tuv & 255, u = (tuv >> 8) & 255, v = tuv >> 16;
-              double val;
-              if (t > 0) {
-                val = X * old[eri_idx(t - 1, u, v)];
-                if (t > 1) val += (t - 1) * old[eri_idx(t - 2, u, v)];
-              } else if (u > 0) {
-                val = Y * old[eri_idx(t, u - 1, v)];
-                if (u > 1) val += (u - 1) * old[eri_idx(t, u - 2, v)];
-              } else if (v > 0) {
-                val = Z * old[eri_idx(t, u, v - 1)];
-                if (v > 1) val += (v - 1) * old[eri_idx(t, u, v - 2)];
-              } else {
-                val = rn[n];
-              }
-              cur[e] = val;
-            }
-            __syncwarp();
-          }
-          const double* Rc = cur;
-          // W[tuv][mc] += pref sum_j M[mc][j] R[(t, u, v) + j]
-          if (nck > 1) {
-            eri_ket_matrix(lc, qq, lane, Mk);
-            __syncwarp();
-          }
-          const int nr = eri_tet(lc + 1);
-          for (int h = 0; h < 2; ++h) {
-            const int e = lane + 32 * h;
-            if (e >= nW) break;
-            const int tuv = c_eri_tuv[e];
-            const int t = tuv & 255, u = (tuv >> 8) & 255, v = tuv >> 16;
-            double* w = h ? w1 : w0;
-            for (int jj = 0; jj < nr; ++jj) {
-              const int kt = c_eri_tuv[jj];
-              const double r =
-                  pref * Rc[eri_idx(t + (kt & 255), u + ((kt >> 8) & 255), v + (kt >> 16))];
-              for (int mc = 0; mc < nsc; ++mc) w[mc] += Mk[mc * kEriNKet + jj] * r;
-            }
-          }
-          __syncwarp();  // R buffers are rewritten by the next primitive
-        }
-        // publish W of this primitive pair, then acc[cab] += sum_bra E W
-        for (int h = 0; h < 2; ++h) {
-          const int e = lane + 32 * h;
-          if (e < nW)
-            for (int mc = 0; mc < nsc; ++mc) W[e * kEriMaxSph + mc] = h ? w1[mc] : w0[mc];
-        }
-        __syncwarp();
-        const double* E = o + 6;
-        for (int h = 0; h < 2; ++h) {
-          const int cab = lane + 32 * h;
-          if (cab >= nca * ncb) break;
-          int ea[3], eb[3];
-          eri_cart(la, cab / ncb, ea);
-          eri_cart(lb, cab % ncb, eb);
-          for (int t = 0; t <= ea[0] + eb[0]; ++t) {
-            const double ex = E[0 * Eax + ea[0] * Esi + eb[0] * Esj + t];
-            if (ex == 0.0) continue;
-            for (int u = 0; u <= ea[1] + eb[1]; ++u) {
-              const double ey = E[1 * Eax + ea[1] * Esi + eb[1] * Esj + u];
-              if (ey == 0.0) continue;
-              for (int v = 0; v <= ea[2] + eb[2]; ++v) {
-                const double ez = E[2 * Eax + ea[2] * Esi + eb[2] * Esj + v];
-                if (ez == 0.0) continue;
-                const double cf = ex * ey * ez;
-                const double* w = W + eri_idx(t, u, v) * kEriMaxSph;
-                double* ac = h ? acc1 : acc0;
-                for (int mc = 0; mc < nsc; ++mc) ac[mc] += cf * w[mc];
-              }
-            }
-          }
-        }
-        __syncwarp();
-      }
-      __syncwarp();  // the next chunk rewrites the Boys values
-      }
-      // spherical (a, b): stage the cartesian accumulators in the warp's
-      // R/W space, then each lane writes outputs (ma, mb, mc)
-      double* st = wbase;
-      for (int h = 0; h < 2; ++h) {
-        const int cab = lane + 32 * h;
-        if (cab < nca * ncb)
-          for (int mc = 0; mc < nsc; ++mc) st[cab * kEriMaxSph + mc] = h ? acc1[mc] : acc0[mc];
-      }
-      __syncwarp();
+  const int I0 = blk_bf_off[I], J0 = blk_bf_off[J];
+  const int KI = panel_K[I], KJ = panel_K[J];
+  double* const PI = B + panel_off[I];
+  double* const PJ = B + panel_off[J];
+  // one result (ma, mb, mc) of auxiliary shell c into the panels; add: the
+  // part of a later chunk of primitive pairs (the same thread wrote the first)
+  auto store = [&](int ma, int mb, int X, double v, bool add) {
+    const int mu = a.bf_off + ma - I0, nu = b.bf_off + mb - J0;
+    double* o1 = PI + ((long long)mu * naux + X) * KI + col_IJ[it.p] + nu;
+    double* o2 = I != J ? PJ + ((long long)nu * naux + X) * KJ + col_JI[it.p] + mu
+                        : (it.a != it.b ? PI + ((long long)nu * naux + X) * KI + col_IJ[it.p] + mu
+                                        : nullptr);
+    if (add) v += *o1;
+    *o1 = v;
+    if (o2) *o2 = v;
+  };
+  int rstep[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) rstep[i] = !SS && lane + 32 * i < kEriNR ? eri_r_step(lane + 32 * i) : 0;
+
+  for (int qs0 = 0; qs0 < npp; qs0 += qcs) {
+    const int qs1 = min(npp, qs0 + qcs);
+    if constexpr (!SS) {
+      // Es[q][ab][e] = sum_{ca, cb} sph_a sph_b E^x_t E^y_u E^z_v
+      __syncthreads();
+      const int nca = (la + 1) * (la + 2) / 2, ncb = (lb + 1) * (lb + 2) / 2;
+      const int Eax = (la + 1) * (lb + 1) * (Lb + 1), Esi = (lb + 1) * (Lb + 1), Esj = Lb + 1;
       const double* sa = c_eri_sph + eri_sph_off(la);
       const double* sb = c_eri_sph + eri_sph_off(lb);
-      const int I0 = blk_bf_off[I], J0 = blk_bf_off[J];
-      const int KI = panel_K[I], KJ = panel_K[J];
-      double* PI = B + panel_off[I];
-      double* PJ = B + panel_off[J];
-      for (int o = lane; o < nsa * nsb * nsc; o += 32) {
-        const int ma = o / (nsb * nsc), mb = (o / nsc) % nsb, mc = o % nsc;
-        double v = 0.0;
+      for (int i = threadIdx.x; i < (qs1 - qs0) * nab * nW; i += blockDim.x) {
+        const int e = i % nW, ab = (i / nW) % nab, q = qs0 + i / (nW * nab);
+        const int ma = ab / nsb, mb = ab % nsb;
+        const int tuv = c_eri_tuv[e];
+        const int t = tuv & 255, u = (tuv >> 8) & 255, v = tuv >> 16;
+        const double* E = pp + q * psz + 6;
+        double sum = 0.0;
         for (int ca = 0; ca < nca; ++ca) {
           const double fa = sa[ma * nca + ca];
           if (fa == 0.0) continue;
-          double s2 = 0.0;
-          for (int cb = 0; cb < ncb; ++cb)
-            s2 += sb[mb * ncb + cb] * st[(ca * ncb + cb) * kEriMaxSph + mc];
-          v += fa * s2;
+          int ea[3];
+          eri_cart(la, ca, ea);
+          for (int cb = 0; cb < ncb; ++cb) {
+            const double fb = sb[mb * ncb + cb];
+            if (fb == 0.0) continue;
+            int eb[3];
+            eri_cart(lb, cb, eb);
+            if (t > ea[0] + eb[0] || u > ea[1] + eb[1] || v > ea[2] + eb[2]) continue;
+            sum += (fa * fb) * (E[ea[0] * Esi + eb[0] * Esj + t] *
+                                E[Eax + ea[1] * Esi + eb[1] * Esj + u] *
+                                E[2 * Eax + ea[2] * Esi + eb[2] * Esj + v]);
+          }
         }
-        const int mu = a.bf_off + ma - I0, nu = b.bf_off + mb - J0;
-        const long long X = c.bf_off + mc;
-        PI[((long long)mu * naux + X) * KI + col_IJ[it.p] + nu] = v;
-        if (I != J)
-          PJ[((long long)nu * naux + X) * KJ + col_JI[it.p] + mu] = v;
-        else if (it.a != it.b)
-          PI[((long long)nu * naux + X) * KI + col_IJ[it.p] + mu] = v;
+        Es[i] = sum;
       }
-      __syncwarp();
+      __syncthreads();
+    }
+    // kept auxiliary shells, kEriList of them at a time
+    if (threadIdx.x == 0) next_A = next_s = 0;
+    for (;;) {
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        int n = 0, A = next_A, s = next_s;
+        while (A < nablk && n < kEriList) {
+          if (!keep[(long long)it.p * nablk + A]) {
+            ++A;
+            s = 0;
+            continue;
+          }
+          const int s0 = ablk_shell_off[A], ns = ablk_shell_off[A + 1] - s0;
+          while (s < ns && n < kEriList) list[n++] = s0 + s++;
+          if (s == ns) {
+            ++A;
+            s = 0;
+          }
+        }
+        nlist = n;
+        next_A = A;
+        next_s = s;
+      }
+      __syncthreads();
+      if (nlist == 0) break;
+      if constexpr (SS) {
+        for (int i = warp; i < nlist; i += kEriWarps) {
+          const EriShell c = ax[list[i]];
+          double acc[kEriMaxSph];
+          if (c.l == 0)
+            eri_ss_aux<0>(pp, psz, npp, c, ax_alpha, ax_coef, ket, boys, lane, Mk, acc);
+          else if (c.l == 1)
+            eri_ss_aux<1>(pp, psz, npp, c, ax_alpha, ax_coef, ket, boys, lane, Mk, acc);
+          else if (c.l == 2)
+            eri_ss_aux<2>(pp, psz, npp, c, ax_alpha, ax_coef, ket, boys, lane, Mk, acc);
+          else
+            eri_ss_aux<3>(pp, psz, npp, c, ax_alpha, ax_coef, ket, boys, lane, Mk, acc);
+          // every lane has the sums
+          double v = acc[0];
+#pragma unroll
+          for (int m = 1; m < kEriMaxSph; ++m) v = lane == m && m < 2 * c.l + 1 ? acc[m] : v;
+          if (lane < 2 * c.l + 1) store(0, 0, c.bf_off + lane, v, false);
+        }
+      } else {
+        const double* Esq = Es - (long long)qs0 * nab * nW;
+        for (int i0 = warp; i0 < nlist;) {
+          // a batch of shells with the same contraction whose combinations fit
+          // the Boys buffer (one shell, in pieces, if it has too many)
+          const int nck = ax[list[i0]].nprim;
+          const int per = (qs1 - qs0) * nck;  // combinations of a shell
+          int nb = 1;
+          while (nb < 32 && i0 + nb * kEriWarps < nlist && (nb + 1) * per <= kEriRnChunk &&
+                 ax[list[i0 + nb * kEriWarps]].nprim == nck)
+            ++nb;
+          const int qch = max(1, min(qs1 - qs0, kEriRnChunk / nck));
+          double acc[6];  // results (ab, mc): lane + 32 i
+          for (int q0 = qs0; q0 < qs1; q0 += qch) {
+            const int q1 = min(qs1, q0 + qch), nqk = (q1 - q0) * nck;
+            __syncwarp();  // the Boys buffer is no longer read
+            for (int jq = lane; jq < nb * nqk; jq += 32) {
+              const int sh = jq / nqk, r0 = jq - sh * nqk;
+              const int q = q0 + r0 / nck, k = r0 % nck;
+              const double* o = pp + q * psz;
+              if (o[5] == 0.0) continue;
+              const EriShell& c = ax[list[i0 + sh * kEriWarps]];
+              const int L = Lb + c.l;
+              const double p = o[0], qq = ax_alpha[c.prim0 + k];
+              const double rs = rsqrt(p + qq);
+              const double alpha = p * qq * (rs * rs);
+              const double X = o[1] - c.A[0], Y = o[2] - c.A[1], Z = o[3] - c.A[2];
+              double F[kEriMaxL + 1];
+              eri_boys(boys, L, alpha * (X * X + Y * Y + Z * Z), F);
+              double fac = o[4] * (ax_coef[c.prim0 + k] / qq) * rs;  // the prefactor rides along
+              double* r = rnq + jq * (kEriMaxL + 1);
+              for (int n = 0; n <= L; ++n) {
+                r[n] = fac * F[n];
+                fac *= -2.0 * alpha;
+              }
+            }
+            __syncwarp();
+            for (int sh = 0; sh < nb; ++sh) {
+              const EriShell c = ax[list[i0 + sh * kEriWarps]];
+              const int lc = c.l, nsc = 2 * lc + 1, L = Lb + lc, nr = eri_tet(lc + 1);
+              const int nw = nW * nsc, no = nab * nsc;
+              // this lane's W entries (e, mc) and results (ab, mc)
+              int wid[8], oid[6];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const int id = lane + 32 * i, e = id / nsc;
+                wid[i] = id < nw ? (e * kEriNKet) | ((id - e * nsc) * kEriNKet) << 16 : 0;
+              }
+#pragma unroll
+              for (int i = 0; i < 6; ++i) {
+                const int id = lane + 32 * i, ab = id / nsc;
+                oid[i] = id < no ? (ab * nW) | (id - ab * nsc) << 16 : 0;
+              }
+              if (q0 == qs0)
+#pragma unroll
+                for (int i = 0; i < 6; ++i) acc[i] = 0.0;
+              if (nck == 1) {
+                eri_load_ket(ket + (long long)c.prim0 * kEriKetSize, nsc, lane, Mk);
+                __syncwarp();
+              }
+              for (int q = q0; q < q1; ++q) {
+                const double* o = pp + q * psz;
+                if (o[5] == 0.0) continue;
+                const double X = o[1] - c.A[0], Y = o[2] - c.A[1], Z = o[3] - c.A[2];
+                double w[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) w[i] = 0.0;
+                for (int k = 0; k < nck; ++k) {
+                  const double* rn = rnq + (sh * nqk + (q - q0) * nck + k) * (kEriMaxL + 1);
+                  // R^n_{tuv}, levels n = L .. 0; level 0 ends in cur
+                  double* cur = (L & 1) ? R1 : R0;
+                  double* old = (L & 1) ? R0 : R1;
+                  if (lane == 0) cur[0] = rn[L];
+                  if (nck > 1)
+                    eri_load_ket(ket + (long long)(c.prim0 + k) * kEriKetSize, nsc, lane, Mk);
+                  __syncwarp();
+                  for (int n = L - 1; n >= 0; --n) {
+                    double* t_ = cur;
+                    cur = old;
+                    old = t_;
+                    const int cnt = eri_tet(L - n + 1);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                      const int e = lane + 32 * i;
+                      if (32 * i >= cnt) break;
+                      if (e < cnt) {
+                        const int st = rstep[i];
+                        const int ax_ = (st >> 16) & 3;
+                        const double x = ax_ == 0 ? X : (ax_ == 1 ? Y : Z);
+                        const double val =
+                            fma(small[st >> 20], old[(st >> 8) & 255], x * old[st & 255]);
+                        cur[e] = e == 0 ? rn[n] : val;
+                      }
+                    }
+                    __syncwarp();
+                  }
+                  // W[e][mc] += sum_j M[mc][j] R[e + j]
+                  for (int jj = 0; jj < nr; ++jj)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                      if (32 * i >= nw) break;
+                      w[i] = fma(Mk[(wid[i] >> 16) + jj], cur[plus[(wid[i] & 0xFFFF) + jj]], w[i]);
+                    }
+                  __syncwarp();  // R and M are rewritten by the next primitive
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                  if (lane + 32 * i < nw) W[lane + 32 * i] = w[i];
+                __syncwarp();
+                const double* Eq = Esq + (long long)q * nab * nW;
+                for (int e = 0; e < nW; ++e)
+#pragma unroll
+                  for (int i = 0; i < 6; ++i) {
+                    if (32 * i >= no) break;
+                    acc[i] = fma(Eq[(oid[i] & 0xFFFF) + e], W[e * nsc + (oid[i] >> 16)], acc[i]);
+                  }
+                __syncwarp();
+              }
+              if (q1 == qs1) {
+#pragma unroll
+                for (int i = 0; i < 6; ++i) {
+                  const int id = lane + 32 * i;
+                  if (id >= no) break;
+                  const int ab = id / nsc, ma = ab / nsb;
+                  store(ma, ab - ma * nsb, c.bf_off + id - ab * nsc, acc[i], qs0 > 0);
+                }
+              }
+            }
+          }
+          i0 += nb * kEriWarps;
+        }
+      }
     }
   }
 }

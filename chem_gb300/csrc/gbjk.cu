@@ -1275,8 +1275,10 @@ gbjk_status gbjk_upload_b_eri3c(gbjk_ctx* ctx, const gbjk_shells* ao, const gbjk
         const int la = hao[a].l, lb = hao[b].l;
         const int ss = la + lb == 0 ? 0 : 1;
         (ss == 0 ? items : rest).push_back({p, a, b});
-        const size_t psz = 6 + 3 * (la + 1) * (lb + 1) * (la + lb + 1);
-        bra_max[ss] = std::max(bra_max[ss], (size_t)hao[a].nprim * hao[b].nprim * psz);
+        const int npp = hao[a].nprim * hao[b].nprim;
+        size_t bra = (size_t)npp * eri_pair_size(la, lb);
+        if (ss) bra += (size_t)eri_sph_chunk(la, lb, npp) * eri_sph_size(la, lb);
+        bra_max[ss] = std::max(bra_max[ss], bra);
       }
   }
   const size_t n_ss = items.size();
@@ -1324,9 +1326,19 @@ gbjk_status gbjk_upload_b_eri3c(gbjk_ctx* ctx, const gbjk_shells* ao, const gbjk
     e = cudaMemcpyToSymbol(c_eri_tuv, tuv, sizeof(tuv));
   }
   if (!e) {
-    double rodd[kEriMaxL + kEriBoysTerms + 1];
-    for (int j = 0; j <= kEriMaxL + kEriBoysTerms; ++j) rodd[j] = 1.0 / (2 * j + 1);
+    double rodd[kEriMaxL + 1];
+    for (int j = 0; j <= kEriMaxL; ++j) rodd[j] = 1.0 / (2 * j + 1);
     e = cudaMemcpyToSymbol(c_eri_rodd, rodd, sizeof(rodd));
+  }
+  void *d_boys = nullptr, *d_ket = nullptr;
+  if (!e) {
+    std::vector<double> boys(kEriBoysTable);
+    eri_boys_table(boys.data());
+    e = up(boys.data(), boys.size() * sizeof(double), &d_boys);
+  }
+  if (!e) {
+    e = cudaMalloc(&d_ket, (size_t)npx * kEriKetSize * sizeof(double));
+    if (!e) tmp.push_back(d_ket);
   }
   if (!e)
     e = cudaFuncSetAttribute(k_eri3c<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1337,6 +1349,9 @@ gbjk_status gbjk_upload_b_eri3c(gbjk_ctx* ctx, const gbjk_shells* ao, const gbjk
   if (!e && !items.empty()) {
     {
       PhaseScope ps(ctx, PH_GATHER);
+      k_eri_ket<<<cdiv(npx, 4), 128, 0, ctx->stream>>>((const EriShell*)d_ax, (int)hax.size(),
+                                                        (const double*)d_axa, npx, (double*)d_ket);
+      ctx->launches++;
       // [0, n_ss): s-s pairs, [n_ss, end): the others; grid slices of 2^30
       const size_t seg[3] = {0, n_ss, items.size()};
       for (int k = 0; k < 2; ++k)
@@ -1346,7 +1361,8 @@ gbjk_status gbjk_upload_b_eri3c(gbjk_ctx* ctx, const gbjk_shells* ao, const gbjk
           kern<<<n, 32 * kEriWarps, smem_k[k], ctx->stream>>>(
               (const EriItem*)d_items + i0, (const EriShell*)d_ao, (const EriShell*)d_ax,
               (const double*)d_aoa, (const double*)d_aoc, (const double*)d_axa,
-              (const double*)d_axc, (const int*)d_pI, (const int*)d_pJ,
+              (const double*)d_axc, (const double*)d_ket, (const double*)d_boys, (const int*)d_pI,
+              (const int*)d_pJ,
               (const unsigned char*)d_keep, nablk, (const int*)d_aoff, ctx->d_boff,
               ctx->d_panel_off, ctx->d_panelK, (const int*)d_cij, (const int*)d_cji, ctx->naux,
               ctx->d_B);

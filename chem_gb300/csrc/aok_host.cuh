@@ -47,8 +47,9 @@ struct AoKState {
   int* d_eCb = nullptr;
   SplitItem* d_items = nullptr;
   SplitJob* d_jobs = nullptr;
-  int i_ht0 = 0, i_htn = 0, i_k0 = 0, i_kn = 0, j_p0 = 0;
-  int p_nrb = 0, r_nrb = 0, r_nkt = 0, p_maxthr = 0;
+  PrepJob* d_pjobs = nullptr;
+  int i_ht0 = 0, i_htn = 0, i_k0 = 0, i_kn = 0;
+  int p_nrb = 0, r_nrb = 0, r_nkt = 0;
 
   template <class T>
   cudaError_t alloc(T** p, size_t n) {
@@ -82,6 +83,7 @@ struct AoKState {
     free_(&d_eCb);
     free_(&d_items);
     free_(&d_jobs);
+    free_(&d_pjobs);
     bytes = 0;
     precision = -1;
     ready = false;
@@ -258,7 +260,7 @@ struct AoKState {
     const int ks = sp.choose_ksplit(r_nkt, ntile);
     const int kt_per = cdiv_(r_nkt, ks);
     ksplit = cdiv_(r_nkt, kt_per);
-    if (alloc(&d_Pg, (size_t)L.ncols_total * nbf) || alloc(&d_cbi, big) ||
+    if (alloc(&d_cbi, big) ||
         alloc(&d_eoff, (size_t)2 * nbf) ||
         alloc(&d_Kpart, (size_t)ksplit * nbf * nbf) || alloc(&d_Pdig, (size_t)ptot) ||
         alloc(&d_Cbdig, (size_t)rdig) || alloc(&d_Bdig, (size_t)rdig) ||
@@ -274,24 +276,24 @@ struct AoKState {
     }
     // jobs: P rows per panel, and (once) the dense Bfit rows N; the digits of
     // the half-transformed rows M are cut from their integers
-    std::vector<SplitJob> jobs;
-    j_p0 = 0;
-    p_maxthr = 0;
+    std::vector<PrepJob> pjobs;
     for (int I = 0; I < nblk; ++I) {
-      SplitJob j;
-      j.src = d_Pg + (long long)(*L.cmoff)[I] * nbf;
+      PrepJob j;
+      j.which = 0;
+      j.off = 0;
       j.rs = 1;
       j.cs = nbf;
+      j.cm = L.d_colmap + (*L.cmoff)[I];
+      j.ncols = (*L.panelK)[I];
       j.row0 = 0;
       j.nrows = nbf;
-      j.ncols = (*L.panelK)[I];
       j.e = d_eP + (long long)I * p_nrb * 32;
       j.nrb = p_nrb;
       j.nkt = sp.nkt[I];
       j.dst = d_Pdig + p_off[I];
-      jobs.push_back(j);
-      p_maxthr = std::max(p_maxthr, (nbf / 8 + 2) * sp.nkt[I] * 32);
+      pjobs.push_back(j);
     }
+    std::vector<SplitJob> jobs;
     const int j_bd = (int)jobs.size();
     {
       SplitJob j;
@@ -405,6 +407,9 @@ struct AoKState {
     }
     i_kn = (int)items.size() - i_k0;
     if (alloc(&d_items, items.size()) || alloc(&d_jobs, jobs.size()) ||
+        alloc(&d_pjobs, pjobs.size()) ||
+        cudaMemcpy(d_pjobs, pjobs.data(), pjobs.size() * sizeof(PrepJob),
+                   cudaMemcpyHostToDevice) ||
         cudaMemcpy(d_items, items.data(), items.size() * sizeof(SplitItem),
                    cudaMemcpyHostToDevice) ||
         cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(SplitJob), cudaMemcpyHostToDevice) ||
@@ -457,14 +462,10 @@ struct AoKState {
                   int64_t* launches, std::string* err) {
     const int nbf = L.nbf;
     const long long nn = (long long)nbf * nbf;
-    k_gather_cols<<<cdiv_((long long)L.ncols_total * nbf, 256), 256, 0, st>>>(
-        dP, nbf, L.d_colmap, L.ncols_total, d_Pg);
-    (*launches)++;
     if (precision == GBJK_SPLIT_BF16) {
       gbjk_status s;
-      k_row_maxexp<<<dim3(cdiv_((long long)nbf * 32, 256), L.nblk), 256, 0, st>>>(d_jobs + j_p0);
-      k_split_tiles<<<dim3(cdiv_(p_maxthr, 256), L.nblk), 256, 0, st>>>(d_jobs + j_p0);
-      *launches += 2;
+      k_prep_rows<<<dim3(cdiv_(nbf, 8), L.nblk), 256, 0, st>>>(d_pjobs, dP, nullptr);
+      (*launches)++;
       if (cudaMemsetAsync(d_eCb, kNoExpByte, (size_t)r_nrb * 32 * 4, st) != cudaSuccess) {
         *err = "DF-AO K: memset failed";
         return GBJK_CUDA_ERROR;
@@ -475,6 +476,9 @@ struct AoKState {
       k_splitk_reduce<<<cdiv_(nn, 256), 256, 0, st>>>(d_Kpart, ksplit, nbf, -1.0, 1, dK);
       (*launches)++;
     } else {
+      k_gather_cols<<<cdiv_((long long)L.ncols_total * nbf, 256), 256, 0, st>>>(
+          dP, nbf, L.d_colmap, L.ncols_total, d_Pg);
+      (*launches)++;
       for (int t0 = 0; t0 < ht_n; t0 += (1 << 20)) {
         const int n = std::min(1 << 20, ht_n - t0);
         k_gemm_fp64<false><<<n, 256, 0, st>>>(d_groups, d_tiles + ht_0 + t0, 1.0);

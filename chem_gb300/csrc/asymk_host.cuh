@@ -45,9 +45,9 @@ struct AsymKState {
   int* d_eC = nullptr;
   int* d_eH = nullptr;
   SplitItem* d_items = nullptr;
-  SplitJob* d_jobs = nullptr;
+  PrepJob* d_jobs = nullptr;
   int i_ht0 = 0, i_htn = 0, i_k0 = 0, i_kn = 0;
-  int c_nrb = 0, h_nrb = 0, h_nkt = 0, c_maxthr = 0;
+  int c_nrb = 0, h_nrb = 0, h_nkt = 0, c_groups = 0;
   long long hdig_side = 0;
 
   template <class T>
@@ -98,8 +98,7 @@ struct AsymKState {
     // the unpadded k = (X, i) order of the oracle
     hld = prec == GBJK_SPLIT_BF16 ? nocc + (nocc & 1) : nocc;
     const size_t nbf = L.nbf;
-    if (alloc(&d_U, nbf * nocc) || alloc(&d_V, nbf * nocc) ||
-        alloc(&d_Ug, (size_t)L.ncols_total * nocc) || alloc(&d_Vg, (size_t)L.ncols_total * nocc)) {
+    if (alloc(&d_U, nbf * nocc) || alloc(&d_V, nbf * nocc)) {
       release();
       *err = "non-symmetric DF-LMO K: out of device memory";
       return GBJK_OOM;
@@ -120,7 +119,8 @@ struct AsymKState {
     const long long kdim = (long long)naux * hld;
     long long kc = kdim;
     gbjk_k_split_plan(L.nbf, L.naux, hld, &ksplit, &kc);
-    if (alloc(&d_Hu, nbf * naux * hld) || alloc(&d_Hv, nbf * naux * hld) ||
+    if (alloc(&d_Ug, (size_t)L.ncols_total * nocc) || alloc(&d_Vg, (size_t)L.ncols_total * nocc) ||
+        alloc(&d_Hu, nbf * naux * hld) || alloc(&d_Hv, nbf * naux * hld) ||
         alloc(&d_Hvf, nbf * naux * hld) || alloc(&d_Kpart, (size_t)ksplit * nbf * nbf)) {
       *err = "non-symmetric DF-LMO K: out of device memory";
       return GBJK_OOM;
@@ -232,25 +232,27 @@ struct AsymKState {
       *err = "non-symmetric DF-LMO K: out of device memory for the split path";
       return GBJK_OOM;
     }
-    std::vector<SplitJob> jobs;
+    std::vector<PrepJob> jobs;
     std::vector<SplitItem> items;
-    c_maxthr = 0;
     for (int side = 0; side < 2; ++side)
       for (int I = 0; I < nblk; ++I) {
-        SplitJob j;
-        j.src = (side ? d_Vg : d_Ug) + (long long)(*L.cmoff)[I] * nocc;
-        j.rs = 1;
-        j.cs = nocc;
+        // u: element (i, k) = U[colmap[k]][i]; v: Vt[i][colmap[k]]
+        PrepJob j;
+        j.which = side;
+        j.off = 0;
+        j.rs = side ? nbf : 1;
+        j.cs = side ? 1 : nocc;
+        j.cm = sp.dd_colmap + (*L.cmoff)[I];
+        j.ncols = (*L.panelK)[I];
         j.row0 = side * hld;
         j.nrows = nocc;
-        j.ncols = (*L.panelK)[I];
         j.e = d_eC + (long long)I * c_nrb * 32;
         j.nrb = c_nrb;
         j.nkt = sp.nkt[I];
         j.dst = d_Cdig + c_off[I];
         jobs.push_back(j);
-        c_maxthr = std::max(c_maxthr, (nocc / 8 + 2) * sp.nkt[I] * 32);
       }
+    c_groups = SplitState::prep_groups(jobs);
     // digits of the two sides of H: exponent offsets per AO function (the
     // tensor's rows, then the columns of u and of v)
     std::vector<long long> eoff((size_t)3 * nbf);
@@ -356,7 +358,7 @@ struct AsymKState {
     if (alloc(&d_items, items.size()) || alloc(&d_jobs, jobs.size()) ||
         cudaMemcpy(d_items, items.data(), items.size() * sizeof(SplitItem),
                    cudaMemcpyHostToDevice) ||
-        cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(SplitJob), cudaMemcpyHostToDevice) ||
+        cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(PrepJob), cudaMemcpyHostToDevice) ||
         cudaMemcpy(d_eoff, eoff.data(), eoff.size() * sizeof(long long), cudaMemcpyHostToDevice)) {
       *err = "non-symmetric DF-LMO K: out of memory for the work lists";
       return GBJK_OOM;
@@ -370,15 +372,10 @@ struct AsymKState {
                   std::string* err) {
     const long long nn = (long long)nbf * nbf;
     const long long gtot = (long long)ncols_total * nocc;
-    k_gather_cols<<<cdiv_(gtot, 256), 256, 0, st>>>(d_U, nocc, d_colmap, ncols_total, d_Ug);
-    k_gather_cols_t<<<cdiv_(gtot, 256), 256, 0, st>>>(d_V, nocc, nbf, d_colmap, ncols_total,
-                                                      d_Vg);
-    *launches += 2;
     if (precision == GBJK_SPLIT_BF16) {
       gbjk_status s;
-      k_row_maxexp<<<dim3(cdiv_((long long)nocc * 32, 256), 2 * nblk), 256, 0, st>>>(d_jobs);
-      k_split_tiles<<<dim3(cdiv_(c_maxthr, 256), 2 * nblk), 256, 0, st>>>(d_jobs);
-      *launches += 2;
+      k_prep_rows<<<dim3(c_groups, 2 * nblk), 256, 0, st>>>(d_jobs, d_U, d_V);
+      (*launches)++;
       if (cudaMemsetAsync(d_eH, kNoExpByte, (size_t)2 * h_nrb * 32 * 4, st) != cudaSuccess) {
         *err = "non-symmetric DF-LMO K: memset failed";
         return GBJK_CUDA_ERROR;
@@ -387,6 +384,10 @@ struct AsymKState {
       SplitState::launch_ints<true>(st, hjobs.data(), 2, launches);
       if ((s = sp.launch_gemm(st, d_items + i_k0, i_kn, launches, err))) return s;
     } else {
+      k_gather_cols<<<cdiv_(gtot, 256), 256, 0, st>>>(d_U, nocc, d_colmap, ncols_total, d_Ug);
+      k_gather_cols_t<<<cdiv_(gtot, 256), 256, 0, st>>>(d_V, nocc, nbf, d_colmap, ncols_total,
+                                                        d_Vg);
+      *launches += 2;
       auto gemm = [&](int t0, int n, bool transB) {
         for (int o = 0; o < n; o += (1 << 20)) {
           const int c = std::min(1 << 20, n - o);

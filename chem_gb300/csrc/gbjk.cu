@@ -1086,7 +1086,8 @@ gbjk_status gbjk_create(gbjk_ctx** out, const gbjk_desc* d) {
   }
   ctx->split.init(ctx->nbf, ctx->naux, ctx->nblk, ctx->bsize, ctx->boff, ctx->panelK, ctx->cmoff,
                   ctx->panel_off, ctx->colmap, ctx->blk_of);
-  ctx->split.set_dev_layout(ctx->d_panel_off, ctx->d_blk_of, ctx->d_boff, ctx->d_panelK);
+  ctx->split.set_dev_layout(ctx->d_panel_off, ctx->d_blk_of, ctx->d_boff, ctx->d_panelK,
+                            ctx->d_colmap);
   *out = ctx;
   return GBJK_OK;
 }
@@ -1763,8 +1764,7 @@ static bool fp64_occ_batched(const gbjk_ctx* ctx, int nocc) {
 
 static gbjk_status prepare_split(gbjk_ctx* ctx, int nocc) {
   if (ctx->precision != GBJK_SPLIT_BF16) return GBJK_OK;
-  return ctx->split.prepare(ctx->stream, ctx->d_B, ctx->d_Linv, ctx->d_Cg, ctx->d_Pg,
-                            ctx->pg_off, nocc, &ctx->launches, &ctx->err);
+  return ctx->split.prepare(ctx->stream, ctx->d_B, ctx->d_Linv, nocc, &ctx->launches, &ctx->err);
 }
 
 // Mixed-precision J + K.  The density rows of every panel ride along as
@@ -1775,22 +1775,6 @@ static gbjk_status run_jk_split(gbjk_ctx* ctx, const double* dP, const double* d
                                 double* dJ, double* dK) {
   const int nbf = ctx->nbf, naux = ctx->naux;
   gbjk_status s;
-  if (dJ) {
-    PhaseScope ps(ctx, PH_GATHER);
-    k_gather_panel_rows<<<dim3(cdiv(ctx->maxK, 128), nbf), 128, 0, ctx->stream>>>(
-        dP, nbf, ctx->d_blk_of, ctx->d_boff, ctx->d_panelK, ctx->d_pg_off, ctx->d_cmoff,
-        ctx->d_colmap, ctx->d_Pg);
-    CKL(PH_GATHER);
-  } else {
-    CK(cudaMemsetAsync(ctx->d_Pg, 0, (size_t)ctx->pg_total * sizeof(double), ctx->stream));
-  }
-  {
-    PhaseScope ps(ctx, PH_GATHER);
-    const long long total = (long long)ctx->ncols_total * nocc;
-    k_gather_cols<<<cdiv(total, 256), 256, 0, ctx->stream>>>(dC, nocc, ctx->d_colmap,
-                                                             ctx->ncols_total, ctx->d_Cg);
-    CKL(PH_GATHER);
-  }
   // J = (L^-1 B)^T dt needs only the half transform's density partials: with
   // overlap on (and no per-phase timing, whose events sit on one stream) it
   // runs on the side stream beside the exchange.  Where J alone fills the
@@ -1803,7 +1787,7 @@ static gbjk_status run_jk_split(gbjk_ctx* ctx, const double* dP, const double* d
                         (ctx->overlap_sms == 0 && ctx->split.j_bytes() < kOverlapJBytes));
   ctx->split.ev_ht = overlap ? ctx->ev_fork : nullptr;
   ctx->split.k_grid = overlap ? ctx->overlap_sms : 0;
-  s = ctx->split.run_k(ctx->stream, dK, &ctx->launches, &ctx->err);
+  s = ctx->split.run_k(ctx->stream, dC, dJ ? dP : nullptr, dK, &ctx->launches, &ctx->err);
   ctx->split.ev_ht = nullptr;
   ctx->split.k_grid = 0;
   if (s) return s;
@@ -1848,7 +1832,6 @@ gbjk_status gbjk_compute_jk_dev(gbjk_ctx* ctx, int kmethod, const double* dP, co
   if ((s = ensure_j_workspace(ctx))) return s;
   if (dK) {
     if (ctx->precision == GBJK_SPLIT_BF16) {
-      if ((s = ensure_c_workspace(ctx, nocc))) return s;
       if ((s = prepare_split(ctx, nocc))) return s;
       return run_jk_split(ctx, dP, dC, nocc, dJ, dK);
     }

@@ -56,12 +56,13 @@ struct Mp2State {
   SplitItem* d_items = nullptr;
   SplitJob* d_jobs = nullptr;
   int i1_0 = 0, i1_n = 0, i2_0 = 0, i2_n = 0, iz_0 = 0, iz_n = 0;
-  int jc_0 = 0, jlv_0 = 0, jh_0 = 0;
+  PrepJob* d_pjobs = nullptr;  // npts x nblk of Lo, then npts of Lv
+  int jh_0 = 0;
   int c_nrb = 0, h_nrb = 0, h_nkt = 0, lv_nrb = 0, w_nrb = 0, w_nkt = 0, ksplit = 1;
   long long hdig_stride = 0, lvdig_stride = 0, wdig_stride = 0;
   long long *d_cofs = nullptr, *d_eoff = nullptr;
   std::vector<SplitIntJob> wjobs;
-  int c_maxthr = 0;
+  int c_groups = 0, lv_groups = 0;
   // profiling
   bool profile = false;
   double ms[kNumPh] = {};
@@ -110,6 +111,7 @@ struct Mp2State {
     free_(&d_Zpart);
     free_(&d_items);
     free_(&d_jobs);
+    free_(&d_pjobs);
     free_(&d_cofs);
     free_(&d_eoff);
     resolve();
@@ -216,8 +218,8 @@ struct Mp2State {
     w_stride = (long long)naux * kw;
     const size_t nn = (size_t)naux * naux;
     if (alloc(&d_Lo, (size_t)npts * nbf * hld) || alloc(&d_Lv, (size_t)npts * nbf * vld) ||
-        alloc(&d_Cg, (size_t)npts * cg_stride) || alloc(&d_H, (size_t)npts * h_stride) ||
-        alloc(&d_W, (size_t)npts * w_stride) || alloc(&d_Z, (size_t)npts * nn) ||
+        (prec == GBJK_FP64 && alloc(&d_Cg, (size_t)npts * cg_stride)) ||
+        alloc(&d_H, (size_t)npts * h_stride) || alloc(&d_W, (size_t)npts * w_stride) || alloc(&d_Z, (size_t)npts * nn) ||
         alloc(&d_rsq, (size_t)npts * naux) || alloc(&d_E, (size_t)npts) ||
         cudaMemsetAsync(d_H, 0, (size_t)npts * h_stride * 8, st) ||
         cudaMemsetAsync(d_W, 0, (size_t)npts * w_stride * 8, st)) {
@@ -381,41 +383,47 @@ struct Mp2State {
       *err = "MP2 batch: out of device memory for the operand digits";
       return GBJK_OOM;
     }
-    // jobs
-    std::vector<SplitJob> jobs;
-    jc_0 = 0;
-    c_maxthr = 0;
+    // jobs: the gathered rows of every point's Lo and the rows of its Lv ...
+    std::vector<PrepJob> pjobs;
     for (int t = 0; t < npts; ++t)
       for (int I = 0; I < nblk; ++I) {
-        SplitJob j;
-        j.src = d_Cg + t * cg_stride + (long long)cmoff[I] * hld;
+        PrepJob j;
+        j.which = 0;
+        j.off = (long long)t * nbf * hld;
         j.rs = 1;
         j.cs = hld;
+        j.cm = sp.dd_colmap + cmoff[I];
+        j.ncols = panelK[I];
         j.row0 = co[t];
         j.nrows = ro[t];
-        j.ncols = panelK[I];
         j.e = d_eC + (long long)I * c_nrb * 32;
         j.nrb = c_nrb;
         j.nkt = sp.nkt[I];
         j.dst = d_Cdig + cdig_off[I];
-        jobs.push_back(j);
-        c_maxthr = std::max(c_maxthr, (ro[t] / 8 + 2) * sp.nkt[I] * 32);
+        pjobs.push_back(j);
       }
-    jlv_0 = (int)jobs.size();
+    c_groups = SplitState::prep_groups(pjobs);
+    std::vector<PrepJob> ljobs;
     for (int t = 0; t < npts; ++t) {
-      SplitJob j;
-      j.src = d_Lv + (long long)t * nbf * vld;
+      PrepJob j;
+      j.which = 0;
+      j.off = (long long)t * nbf * vld;
       j.rs = 1;
       j.cs = vld;
+      j.cm = nullptr;
+      j.ncols = nbf;
       j.row0 = 0;
       j.nrows = rv[t];
-      j.ncols = nbf;
       j.e = d_eLv + (long long)t * lv_nrb * 32;
       j.nrb = lv_nrb;
       j.nkt = h_nkt;
       j.dst = d_Lvdig + t * lvdig_stride;
-      jobs.push_back(j);
+      ljobs.push_back(j);
     }
+    lv_groups = SplitState::prep_groups(ljobs);
+    pjobs.insert(pjobs.end(), ljobs.begin(), ljobs.end());
+    // ... and the rows (X, i) of H
+    std::vector<SplitJob> jobs;
     jh_0 = (int)jobs.size();
     for (int t = 0; t < npts; ++t) {
       SplitJob j;
@@ -560,6 +568,9 @@ struct Mp2State {
     }
     iz_n = (int)items.size() - iz_0;
     if (alloc(&d_items, items.size()) || alloc(&d_jobs, jobs.size()) ||
+        alloc(&d_pjobs, pjobs.size()) ||
+        cudaMemcpy(d_pjobs, pjobs.data(), pjobs.size() * sizeof(PrepJob),
+                   cudaMemcpyHostToDevice) ||
         cudaMemcpy(d_items, items.data(), items.size() * sizeof(SplitItem),
                    cudaMemcpyHostToDevice) ||
         cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(SplitJob), cudaMemcpyHostToDevice) ||
@@ -597,24 +608,13 @@ struct Mp2State {
   gbjk_status run(cudaStream_t st, int nbf, int naux, int nblk, int ncols_total,
                   const int* d_colmap, SplitState& sp, int64_t* launches, std::string* err) {
     const long long nn = (long long)naux * naux;
-    {
-      Scope sc(this, kOps, st);
-      k_mp2_gather<<<dim3(cdiv_((long long)ncols_total * hld, 256), npts), 256, 0, st>>>(
-          d_Lo, (long long)nbf * hld, hld, d_colmap, ncols_total, d_Cg, cg_stride);
-      (*launches)++;
-    }
     if (precision == GBJK_SPLIT_BF16) {
       gbjk_status s;
       {
         Scope sc(this, kOps, st);
-        const int maxrows = std::max(*std::max_element(ro.begin(), ro.end()),
-                                     *std::max_element(rv.begin(), rv.end()));
-        k_row_maxexp<<<dim3(cdiv_((long long)maxrows * 32, 256), npts * nblk + npts), 256, 0, st>>>(
-            d_jobs + jc_0);
-        k_split_tiles<<<dim3(cdiv_(c_maxthr, 256), npts * nblk), 256, 0, st>>>(d_jobs + jc_0);
-        const long long lvthr = (long long)(vld / 8 + 2) * h_nkt * 32;
-        k_split_tiles<<<dim3(cdiv_(lvthr, 256), npts), 256, 0, st>>>(d_jobs + jlv_0);
-        *launches += 3;
+        k_prep_rows<<<dim3(c_groups, npts * nblk), 256, 0, st>>>(d_pjobs, d_Lo, nullptr);
+        k_prep_rows<<<dim3(lv_groups, npts), 256, 0, st>>>(d_pjobs + npts * nblk, d_Lv, nullptr);
+        *launches += 2;
       }
       {
         Scope sc(this, kT1, st);
@@ -651,6 +651,12 @@ struct Mp2State {
         (*launches)++;
       }
     } else {
+      {
+        Scope sc(this, kOps, st);
+        k_mp2_gather<<<dim3(cdiv_((long long)ncols_total * hld, 256), npts), 256, 0, st>>>(
+            d_Lo, (long long)nbf * hld, hld, d_colmap, ncols_total, d_Cg, cg_stride);
+        (*launches)++;
+      }
       auto gemm = [&](int ph, int tile0, int ntiles, int kind) {
         Scope sc(this, ph, st);
         for (int t0 = 0; t0 < ntiles; t0 += (1 << 20)) {

@@ -450,6 +450,126 @@ __device__ __forceinline__ void store_digits8(const unsigned long long (&X)[8], 
   }
 }
 
+// X = rint(|x| 2^(39-e)) and the sign of an FP64 element of a row of exponent e.
+__device__ __forceinline__ unsigned long long digit_int(double x, int e, bool* neg) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  const int E = (int)((u >> 52) & 0x7FF);
+  const unsigned long long m = (u & ((1ull << 52) - 1)) | (1ull << 52);
+  *neg = (u >> 63) != 0;
+  // m / 2^sh rounded, sh = 1036 + e - E >= 14 since |x| < 2^e
+  return E != 0 && e > -2000 ? (shr_u64(m, 1035 + e - E) + 1) >> 1 : 0;
+}
+// Element offset of digit 0 of (row r, k-tile kt, columns 8 kc .. 8 kc + 7) in
+// the slice images of an operand of nrb row blocks.
+__device__ __forceinline__ long long image_offset(int r, int kt, int kc, int nrb) {
+  return ((long long)kt * kSlices * nrb + (r >> 5)) * kImage + ((r & 31) >> 3) * 256 + kc * 64 +
+         (r & 7) * 8;
+}
+
+// Operand rows taken from a matrix by columns of a panel: row row0 + i, column k
+// is src[off + i * rs + cm[k] * cs] (cm null: k itself), src the first or second
+// base pointer of the launch (null: zeros).
+struct PrepJob {
+  int which;
+  long long off, rs, cs;
+  const int* cm;
+  int ncols, row0, nrows;
+  int* e;
+  int nrb, nkt;
+  uint16_t* dst;
+};
+
+// Row exponents and digits of such operands in one launch.  Latency is what
+// bounds it, so a block takes eight rows: all its threads find the exponents,
+// then its warps share the k-tiles and find the values in L1.  Gathering the
+// columns, the exponents and the digits were four launches: 20 -> 9 us of a
+// C10H22 build, 33 -> 19 us of a C20H42 one.
+// grid (most 8-row groups of a job + 1, njobs), block 256.
+__global__ void __launch_bounds__(256)
+    k_prep_rows(const PrepJob* __restrict__ jobs, const double* __restrict__ b0,
+                const double* __restrict__ b1) {
+  __shared__ unsigned int smx[8];
+  const PrepJob jb = jobs[blockIdx.y];
+  const int g = (jb.row0 >> 3) + blockIdx.x;
+  if (8 * g >= jb.row0 + jb.nrows) return;
+  const double* base = jb.which ? b1 : b0;
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid < 8) smx[tid] = 0;
+  __syncthreads();
+  {
+    const int i = 8 * g + (tid & 7) - jb.row0;
+    unsigned int mx = 0;
+    if (base && i >= 0 && i < jb.nrows) {
+      const double* p = base + jb.off + i * jb.rs;
+#pragma unroll 4
+      for (int k = tid >> 3; k < jb.ncols; k += 32) {
+        const long long c = jb.cm ? jb.cm[k] : k;
+        mx = max(mx, (unsigned int)(__double_as_longlong(p[c * jb.cs]) >> 52) & 0x7FF);
+      }
+    }
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+    if (lane < 8 && mx) atomicMax(&smx[lane], mx);
+  }
+  __syncthreads();
+  const int rr = lane & 7, kc = lane >> 3, r = 8 * g + rr, i = r - jb.row0;
+  if (i < 0 || i >= jb.nrows) return;
+  const int e = smx[rr] ? (int)smx[rr] - 1022 : -2000;
+  if (tid < 8) jb.e[r] = e;
+  const double* p = base ? base + jb.off + i * jb.rs : nullptr;
+  for (int kt = tid >> 5; kt < jb.nkt; kt += 8) {
+    unsigned long long X[8];
+    bool neg[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int k = kt * 32 + kc * 8 + j;
+      double x = 0.0;
+      if (p && k < jb.ncols) x = p[(jb.cm ? (long long)jb.cm[k] : k) * jb.cs];
+      X[j] = digit_int(x, e, &neg[j]);
+    }
+    store_digits8(X, neg, jb.dst + image_offset(r, kt, kc, jb.nrb), (long long)jb.nrb * kImage);
+  }
+}
+
+// Row exponents and digits of SplitJob rows that lie contiguous in memory
+// (cs = 1): one warp per 8-row group and all its k-tiles, the second reading from
+// L1 or L2.  HBM bounds it: 8 bytes an element read, 10 written.  Exponents and
+// digits in a launch each read the tensor from HBM twice: 862 -> 564 us for the
+// 1.5e8 elements of a batch of the 1200-function synthetic tensor.
+// grid (ceil(most groups / 8), njobs), block 256.
+__global__ void __launch_bounds__(256) k_split_rows(const SplitJob* __restrict__ jobs) {
+  const SplitJob jb = jobs[blockIdx.y];
+  const int g = (jb.row0 >> 3) + blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (8 * g >= jb.row0 + jb.nrows) return;
+  const int lane = threadIdx.x & 31, rr = lane & 7, kc = lane >> 3;
+  const int r = 8 * g + rr, i = r - jb.row0;
+  const bool in = i >= 0 && i < jb.nrows;
+  const double* p = jb.src + (long long)max(i, 0) * jb.rs + kc * 8;
+  const int ncols = in ? (int)jb.ncols : 0;
+  unsigned int mx = 0;
+#pragma unroll 2
+  for (int kt = 0; kt < jb.nkt; ++kt)
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (kt * 32 + kc * 8 + j < ncols)
+        mx = max(mx, (unsigned int)(__double_as_longlong(p[kt * 32 + j]) >> 52) & 0x7FF);
+  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+  if (!in) return;
+  const int e = mx ? (int)mx - 1022 : -2000;
+  if (kc == 0) jb.e[r] = e;
+  for (int kt = 0; kt < jb.nkt; ++kt) {
+    unsigned long long X[8];
+    bool neg[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const double x = kt * 32 + kc * 8 + j < ncols ? p[kt * 32 + j] : 0.0;
+      X[j] = digit_int(x, e, &neg[j]);
+    }
+    store_digits8(X, neg, jb.dst + image_offset(r, kt, kc, jb.nrb), (long long)jb.nrb * kImage);
+  }
+}
+
 // Slice images.  One warp per (8-row group, k-tile): lane (rr, kc) =
 // (lane & 7, lane >> 3) handles row 8g + rr, columns 32kt + 8kc .. +7, so
 // each warp writes 512 contiguous bytes per slice.  grid (warps/8, njobs).
@@ -471,18 +591,9 @@ __global__ void k_split_tiles(const SplitJob* __restrict__ jobs) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const long long c = (long long)kt * 32 + kc * 8 + j;
-    const double x = c < jb.ncols ? src[c * jb.cs] : 0.0;
-    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-    const int E = (int)((u >> 52) & 0x7FF);
-    const unsigned long long m = (u & ((1ull << 52) - 1)) | (1ull << 52);
-    // X = rint(m / 2^sh); sh >= 14 since |x| < 2^er
-    X[j] = E != 0 && er > -2000 ? (shr_u64(m, 1035 + er - E) + 1) >> 1 : 0;
-    neg[j] = (u >> 63) != 0;
+    X[j] = digit_int(c < jb.ncols ? src[c * jb.cs] : 0.0, er, &neg[j]);
   }
-  store_digits8(X, neg,
-                jb.dst + ((long long)kt * kSlices * jb.nrb + (r >> 5)) * kImage +
-                    ((r & 31) >> 3) * 256 + kc * 64 + rr * 8,
-                (long long)jb.nrb * kImage);
+  store_digits8(X, neg, jb.dst + image_offset(r, kt, kc, jb.nrb), (long long)jb.nrb * kImage);
 }
 
 // Digit slices of an operand whose elements are the integers V of a split
@@ -596,10 +707,7 @@ __global__ void k_split_ints(const __grid_constant__ SplitIntJobs jobs) {
     for (int j = 0; j < 8; ++j)
       X[j] = sh[j] >= 1 ? (shr_u64(X[j], sh[j] - 1) + 1) >> 1 : X[j] << min(-sh[j], 63);
   }
-  store_digits8(X, neg,
-                jb.dst + ((long long)kt * kSlices * jb.nrb + (r >> 5)) * kImage +
-                    ((r & 31) >> 3) * 256 + kc * 64 + rr * 8,
-                (long long)jb.nrb * kImage);
+  store_digits8(X, neg, jb.dst + image_offset(r, kt, kc, jb.nrb), (long long)jb.nrb * kImage);
 }
 
 // ------------------------------------------------------------ the GEMM

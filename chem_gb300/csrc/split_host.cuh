@@ -55,7 +55,7 @@ struct SplitState {
   std::vector<int> colmap, blk_of;
   // the context's device copies of the panel layout (not owned)
   const long long* dd_panel_off = nullptr;
-  const int *dd_blk_of = nullptr, *dd_boff = nullptr, *dd_panelK = nullptr;
+  const int *dd_blk_of = nullptr, *dd_boff = nullptr, *dd_panelK = nullptr, *dd_colmap = nullptr;
   uint16_t* d_Aslices = nullptr;
   // auxiliary batching: xb auxiliary rows per batch (nbatch > 1 streams the
   // half transform and the exchange batch by batch; A digits per batch)
@@ -68,7 +68,6 @@ struct SplitState {
   // round trip and digit pass they replace.
   bool hfuse = false, hfuse_eff = false;
   SplitJob* d_bjobs = nullptr;  // A-digit jobs, nbatch * nbf (one per (batch, mu))
-  int bjob_maxthr = 0;
   std::vector<long long> a_off, eA_off;
   std::vector<int> a_nrb, nkt;
   int* d_eA = nullptr;
@@ -90,13 +89,12 @@ struct SplitState {
   int maxb = 0;
   SplitItem* d_items = nullptr;
   int ht_nitems = 0, k_nitems = 0;
-  SplitJob* d_jobs = nullptr;  // [0,nblk): C rows, [nblk,2nblk): P rows
+  PrepJob* d_jobs = nullptr;  // [0,nblk): C rows, [nblk,2nblk): P rows
   std::vector<SplitIntJob> hjobs;  // digits of H, one per distinct batch size
   long long* d_eoff = nullptr;     // their exponent offsets per AO function
-  int c_maxthreads = 0, c_maxrows = 0;
+  int c_groups = 0;  // most 8-row groups of a job
   long long h_threads = 0;
   int* d_err = nullptr;
-  const double* d_Cg = nullptr;
   int nsm = 148;
   bool profile = false;
   // set by the caller for one build: event recorded right after the half
@@ -114,7 +112,9 @@ struct SplitState {
   int64_t nl[4] = {0, 0, 0, 0};
   std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> pending;
 
-  void set_dev_layout(const long long* po, const int* blk_of, const int* bo, const int* pk) {
+  void set_dev_layout(const long long* po, const int* blk_of, const int* bo, const int* pk,
+                      const int* cm) {
+    dd_colmap = cm;
     dd_panel_off = po;
     dd_blk_of = blk_of;
     dd_boff = bo;
@@ -241,6 +241,13 @@ struct SplitState {
   };
 
   static int cdiv_(long long a, long long b) { return (int)((a + b - 1) / b); }
+  // most 8-row groups of a job: the grid of k_prep_rows
+  static int prep_groups(const std::vector<PrepJob>& jobs) {
+    int g = 1;
+    for (const PrepJob& j : jobs)
+      if (j.nrows) g = std::max(g, (j.row0 + j.nrows + 7) / 8 - j.row0 / 8);
+    return g;
+  }
   // digits of operands left as integers by a split GEMM
   template <bool kFull>
   static void launch_ints(cudaStream_t st, const SplitIntJob* jobs, int n, int64_t* launches) {
@@ -630,7 +637,6 @@ struct SplitState {
     if (nbatch == 1) {
       // one job per AO function: its naux rows (m, y) at m * apitch + y
       std::vector<SplitJob> jobs(nbf);
-      long long maxthr = 0;
       for (int I = 0; I < nblk; ++I)
         for (int m = 0; m < bsize[I]; ++m) {
           SplitJob& j = jobs[boff[I] + m];
@@ -644,7 +650,6 @@ struct SplitState {
           j.nrb = a_nrb[I];
           j.nkt = nkt[I];
           j.dst = d_Aslices + a_off[I];
-          maxthr = std::max(maxthr, (long long)(naux / 8 + 2) * j.nkt * 32);
         }
       SplitJob* dj = nullptr;
       if (alloc(&dj, jobs.size()) != cudaSuccess) {
@@ -654,16 +659,14 @@ struct SplitState {
       cudaMemcpy(dj, jobs.data(), jobs.size() * sizeof(SplitJob), cudaMemcpyHostToDevice);
       {
         Scope sc(this, 2, st);
-        k_row_maxexp<<<dim3(cdiv_((long long)naux * 32, 256), nbf), 256, 0, st>>>(dj);
-        k_split_tiles<<<dim3(cdiv_(maxthr, 256), nbf), 256, 0, st>>>(dj);
-        *launches += 2;
+        k_split_rows<<<dim3(cdiv_(naux / 8 + 2, 8), nbf), 256, 0, st>>>(dj);
+        (*launches)++;
       }
       cudaStreamSynchronize(st);
       cudaFree(dj);
     } else {
       // one job per (batch, AO function): rows (m, y) of its panel
       std::vector<SplitJob> jobs((size_t)nbatch * nbf);
-      bjob_maxthr = 0;
       for (int b = 0; b < nbatch; ++b) {
         const int Y0 = b * xb, xbc = std::min(xb, naux - Y0);
         for (int I = 0; I < nblk; ++I)
@@ -679,7 +682,6 @@ struct SplitState {
             j.nrb = a_nrb[I];
             j.nkt = nkt[I];
             j.dst = d_Aslices + a_off[I];
-            bjob_maxthr = std::max(bjob_maxthr, (xbc / 8 + 2) * nkt[I] * 32);
           }
       }
       if (alloc(&d_bjobs, jobs.size()) != cudaSuccess) {
@@ -800,7 +802,7 @@ struct SplitState {
     k_fill_int<<<(int)std::min<size_t>(cdiv_((long long)nEs, 256), 4 * nsm), 256, 0, st>>>(
         d_eHs, (long long)nEs, -2000);
     std::vector<SplitItem> items;
-    std::vector<SplitJob> jobs(2 * nblk);
+    std::vector<PrepJob> jobs(2 * nblk);
     hjobs.clear();
     std::vector<long long> eoff(2 * sizes.size() * nbf);
     plans.clear();
@@ -937,33 +939,32 @@ struct SplitState {
     ht_nitems = plans[0].nht;
     ks_eff = plans[0].ksplit;
     k_nitems = plans[0].nk;
-    c_maxthreads = 0;
-    c_maxrows = std::max(nocc_, maxb);
     for (int I = 0; I < nblk; ++I) {
-      SplitJob& pj = jobs[nblk + I];  // density rows: Pg panel rows (none when batched)
-      pj.src = nullptr;               // set per build
-      pj.rs = panelK[I];
-      pj.cs = 1;
-      pj.row0 = nocc_;
-      pj.nrows = jfused ? bsize[I] : 0;
-      pj.ncols = panelK[I];
-      pj.e = d_eC + (long long)I * c_nrb * 32;
-      pj.nrb = c_nrb;
-      pj.nkt = nkt[I];
-      pj.dst = d_Cslices + c_off[I];
-      SplitJob& j = jobs[I];
-      j.src = nullptr;  // set per build (Cg pointer owned by the context)
+      // rows of C: element (i, k) = C[colmap[k]][i]; then the density rows of the
+      // panel's functions: P[boff + m][colmap[k]] (none when batched)
+      PrepJob j;
+      j.which = 0;
+      j.off = 0;
       j.rs = 1;
       j.cs = nocc_;
+      j.cm = dd_colmap + cmoff[I];
+      j.ncols = panelK[I];
       j.row0 = 0;
       j.nrows = nocc_;
-      j.ncols = panelK[I];
       j.e = d_eC + (long long)I * c_nrb * 32;
       j.nrb = c_nrb;
       j.nkt = nkt[I];
       j.dst = d_Cslices + c_off[I];
-      c_maxthreads = std::max(c_maxthreads, ((nocc_ + maxb) / 8 + 2) * nkt[I] * 32);
+      jobs[I] = j;
+      j.which = 1;
+      j.off = (long long)boff[I] * nbf;
+      j.rs = nbf;
+      j.cs = 1;
+      j.row0 = nocc_;
+      j.nrows = jfused ? bsize[I] : 0;
+      jobs[nblk + I] = j;
     }
+    c_groups = prep_groups(jobs);
     if (alloc(&d_items, items.size()) != cudaSuccess || alloc(&d_jobs, jobs.size()) != cudaSuccess) {
       release_build();
       *err = "split path: out of memory for the work lists";
@@ -971,41 +972,25 @@ struct SplitState {
     }
     cudaMemcpy(d_items, items.data(), items.size() * sizeof(SplitItem), cudaMemcpyHostToDevice);
     cudaMemcpy(d_eoff, eoff.data(), eoff.size() * sizeof(long long), cudaMemcpyHostToDevice);
-    host_jobs = jobs;
-    jobs_cg = jobs_pg = nullptr;
+    cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(PrepJob), cudaMemcpyHostToDevice);
     nocc = nocc_;
     return GBJK_OK;
   }
-  std::vector<SplitJob> host_jobs;
-  const double* jobs_cg = nullptr;
-  const double* jobs_pg = nullptr;
 
-  gbjk_status prepare(cudaStream_t st, const double* d_B, const double* d_Linv,
-                      const double* d_Cg_, const double* d_Pg, const std::vector<long long>& pg_off,
-                      int nocc_, int64_t* launches, std::string* err) {
+  gbjk_status prepare(cudaStream_t st, const double* d_B, const double* d_Linv, int nocc_,
+                      int64_t* launches, std::string* err) {
     gbjk_status s;
     if (!b_ready && (s = prepare_b(st, d_B, d_Linv, launches, err))) return s;
     if (nocc != nocc_ && (s = prepare_nocc(st, nocc_, err))) return s;
-    if (jobs_cg != d_Cg_ || jobs_pg != d_Pg) {
-      for (int I = 0; I < nblk; ++I) {
-        host_jobs[I].src = d_Cg_ + (long long)cmoff[I] * nocc_;
-        host_jobs[nblk + I].src = d_Pg + pg_off[I];
-      }
-      jobs_cg = d_Cg_;
-      jobs_pg = d_Pg;
-      if (cudaMemcpy(d_jobs, host_jobs.data(), host_jobs.size() * sizeof(SplitJob),
-                     cudaMemcpyHostToDevice) != cudaSuccess) {
-        *err = "split path: job upload failed";
-        return GBJK_CUDA_ERROR;
-      }
-    }
     return GBJK_OK;
   }
 
   bool fused_j() const { return nbatch == 1; }
 
   // --- per build ------------------------------------------------------------
-  gbjk_status run_k(cudaStream_t st, double* dK, int64_t* launches, std::string* err) {
+  // dC: nbf x nocc; dP: nbf x nbf, or null (no density partials)
+  gbjk_status run_k(cudaStream_t st, const double* dC, const double* dP, double* dK,
+                    int64_t* launches, std::string* err) {
     gbjk_status s;
     // the flag a timed-out wait sets is per build: cleared at its start
     if (cudaMemsetAsync(d_err, 0, sizeof(int), st) != cudaSuccess) {
@@ -1014,18 +999,16 @@ struct SplitState {
     }
     {
       Scope sc(this, 2, st);
-      k_row_maxexp<<<dim3(cdiv_((long long)c_maxrows * 32, 256), 2 * nblk), 256, 0, st>>>(d_jobs);
-      k_split_tiles<<<dim3(cdiv_((long long)c_maxthreads, 256), 2 * nblk), 256, 0, st>>>(d_jobs);
-      *launches += 2;
+      k_prep_rows<<<dim3(c_groups, 2 * nblk), 256, 0, st>>>(d_jobs, dC, dP);
+      (*launches)++;
     }
     for (int b = 0; b < nbatch; ++b) {
       const BatchPlan& pl = plans[(b == nbatch - 1 && plans.size() > 1) ? 1 : 0];
       if (nbatch > 1) {
         Scope sc(this, 2, st);
         const SplitJob* bj = d_bjobs + (size_t)b * nbf;
-        k_row_maxexp<<<dim3(cdiv_((long long)pl.xbc * 32, 256), nbf), 256, 0, st>>>(bj);
-        k_split_tiles<<<dim3(cdiv_((long long)bjob_maxthr, 256), nbf), 256, 0, st>>>(bj);
-        *launches += 2;
+        k_split_rows<<<dim3(cdiv_(pl.xbc / 8 + 2, 8), nbf), 256, 0, st>>>(bj);
+        (*launches)++;
       }
       if (nbatch > 1 && !hfuse_eff && pad32(pl.xbc) != pl.xbc) {
         // the last batch's H layout reuses slots the full batches wrote:

@@ -889,8 +889,8 @@ gbjk_status launch_gemm(gbjk_ctx* ctx, int tile0, int ntiles, bool transB, doubl
 gbjk_status filter(gbjk_ctx* ctx, double* M, cudaStream_t st) {
   if (ctx->eps <= 0) return GBJK_OK;
   PhaseScope ps(ctx, PH_FILTER);
-  k_block_filter<<<dim3(ctx->nblk, ctx->nblk), 128, 0, st>>>(M, ctx->nbf, ctx->d_boff,
-                                                                      ctx->eps);
+  k_block_filter<<<cdiv((long long)ctx->nblk * ctx->nblk, 8), 256, 0, st>>>(
+      M, ctx->nbf, ctx->d_boff, ctx->nblk, ctx->eps);
   CKL(PH_FILTER);
   return GBJK_OK;
 }
@@ -1809,8 +1809,8 @@ static gbjk_status run_jk_split(gbjk_ctx* ctx, const double* dP, const double* d
     }
     if (ctx->eps > 0) {
       PhaseScope ps(ctx, PH_FILTER);
-      k_block_filter<<<dim3(ctx->nblk, ctx->nblk), 128, 0, js>>>(dJ, ctx->nbf, ctx->d_boff,
-                                                                 ctx->eps);
+      k_block_filter<<<cdiv((long long)ctx->nblk * ctx->nblk, 8), 256, 0, js>>>(
+          dJ, ctx->nbf, ctx->d_boff, ctx->nblk, ctx->eps);
       CKL(PH_FILTER);
     }
     if (overlap) CK(cudaEventRecord(ctx->ev_join, js));
@@ -2528,6 +2528,7 @@ extern "C" gbjk_status gbjk_compute_j_noalloc(const gbjk_desc* d, const int* d_c
   k_j_colsum<<<dim3(cdiv(std::max(maxK, 1), 32), nbf), 128, 0, st>>>(
       d_B, poff, blk_of, boff, panelK, cmoff, d_colmap, h, nbf, naux, d_J);
   if (d->filter_eps > 0)
-    k_block_filter<<<dim3(nblk, nblk), 128, 0, st>>>(d_J, nbf, boff, d->filter_eps);
+    k_block_filter<<<cdiv((long long)nblk * nblk, 8), 256, 0, st>>>(d_J, nbf, boff, nblk,
+                                                                    d->filter_eps);
   return ck(cudaGetLastError(), "J kernels");
 }

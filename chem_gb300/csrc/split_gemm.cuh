@@ -570,6 +570,46 @@ __global__ void __launch_bounds__(256) k_split_rows(const SplitJob* __restrict__
   }
 }
 
+// Row exponents and digits of SplitJob rows that lie side by side (rs = 1, row0 =
+// 0): a block takes 32 rows, whose columns are segments of 256 bytes, finds the
+// exponents and reads the values again from L1 or L2 for the digits.  HBM bounds
+// it (45 + 115 us as two launches, 140 as one, for the 3.8e7 elements of the half
+// transforms of an eight-point C8H18 batch).
+// grid (ceil(most rows / 32), njobs), block 256.
+__global__ void __launch_bounds__(256) k_split_cols(const SplitJob* __restrict__ jobs) {
+  __shared__ unsigned int smx[32];
+  const SplitJob jb = jobs[blockIdx.y];
+  const long long r0 = (long long)blockIdx.x * 32;
+  if (r0 >= jb.nrows) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (w == 0) smx[lane] = 0;
+  __syncthreads();
+  if (r0 + lane < jb.nrows) {
+    const double* p = jb.src + r0 + lane;
+    unsigned int mx = 0;
+#pragma unroll 4
+    for (int k = w; k < jb.ncols; k += 8)
+      mx = max(mx, (unsigned int)(__double_as_longlong(p[k * jb.cs]) >> 52) & 0x7FF);
+    if (mx) atomicMax(&smx[lane], mx);
+  }
+  __syncthreads();
+  if (w == 0 && r0 + lane < jb.nrows) jb.e[r0 + lane] = smx[lane] ? (int)smx[lane] - 1022 : -2000;
+  const int rr = lane & 7, kc = lane >> 3;
+  for (int it = w; it < 4 * jb.nkt; it += 8) {
+    const int kt = it >> 2, i = 8 * (it & 3) + rr, r = (int)r0 + i;
+    if (r >= jb.nrows) continue;
+    const int e = smx[i] ? (int)smx[i] - 1022 : -2000;
+    unsigned long long X[8];
+    bool neg[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const long long k = kt * 32 + kc * 8 + j;
+      X[j] = digit_int(k < jb.ncols ? jb.src[k * jb.cs + r] : 0.0, e, &neg[j]);
+    }
+    store_digits8(X, neg, jb.dst + image_offset(r, kt, kc, jb.nrb), (long long)jb.nrb * kImage);
+  }
+}
+
 // Slice images.  One warp per (8-row group, k-tile): lane (rr, kc) =
 // (lane & 7, lane >> 3) handles row 8g + rr, columns 32kt + 8kc .. +7, so
 // each warp writes 512 contiguous bytes per slice.  grid (warps/8, njobs).

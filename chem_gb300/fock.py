@@ -487,8 +487,8 @@ class JKEngine:
         n = len(lo)
         ro = np.array([a.shape[1] for a in lo], np.int32)
         rv = np.array([a.shape[1] for a in lv], np.int32)
-        dpp = C.POINTER(C.c_double) * n
-        plo, plv = dpp(*[_dp(a) for a in lo]), dpp(*[_dp(a) for a in lv])
+        dpp = C.POINTER(C.POINTER(C.c_double))
+        plo, plv = (C.cast((C.c_void_p * n)(*[a.ctypes.data for a in v]), dpp) for v in (lo, lv))
         self._check(lib().gbjk_mp2_set_factors(self.h, n, ro.ctypes.data_as(C.POINTER(C.c_int)), plo,
                                                rv.ctypes.data_as(C.POINTER(C.c_int)), plv),
                     "gbjk_mp2_set_factors")

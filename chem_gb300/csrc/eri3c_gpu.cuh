@@ -56,11 +56,13 @@ __constant__ int c_eri_tuv[kEriNR];
 __constant__ double c_eri_rodd[kEriMaxL + 1];
 
 struct EriShell {
-  int l, nprim, prim0, bf_off;
+  int l, nprim, prim0, bf_off, blk;  // blk: auxiliary block (auxiliary shells)
   double A[3];
 };
+// AO shells a, b of block pair p with the auxiliary blocks [A0, A1), of their
+// shells those with a momentum in the mask ls
 struct EriItem {
-  int p, a, b;
+  int p, a, b, A0, A1, ls;
 };
 
 __device__ __forceinline__ int eri_tet(int n) { return n * (n + 1) * (n + 2) / 6; }
@@ -373,6 +375,19 @@ __device__ __forceinline__ int eri_r_step(int e) {
 __host__ __device__ constexpr int eri_pair_size(int la, int lb) {
   return 6 + 3 * (la + 1) * (lb + 1) * (la + lb + 1);
 }
+// FP64 warp instructions of a primitive pair of angular momentum Lb with a
+// primitive of an auxiliary shell of lc, about: Boys values, R levels, W, and
+// the results' share; what the work items are balanced by
+inline double eri_cost(int la, int lb, int lc) {
+  auto tet = [](int n) { return n * (n + 1) * (n + 2) / 6; };
+  auto warps = [](int n) { return (n + 31) / 32; };
+  const int L = la + lb + lc, nsc = 2 * lc + 1;
+  double c = 4.0 + L;
+  for (int l = 1; l <= L; ++l) c += 2 * warps(tet(l + 1));
+  c += warps(tet(la + lb + 1) * nsc) * tet(lc + 1);
+  c += warps((2 * la + 1) * (2 * lb + 1) * nsc) * tet(la + lb + 1);
+  return c;
+}
 // doubles of its Hermite -> spherical (a, b) matrix (not for s-s pairs)
 __host__ __device__ constexpr int eri_sph_size(int la, int lb) {
   return (2 * la + 1) * (2 * lb + 1) * ((la + lb + 1) * (la + lb + 2) * (la + lb + 3) / 6);
@@ -384,8 +399,8 @@ __host__ __device__ constexpr int eri_sph_chunk(int la, int lb, int npp) {
   return n < npp ? n : npp;
 }
 
-// One block per AO shell pair (a, b); its warps take the kept auxiliary shells
-// in turn.  What bounds it is the FP64 pipe, where a warp instruction costs 16
+// One block per AO shell pair (a, b) and range of auxiliary blocks; its warps
+// take the kept shells of the range in turn.  What bounds it is the FP64 pipe, where a warp instruction costs 16
 // clocks however few lanes take part, so every phase spreads over the lanes:
 //   Boys values   lanes over the (shell, primitive pair, primitive)
 //                 combinations of up to 64 at once, several shells together
@@ -396,7 +411,8 @@ __host__ __device__ constexpr int eri_sph_chunk(int la, int lb, int npp) {
 // SS: the launch holds only s-s shell pairs (lanes over primitive pairs),
 // else only the other pairs; two kernels with half the code each keep the
 // instruction working set of a block small.  Six waters / jkfit: s-s 13.1 -> 4.2
-// ms, the others 34.4 -> 8.4 ms against lanes over e and over cartesian pairs.
+// ms, the others 34.4 -> 8.4 ms against lanes over e and over cartesian pairs,
+// and 2.6 and 3.7 ms with the work in even items.
 template <bool SS>
 __global__ void __launch_bounds__(32 * kEriWarps, 4)
     k_eri3c(const EriItem* __restrict__ items, const EriShell* __restrict__ ao,
@@ -412,7 +428,7 @@ __global__ void __launch_bounds__(32 * kEriWarps, 4)
   extern __shared__ double sm[];
   __shared__ unsigned char plus[kEriNW * kEriNKet];  // index of e + j (Hermite indices)
   __shared__ int list[kEriList];                     // kept auxiliary shells
-  __shared__ int nlist, next_A, next_s;
+  __shared__ int nlist, next_s;
   __shared__ double small[kEriMaxL];  // 0, 1, .. (a conversion is an FP64 instruction too)
   const EriItem it = items[blockIdx.x];
   const EriShell a = ao[it.a], b = ao[it.b];
@@ -525,30 +541,29 @@ __global__ void __launch_bounds__(32 * kEriWarps, 4)
       __syncthreads();
     }
     // kept auxiliary shells, kEriList of them at a time
-    if (threadIdx.x == 0) next_A = next_s = 0;
+    const int s_end = ablk_shell_off[it.A1];
+    if (threadIdx.x == 0) next_s = ablk_shell_off[it.A0];
     for (;;) {
       __syncthreads();
-      if (threadIdx.x == 0) {
-        int n = 0, A = next_A, s = next_s;
-        while (A < nablk && n < kEriList) {
-          if (!keep[(long long)it.p * nablk + A]) {
-            ++A;
-            s = 0;
-            continue;
+      if (warp == 0) {
+        int n = 0, s = next_s;
+        for (; s < s_end && n + 32 <= kEriList; s += 32) {
+          bool in = s + lane < s_end;
+          if (in) {
+            const EriShell& c = ax[s + lane];
+            in = (it.ls >> c.l & 1) && keep[(long long)it.p * nablk + c.blk];
           }
-          const int s0 = ablk_shell_off[A], ns = ablk_shell_off[A + 1] - s0;
-          while (s < ns && n < kEriList) list[n++] = s0 + s++;
-          if (s == ns) {
-            ++A;
-            s = 0;
-          }
+          const unsigned int m = __ballot_sync(0xffffffffu, in);
+          if (in) list[n + __popc(m & ((1u << lane) - 1))] = s + lane;
+          n += __popc(m);
         }
-        nlist = n;
-        next_A = A;
-        next_s = s;
+        if (lane == 0) {
+          nlist = n;
+          next_s = s;
+        }
       }
       __syncthreads();
-      if (nlist == 0) break;
+      if (nlist == 0 && next_s >= s_end) break;
       if constexpr (SS) {
         for (int i = warp; i < nlist; i += kEriWarps) {
           const EriShell c = ax[list[i]];

@@ -532,40 +532,59 @@ __global__ void __launch_bounds__(256)
 }
 
 // Row exponents and digits of SplitJob rows that lie contiguous in memory
-// (cs = 1): one warp per 8-row group and all its k-tiles, the second reading from
-// L1 or L2.  HBM bounds it: 8 bytes an element read, 10 written.  Exponents and
-// digits in a launch each read the tensor from HBM twice: 862 -> 564 us for the
-// 1.5e8 elements of a batch of the 1200-function synthetic tensor.
+// (cs = 1): one warp per 8-row group and all its k-tiles, the second time from L1
+// or L2.  8 bytes an element come from HBM and 10 go there.  The lanes read along
+// a row and pass a tile through shared memory to the lanes of the image, the next
+// one already on its way: their own loads touch 16 lines an instruction, and the
+// L1 tags bound both passes.  A batch of the 1200-function synthetic tensor (1.5e8
+// elements): 862 us with exponents and digits in a launch each, 564 with the
+// image's loads in both passes, 500 in the second one, 474 so.
 // grid (ceil(most groups / 8), njobs), block 256.
 __global__ void __launch_bounds__(256) k_split_rows(const SplitJob* __restrict__ jobs) {
+  __shared__ double tile[8][8][33];  // per warp; the odd row length spreads the banks
+  double(*t)[33] = tile[threadIdx.x >> 5];
   const SplitJob jb = jobs[blockIdx.y];
   const int g = (jb.row0 >> 3) + blockIdx.x * 8 + (threadIdx.x >> 5);
   if (8 * g >= jb.row0 + jb.nrows) return;
   const int lane = threadIdx.x & 31, rr = lane & 7, kc = lane >> 3;
-  const int r = 8 * g + rr, i = r - jb.row0;
-  const bool in = i >= 0 && i < jb.nrows;
-  const double* p = jb.src + (long long)max(i, 0) * jb.rs + kc * 8;
-  const int ncols = in ? (int)jb.ncols : 0;
-  unsigned int mx = 0;
+  const int i0 = 8 * g - jb.row0, ncols = (int)jb.ncols, rs = (int)jb.rs;
+  // rows [q0, q1) of the group are the job's; the others read as the nearest
+  const int q0 = max(0, -i0), q1 = min(8, jb.nrows - i0);
+  const double* const p = jb.src + (long long)i0 * jb.rs;
+  unsigned int mx[8] = {};
 #pragma unroll 2
-  for (int kt = 0; kt < jb.nkt; ++kt)
+  for (int k = lane; k < ncols; k += 32)
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (kt * 32 + kc * 8 + j < ncols)
-        mx = max(mx, (unsigned int)(__double_as_longlong(p[kt * 32 + j]) >> 52) & 0x7FF);
-  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-  if (!in) return;
-  const int e = mx ? (int)mx - 1022 : -2000;
-  if (kc == 0) jb.e[r] = e;
+    for (int q = 0; q < 8; ++q)
+      mx[q] = max(mx[q], (unsigned int)(__double_as_longlong(
+                             p[min(max(q, q0), q1 - 1) * rs + k]) >> 52) & 0x7FF);
+  unsigned int m = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const unsigned int w = __reduce_max_sync(0xffffffffu, mx[q]);
+    if (rr == q) m = w;
+  }
+  const int e = m ? (int)m - 1022 : -2000, r = 8 * g + rr;
+  const bool mine = rr >= q0 && rr < q1;
+  if (mine && kc == 0) jb.e[r] = e;
+  double v[8];  // the next tile's column of each row
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    v[q] = lane < ncols ? p[min(max(q, q0), q1 - 1) * rs + lane] : 0.0;
   for (int kt = 0; kt < jb.nkt; ++kt) {
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t[q][lane] = v[q];
+    __syncwarp();
+    const int k = kt * 32 + 32 + lane;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      v[q] = k < ncols ? p[min(max(q, q0), q1 - 1) * rs + k] : 0.0;
+    if (!mine) continue;
     unsigned long long X[8];
     bool neg[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const double x = kt * 32 + kc * 8 + j < ncols ? p[kt * 32 + j] : 0.0;
-      X[j] = digit_int(x, e, &neg[j]);
-    }
+    for (int j = 0; j < 8; ++j) X[j] = digit_int(t[rr][kc * 8 + j], e, &neg[j]);
     store_digits8(X, neg, jb.dst + image_offset(r, kt, kc, jb.nrb), (long long)jb.nrb * kImage);
   }
 }

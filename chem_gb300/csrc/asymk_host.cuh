@@ -14,7 +14,7 @@
 // K = -(Bfit u)(Bfit v)^T over k = (Y, i): both half transforms as one split
 // GEMM over the columns [u | v] (one 96-wide tile holds up to 48 vectors of
 // each side; a tile per side computed twice the products and read the tensor's
-// digits twice: 614 us against 300 for C14H30, 37 vectors), integers out, then
+// digits twice: 614 us against 345 for C14H30, 37 vectors), integers out, then
 // the exchange over all tiles, split over k.
 #pragma once
 #include <algorithm>

@@ -36,9 +36,8 @@ using namespace gbjk;
 
 // SMs the mixed-path exchange GEMM leaves to the concurrent J column sums
 // unless gbjk_set_overlap says otherwise: 0, the exchange takes every SM and
-// the J blocks fill the registers and shared memory its CTAs leave free
-// (a build through the host call: C20H42 1.89 ms against 1.92 in order, C10H22
-// 0.403 against 0.422, five waters 0.164 against 0.182).
+// the J blocks fill the registers and shared memory its CTAs leave free (five
+// waters, a build through the host call: 155 us against 166 in order)
 constexpr int kDefaultOverlapSms = 0;
 // ... as long as J's tensor copy is smaller than this
 constexpr size_t kOverlapJBytes = size_t(384) << 20;

@@ -454,6 +454,12 @@ gbjk_status ensure_k_workspace(gbjk_ctx* ctx, int nocc) {
     groups.push_back(g);
   }
   ctx->fit_ntiles = (int)tiles.size() - ctx->fit_tile0;
+  // A row tile of L^-1 costs what its last row is; of a few blocks per SM the
+  // last should be the short ones.  (Larger problems have many blocks per SM,
+  // and read H in its own order.)
+  if (elem_ht)
+    std::stable_sort(tiles.begin() + ctx->fit_tile0, tiles.end(),
+                     [](const GemmTile& x, const GemmTile& y) { return x.mt > y.mt; });
   // fit with V^-1 (full) for DF-LMO: same shapes, groups pointing at V^-1
   ctx->fitV_group0 = (int)groups.size();
   for (size_t mu = 0; mu < nbf; ++mu) {

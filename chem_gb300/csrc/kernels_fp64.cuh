@@ -609,7 +609,11 @@ __global__ void __launch_bounds__(TN * 4)
 // be mostly padding and the few tiles would leave most SMs' FP64 units idle.
 // Bound by latency: 64 k of both operands are staged in shared memory at a
 // time, the next 64 in registers meanwhile, so the chain waits for memory
-// once per tile and not once per eight k.
+// once per tile and not once per eight k.  The threads take the outputs that
+// the matrix has, in row order: an FP64 instruction of a warp costs 16 clocks
+// however few lanes it has, and five columns are three warps' work and not eight
+// (the half transform of one water molecule 6.8 -> 5.2 us; its fit 18.3 -> 9.1,
+// with the long tiles first).
 template <bool TRANSB>
 __global__ void __launch_bounds__(256)
     k_gemm_fp64_elem(const GemmGroup* __restrict__ groups, const GemmTile* __restrict__ tiles,
@@ -620,12 +624,14 @@ __global__ void __launch_bounds__(256)
   const GemmTile t = tiles[blockIdx.x];
   const GemmGroup g = groups[t.group];
   const int tid = threadIdx.x;
-  const int ty = tid >> 4, tx = tid & 15;
   const int m0 = t.mt * 16, n0 = t.nt * 16;
+  const int nc = min(16, g.N - n0);
+  const bool used = tid < nc * min(16, g.M - m0);
+  const int ty = used ? tid / nc : 0, tx = used ? tid - ty * nc : 0;
   const int gm = m0 + ty, gn = n0 + tx;
   int kblk = t.k1;  // end of the tile's k range, and of this row's
   if ((g.flags & kLowerA) && kblk > m0 + 16) kblk = m0 + 16;
-  const int kend = (g.flags & kLowerA) ? min(kblk, gm + 1) : kblk;
+  const int kend = !used ? t.k0 : (g.flags & kLowerA) ? min(kblk, gm + 1) : kblk;
   double ra[4], rb[4];
   auto fetch = [&](int k0) {
 #pragma unroll
@@ -663,7 +669,7 @@ __global__ void __launch_bounds__(256)
       for (int u = 0; u < 8; ++u) acc = fma(As[ty][k + u], Bs[k + u][tx], acc);
     for (; k < n; ++k) acc = fma(As[ty][k], Bs[k][tx], acc);
   }
-  if (gm >= g.M || gn >= g.N) return;
+  if (!used) return;
   double* C = g.C + t.coff + (long long)gm * g.ldc + gn;
   double v = alpha * acc;
   if (g.flags & kAccum) v += *C;

@@ -1288,7 +1288,7 @@ gbjk_status gbjk_upload_b_eri3c(gbjk_ctx* ctx, const gbjk_shells* ao, const gbjk
   // in its order: four code paths at once did not fit the instruction cache.
   // (Six waters / jkfit: s-s 4.0 -> 2.6 ms, 3.1 before the order; others 8.0 -> 3.7.)
   std::vector<EriItem> items, rest;
-  size_t bra_max[2] = {0, 0};
+  size_t bra_max[2] = {0, 0}, pair_max = 0;
   // costs of a primitive pair with auxiliary block A: s-s pairs by the block's s,
   // p, d, f shells, then every (la, lb) with all of them
   constexpr int kSs = kEriMaxLaux + 1, kCosts = kSs + (kEriMaxLao + 1) * (kEriMaxLao + 1);
@@ -1333,6 +1333,7 @@ gbjk_status gbjk_upload_b_eri3c(gbjk_ctx* ctx, const gbjk_shells* ao, const gbjk
           total[ss] += cost;
         }
         size_t bra = (size_t)npp * eri_pair_size(la, lb);
+        pair_max = std::max(pair_max, bra);
         if (ss) bra += (size_t)eri_sph_chunk(la, lb, npp) * eri_sph_size(la, lb);
         bra_max[ss] = std::max(bra_max[ss], bra);
       }
@@ -1369,8 +1370,9 @@ gbjk_status gbjk_upload_b_eri3c(gbjk_ctx* ctx, const gbjk_shells* ao, const gbjk
   size_t smem_k[2];
   for (int k = 0; k < 2; ++k)
     smem_k[k] = (bra_max[k] + (size_t)kEriWarps * kEriWarpDoubles) * sizeof(double);
-  const size_t smem = std::max(smem_k[0], smem_k[1]);
-  if (smem > 224 * 1024)
+  // the pairs' tables and the warps' buffers within 200 KB, the others' matrices
+  // (24 KB at most) on top
+  if ((pair_max + (size_t)kEriWarps * kEriWarpDoubles) * sizeof(double) > 200 * 1024)
     return fail(ctx, GBJK_INVALID_ARG, "gbjk_upload_b_eri3c: contraction too long for the kernel");
   gbjk_status s;
   if ((s = dalloc(ctx, &ctx->d_B, (size_t)ctx->nnz))) return s;

@@ -599,10 +599,9 @@ struct Mp2State {
   // ordered on the stream after any evaluation still in flight.
   gbjk_status upload(cudaStream_t st, int nbf, const double* const* Lo, const double* const* Lv,
                      std::string* err) {
-    // Through page-locked memory that outlives the call, the copy of Lo under the
-    // packing of Lv; the stream is idle first, so nothing still reads it.  (A fresh
-    // buffer per call, zeroed and packed by rows, and a wait for the copies took
-    // 270 us for eight points of C8H18; 100 so.)
+    // Through page-locked memory kept with the plan, the copy of Lo under the
+    // packing of Lv.  (A fresh buffer per call, zeroed and packed by rows, took 270
+    // us for eight points of C8H18; this 100, and the wait for its copies.)
     const size_t nlo = (size_t)npts * nbf * hld, nlv = (size_t)npts * nbf * vld;
     std::vector<double> pageable;
     double* lo = h_stage;
@@ -623,12 +622,11 @@ struct Mp2State {
       }
     };
     double* lv = lo + nlo;
-    bool bad = cudaStreamSynchronize(st) != cudaSuccess;
     pack(lo, Lo, ro, hld);
-    bad |= cudaMemcpyAsync(d_Lo, lo, nlo * 8, cudaMemcpyHostToDevice, st) != cudaSuccess;
+    bool bad = cudaMemcpyAsync(d_Lo, lo, nlo * 8, cudaMemcpyHostToDevice, st) != cudaSuccess;
     pack(lv, Lv, rv, vld);
     bad |= cudaMemcpyAsync(d_Lv, lv, nlv * 8, cudaMemcpyHostToDevice, st) != cudaSuccess;
-    if (!h_stage) bad |= cudaStreamSynchronize(st) != cudaSuccess;
+    bad |= cudaStreamSynchronize(st) != cudaSuccess;
     if (bad) {
       *err = "MP2 batch: factor upload failed";
       return GBJK_CUDA_ERROR;

@@ -346,7 +346,8 @@ class JKEngine:
     def set_overlap(self, sms):
         """SMs the mixed-path exchange leaves to the concurrent J column
         sums on a second stream (0, default: none, the J blocks co-reside
-        with the exchange CTAs; -1: phases in order on one stream)."""
+        with the exchange CTAs while the tensor copy they read is small;
+        -1: phases in order on one stream)."""
         self._check(lib().gbjk_set_overlap(self.h, int(sms)), "gbjk_set_overlap")
 
     def get_overlap(self):

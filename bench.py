@@ -1010,7 +1010,7 @@ def main():
         "config": dict(workload_config(ds, mol, args.alkane, args.precision, world),
                        h_digits="cut in the half-transform epilogue, exponent per (AO function, "
                                 "32 auxiliary indices)" if eng.get_split_fuse()
-                       else "separate pass over FP64 H, exponent per AO function"
+                       else "separate pass over the half transform's integers, exponent per AO function"
                        if args.precision == "split" else None,
                        autotune={"chosen": tune["chosen"], "best_ms": tune["best_ms"],
                                  "candidates": [(c["effective"], round(c["ms"], 4))

@@ -228,7 +228,9 @@ struct AsymKState {
         alloc(&d_Kpart, (size_t)ksplit * nbf * nbf) ||
         cudaMemset(d_Cdig, 0, (size_t)ctot * 2) || cudaMemset(d_Hi, 0, (size_t)nbf * hrow * 8) ||
         cudaMemset(d_Hdig, 0, (size_t)2 * hdig_side * 2) ||
-        cudaMemset(d_eC, 0, (size_t)nblk * c_nrb * 32 * 4)) {
+        // the zero column after each side of an odd count has no exponent: one
+        // of 0 would set the scale of the rows of much smaller vectors
+        cudaMemset(d_eC, kNoExpByte, (size_t)nblk * c_nrb * 32 * 4)) {
       *err = "non-symmetric DF-LMO K: out of device memory for the split path";
       return GBJK_OOM;
     }

@@ -62,3 +62,22 @@ def c20h42():
     s, x = geometry.alkane(20)
     mol = molecule_from_angstrom(s, x, "cc-pvdz", "cc-pvdz-jkfit")
     return build_dfsystem(mol, eps=1e-10)
+
+
+@pytest.fixture(scope="session")
+def dense_to_panels():
+    """(layout, T) -> the panel array of T's kept blocks, and T with its other
+    blocks zeroed; T is (naux, nbf, nbf)."""
+    import numpy as np
+
+    def pack(lay, T):
+        off = lay.boff
+        B, D = np.zeros(lay.nnz), np.zeros_like(T)
+        for i, cols in enumerate(lay.column_map()):
+            b, k, o = int(lay.bsizes[i]), len(cols), int(lay.panel_off[i])
+            blk = T[:, off[i]:off[i + 1]][:, :, cols]
+            B[o:o + b * T.shape[0] * k] = blk.transpose(1, 0, 2).ravel()
+            D[:, off[i]:off[i + 1], cols] = blk
+        return B, D
+
+    return pack

@@ -1234,8 +1234,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         if constexpr (kInt) {
           // columns kept by this warp; a row's exponent is that of
           // max_c |V_c| 2^eb[c]: OR the magnitudes, each shifted to the
-          // largest column exponent (`any` keeps a nonzero row nonzero).
-          // Columns from cs on belong to the second set of exponents.
+          // largest column exponent.  Columns from cs on belong to the second
+          // set of exponents.
           const int nv = min(max(nstore - cbase, 0), kEpiCols);
           const int cs = kOut == kOutIntTwo ? min(max(w.csplit - cbase, 0), kEpiCols) : kEpiCols;
           const int ecm0 = __reduce_max_sync(0xffffffffu, lane < min(nv, cs) ? ecl : kNone);
@@ -1277,15 +1277,27 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (rvalid)
               *reinterpret_cast<longlong2*>(orow + (c >> 1) * pstep) = make_longlong2(v0, v1);
           }
-          // |x| <= 2^e, e = bit length + er + ecm - 46
-          if (rvalid && any0)
-            e_row = (mag0 ? 64 - __clzll((long long)mag0) : 1) + er + ecm0 - 46;
+          // |x| <= 2^e, e = b + er - 46, b = bit length + ecm
+          int b0 = mag0 ? 64 - __clzll((long long)mag0) + ecm0 : kNone;
+          int b1 = mag1 ? 64 - __clzll((long long)mag1) + ecm1 : kNone;
+          // A row that is nonzero only in columns so far below the largest that
+          // every bit was shifted out: the bit lengths of what it just stored,
+          // column by column (rare; V is kept no longer for it).
+          if (rvalid && ((any0 && !mag0) || (any1 && !mag1)))
+            for (int c = 0; c < nv; ++c) {
+              const long long v = orow[(c >> 1) * pstep + (c & 1)];
+              if (v == 0) continue;
+              const int b = 64 - __clzll((v ^ (v >> 63)) | 1) + w.eb[cbase + c];
+              if (kOut != kOutIntTwo || c < cs)
+                b0 = max(b0, b);
+              else
+                b1 = max(b1, b);
+            }
+          if (rvalid && any0) e_row = b0 + er - 46;
           if constexpr (kOut == kOutIntTwo) {
             // the padded A rows make a warp's 32 rows one AO function
-            const int m = __reduce_max_sync(
-                0xffffffffu,
-                rvalid && any1 ? (mag1 ? 64 - __clzll((long long)mag1) : 1) + er + ecm1 - 46
-                               : kNone);
+            const int m =
+                __reduce_max_sync(0xffffffffu, rvalid && any1 ? b1 + er - 46 : kNone);
             if (lane == 0 && m > kNone) atomicMax(w.emax2 + R / emax_div, m);
           }
           // the density column of this warp's AO function, in FP64

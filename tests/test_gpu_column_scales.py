@@ -45,3 +45,28 @@ def test_small_vectors(nocc, su, sv, dense_to_panels):
     # three operands of 39 bits below their rows' exponents
     bound = 2.0 ** -33 * np.outer(np.linalg.norm(Hu, axis=1), np.linalg.norm(Hv, axis=1))
     assert (np.abs(K + Hu @ Hv.T) <= bound).all()
+
+
+@pytest.mark.parametrize("scale", [1e-3, 1e-16, 1e-25])
+@pytest.mark.parametrize("nocc", [2, 33, 70])
+@pytest.mark.parametrize("call", ["dfmo", "asym"])
+def test_rows_without_the_large_columns(call, nocc, scale, dense_to_panels):
+    """Functions whose integrals with the first orbital's functions are all
+    zero: their rows hold the other orbitals alone, `scale` times as large."""
+    rng = np.random.default_rng(nocc)
+    lay = _layout()
+    n = lay.nbf
+    T = _tensor(rng, n)
+    big, rows = np.arange(16, 20), np.array([3, 20, 47, 60])
+    T[:, rows[:, None], big] = 0.0
+    T[:, big[:, None], rows] = 0.0
+    B, D = dense_to_panels(lay, T)
+    C = scale * rng.standard_normal((n, nocc))
+    C[:, 0] = 0.0
+    C[big, 0] = rng.standard_normal(4)
+    eng = JKEngine(lay, B, None, None, fitted=True, precision="split")
+    K = eng.compute_jk(None, C)[1] if call == "dfmo" else eng.compute_k_lmo_asym(C, C.T.copy())
+    eng.close()
+    H = _half(D, C)
+    norm = np.linalg.norm(H, axis=1)
+    assert (np.abs(K + H @ H.T) <= 2.0 ** -33 * np.outer(norm, norm)).all()

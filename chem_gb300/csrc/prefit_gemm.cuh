@@ -3,7 +3,10 @@
 //
 // FP64 operands become 63-bit integers: a row's elements relative to the
 // row's exponent e (|x| < 2^e), X = rint(|x| 2^(63-e)), in eight balanced
-// base-256 digits, exact in BF16 (the top one in [0, 128]).  The product keeps
+// base-256 digits, exact in BF16 (the top one in [0, 128]).  Before that the
+// contracted index is balanced: column Y of L^-1 is divided, row Y of B
+// multiplied, by the power of two that makes their largest elements alike
+// (k_pf_balance), so that the scale of an auxiliary function does not matter.  The product keeps
 // the 36 digit pairs (s, t) with s + t <= 7; all eight diagonals d = s + t are
 // summed exactly: a digit product is at most 2^14, so 128 k of at most eight
 // pairs stay within 2^24, exact in the FP32 accumulators.  Every 128 k the
@@ -11,8 +14,11 @@
 //   HI = sum_{d<4} r_d 256^(3-d),  LO = sum_{d>=4} r_d 256^(7-d),
 // and a result is (HI 2^32 + LO) 2^(eA+eB-70), rounded once.  What is lost is
 // the operands' rounding at 2^-63 of their rows' largest elements and the
-// dropped pairs (2^-56 of the product of the two maxima, times their digits'
-// signs); an in-order FP64 sum loses 2^-53 of every partial sum.
+// dropped pairs: for a result (X, c) about 2^-56 max_Y |L^-1[X][Y]| max_Y
+// |B[Y][c]| of the balanced operands.  An in-order FP64 sum loses 2^-53 of its
+// partial sums.  Over a tensor the first is the smaller by far, but a
+// single result whose terms are all far below that product of maxima is further
+// off here; those who read the result take sums over X or k, where it drowns.
 //
 // This is the set-up cost of every new molecule: naux nnz(B) / 2 products, on
 // GB300's FP64 pipe (6e11 fma/s) 162 ms for C12H26 and 740 ms for C20H42.
@@ -40,6 +46,9 @@ constexpr int kPfStages = 2;
 constexpr int kPfBytesA = kPfDigits * kPfM * kPfK * 2, kPfBytesB = kPfDigits * kPfN * kPfK * 2;
 constexpr int kPfSmem = kPfStages * (kPfBytesA + kPfBytesB) + 1024;
 constexpr int kPfCols = kPfN / 3;  // output columns per epilogue thread
+// exponent of a row without a nonzero element; those of balanced rows reach
+// from -2044 to 2048
+constexpr int kPfNone = -1000000;
 
 // 128 tensor columns: c = c0 .. c0 + 127 of the panel's ncol = b_I K_I columns
 // (m, k), element Y at src[(m * naux + Y) * K + k], results likewise in dst.
@@ -49,9 +58,10 @@ struct PfTile {
   int K, c0, ncol;
 };
 
-// The eight digits of eight elements of one row (k run), 16 bytes per digit.
-__device__ __forceinline__ void store_digits8x8(const double (&x)[8], int e, uint16_t* p,
-                                                int sstride) {
+// The eight digits of eight elements x 2^b of one row (k run), 16 bytes per
+// digit.
+__device__ __forceinline__ void store_digits8x8(const double (&x)[8], const int (&b)[8], int e,
+                                                uint16_t* p, int sstride) {
   unsigned long long T[8];
   uint32_t sgn[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -59,10 +69,10 @@ __device__ __forceinline__ void store_digits8x8(const double (&x)[8], int e, uin
     const unsigned long long u = (unsigned long long)__double_as_longlong(x[j]);
     const int E = (int)((u >> 52) & 0x7FF);
     const unsigned long long m = (u & ((1ull << 52) - 1)) | (1ull << 52);
-    // X = m 2^-sh, sh >= -10 since |x| < 2^e
-    const int sh = e + 1012 - E;
+    // X = m 2^-sh, sh >= -10 since |x 2^b| < 2^e
+    const int sh = e + 1012 - E - b[j];
     unsigned long long X = sh <= 0 ? m << min(-sh, 10) : (shr_u64(m, sh - 1) + 1) >> 1;
-    if (E == 0 || e <= -2000) X = 0;
+    if (E == 0 || e == kPfNone) X = 0;
     T[j] = X + 0x0080808080808080ull;
     if (u >> 63) sgn[j >> 1] |= (j & 1) ? 0x80000000u : 0x8000u;
   }
@@ -76,8 +86,8 @@ __device__ __forceinline__ void store_digits8x8(const double (&x)[8], int e, uin
       for (int h = 0; h < 2; ++h) {
         const unsigned long long t = T[2 * j + h];
         const uint32_t w = s < 4 ? (uint32_t)(t >> 32) : (uint32_t)t;
-        const float b = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 | (3 - (s & 3))));
-        f[h] = s == 0 ? b - 8388608.0f : b - 8388736.0f;
+        const float d = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 | (3 - (s & 3))));
+        f[h] = s == 0 ? d - 8388608.0f : d - 8388736.0f;
       }
       o[j] = __byte_perm(__float_as_uint(f[0]), __float_as_uint(f[1]), 0x7632) ^ sgn[j];
     }
@@ -85,27 +95,81 @@ __device__ __forceinline__ void store_digits8x8(const double (&x)[8], int e, uin
   }
 }
 
+// The largest exponent field of row Y of the tensor over all panels, into EB[Y]
+// (zeroed).  A warp takes one Y of sixteen AO functions.  Bound by HBM: one more
+// pass over the tensor (C12H26, 0.9 GB: 0.14 ms of the 20 of a new molecule).
+// grid (ceil(naux / 8), ceil(nbf / 16)), block 256.
+__global__ void __launch_bounds__(256)
+    k_pf_rowmax(const double* __restrict__ B, const long long* __restrict__ panel_off,
+                const int* __restrict__ blk_of, const int* __restrict__ boff,
+                const int* __restrict__ panel_K, int nbf, int naux,
+                unsigned int* __restrict__ EB) {
+  const int Y = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (Y >= naux) return;
+  unsigned int mx = 0;
+  const int mu1 = min(nbf, (int)(blockIdx.y + 1) * 16);
+  for (int mu = blockIdx.y * 16; mu < mu1; ++mu) {
+    const int I = blk_of[mu], K = panel_K[I];
+    const double* p = B + panel_off[I] + ((long long)(mu - boff[I]) * naux + Y) * K;
+#pragma unroll 4
+    for (int k = lane; k < K; k += 32)
+      mx = max(mx, (unsigned int)(__double_as_longlong(__ldg(p + k)) >> 52) & 0x7FF);
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0 && mx) atomicMax(EB + Y, mx);
+}
+
+// b[Y]: half the distance between the exponents of the largest element of column
+// Y of L^-1 and of row Y of the tensor, rounded down; a function taken 2^s times
+// as large lowers it by s, which leaves every digit as it is.  (On C4H10 and
+// C8H18 in their fitting basis the error bound above is 0.6 times that of
+// unbalanced operands, and twice it where L^-1 alone is balanced.)  Column maxima
+// of the lower triangle: a block walks 32 columns, 32 rows at a time.
+// grid ceil(naux / 32), block (32, 32).
+__global__ void __launch_bounds__(1024)
+    k_pf_balance(const double* __restrict__ L, int naux, const unsigned int* __restrict__ EB,
+                 int* __restrict__ b) {
+  __shared__ unsigned int sm[32][33];
+  const int Y = blockIdx.x * 32 + threadIdx.x;
+  unsigned int mx = 0;
+  if (Y < naux)
+#pragma unroll 4
+    for (int X = blockIdx.x * 32 + threadIdx.y; X < naux; X += 32)
+      if (X >= Y)
+        mx = max(mx, (unsigned int)(__double_as_longlong(L[(long long)X * naux + Y]) >> 52) & 0x7FF);
+  sm[threadIdx.x][threadIdx.y] = mx;
+  __syncthreads();
+  // warp y holds column 32 blockIdx.x + y
+  mx = __reduce_max_sync(0xffffffffu, sm[threadIdx.y][threadIdx.x]);
+  const int Yw = blockIdx.x * 32 + threadIdx.y;
+  if (threadIdx.x == 0)
+    b[Yw] = Yw < naux && mx && EB[Yw] ? ((int)mx - (int)EB[Yw]) >> 1 : 0;
+}
+
 // Exponents of a tile's 128 tensor columns (max over Y); grid ntiles, block
 // (128, 4).
 __global__ void __launch_bounds__(512)
-    k_pf_colexp(const PfTile* __restrict__ tiles, int naux, int* __restrict__ e) {
-  __shared__ unsigned int sm[4][128];
+    k_pf_colexp(const PfTile* __restrict__ tiles, const int* __restrict__ b, int naux,
+                int* __restrict__ e) {
+  __shared__ int sm[4][128];
   const PfTile t = tiles[blockIdx.x];
   const int c = t.c0 + threadIdx.x;
-  unsigned int mx = 0;
+  int mx = kPfNone;
   if (c < t.ncol) {
     const int m = c / t.K, k = c - m * t.K;
     const double* p = t.src + (long long)m * naux * t.K + k;
 #pragma unroll 8
-    for (int Y = threadIdx.y; Y < naux; Y += 4)
-      mx = max(mx, (unsigned int)(__double_as_longlong(__ldg(p + (long long)Y * t.K)) >> 52) & 0x7FF);
+    for (int Y = threadIdx.y; Y < naux; Y += 4) {
+      const int E = (int)(__double_as_longlong(__ldg(p + (long long)Y * t.K)) >> 52) & 0x7FF;
+      if (E) mx = max(mx, E + b[Y] - 1022);
+    }
   }
   sm[threadIdx.y][threadIdx.x] = mx;
   __syncthreads();
   if (threadIdx.y == 0) {
     mx = max(max(sm[0][threadIdx.x], sm[1][threadIdx.x]),
              max(sm[2][threadIdx.x], sm[3][threadIdx.x]));
-    e[blockIdx.x * kPfM + threadIdx.x] = mx == 0 ? -2000 : (int)mx - 1022;
+    e[blockIdx.x * kPfM + threadIdx.x] = mx;
   }
 }
 
@@ -113,8 +177,8 @@ __global__ void __launch_bounds__(512)
 // (rr, kc) handles column 8 g + rr, Y = 32 kt + 8 kc .. + 7.  grid (ntiles,
 // ceil(16 nkt / 8)), block 256.
 __global__ void __launch_bounds__(256)
-    k_pf_coldigits(const PfTile* __restrict__ tiles, const int* __restrict__ e, int naux, int nkt,
-                   uint16_t* __restrict__ dst) {
+    k_pf_coldigits(const PfTile* __restrict__ tiles, const int* __restrict__ e,
+                   const int* __restrict__ b, int naux, int nkt, uint16_t* __restrict__ dst) {
   const int wid = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int g = wid & 15, kt = wid >> 4;
   if (kt >= nkt) return;
@@ -123,14 +187,17 @@ __global__ void __launch_bounds__(256)
   const int c = t.c0 + r;
   const int Y0 = kt * kPfK + kc * 8;
   double x[8];
+  int bal[8];
   const int m = c / t.K, k = c - m * t.K;
   const double* p = t.src + ((long long)m * naux + Y0) * t.K + k;
 #pragma unroll
-  for (int j = 0; j < 8; ++j)
+  for (int j = 0; j < 8; ++j) {
     x[j] = c < t.ncol && Y0 + j < naux ? __ldg(p + (long long)j * t.K) : 0.0;
+    bal[j] = __ldg(b + Y0 + j);
+  }
   uint16_t* o = dst + ((long long)blockIdx.x * nkt + kt) * (kPfBytesA / 2) + g * 256 + kc * 64 +
                 (lane & 7) * 8;
-  store_digits8x8(x, e[blockIdx.x * kPfM + r], o, kPfM * kPfK);
+  store_digits8x8(x, bal, e[blockIdx.x * kPfM + r], o, kPfM * kPfK);
 }
 
 // Exponents and digits of the rows of L^-1 (entries right of the diagonal are
@@ -138,20 +205,22 @@ __global__ void __launch_bounds__(256)
 // the exponents of its eight rows, then share their k-tiles.  Row X goes to
 // tile X / 48; rows of the last tile beyond naux stay as allocated (zero).
 __global__ void __launch_bounds__(256)
-    k_pf_metric(const double* __restrict__ L, int naux, int nkt, int* __restrict__ e,
-                uint16_t* __restrict__ dst) {
+    k_pf_metric(const double* __restrict__ L, const int* __restrict__ b, int naux, int nkt,
+                int* __restrict__ e, uint16_t* __restrict__ dst) {
   __shared__ int se[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   {
     const int X = blockIdx.x * 8 + warp;
-    unsigned int mx = 0;
+    int mx = kPfNone;
     if (X < naux)
-      for (int Y = lane; Y <= X; Y += 32)
-        mx = max(mx, (unsigned int)(__double_as_longlong(L[(long long)X * naux + Y]) >> 52) & 0x7FF);
+      for (int Y = lane; Y <= X; Y += 32) {
+        const int E = (int)(__double_as_longlong(L[(long long)X * naux + Y]) >> 52) & 0x7FF;
+        if (E) mx = max(mx, E - b[Y] - 1022);
+      }
     mx = __reduce_max_sync(0xffffffffu, mx);
     if (lane == 0) {
-      se[warp] = mx == 0 ? -2000 : (int)mx - 1022;
-      if (X < naux) e[X] = se[warp];
+      se[warp] = mx;
+      if (X < naux) e[X] = mx;
     }
   }
   __syncthreads();
@@ -161,10 +230,13 @@ __global__ void __launch_bounds__(256)
   for (int kt = warp; kt < nkt; kt += 8) {
     const int Y0 = kt * kPfK + kc * 8;
     double x[8];
+    int bal[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 8; ++j) {
       x[j] = X < naux && Y0 + j <= X ? L[(long long)X * naux + Y0 + j] : 0.0;
-    store_digits8x8(x, se[rr],
+      bal[j] = -__ldg(b + Y0 + j);
+    }
+    store_digits8x8(x, bal, se[rr],
                     dst + ((long long)xt * nkt + kt) * (kPfBytesB / 2) + g * 256 + kc * 64 + rr * 8,
                     kPfN * kPfK);
   }
@@ -377,7 +449,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (X0 + c >= naux) break;
           const int ec = __ldg(eb + X0 + c);
           const double v = fma((double)HI[c], 4294967296.0, (double)LO[c]);
-          o[(long long)c * K] = er <= -2000 || ec <= -2000 ? 0.0 : scale_exp2(v, er + ec - 70);
+          o[(long long)c * K] = er == kPfNone || ec == kPfNone ? 0.0 : scale_exp2(v, er + ec - 70);
         }
       }
     }

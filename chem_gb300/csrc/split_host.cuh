@@ -393,7 +393,9 @@ struct SplitState {
     }
     PfTile* dt = nullptr;
     uint16_t* db = nullptr;
-    int* de = nullptr;  // exponents of the X rows, then of the tensor columns
+    // balance and largest exponents of Y, exponents of the X rows and of the tensor columns
+    int* de = nullptr;
+    const size_t ny = (size_t)nkt_all * kPfK;
     auto done = [&]() {
       cudaFree(own);
       cudaFree(dt);
@@ -402,7 +404,8 @@ struct SplitState {
     };
     if (per == 0 || cudaMalloc((void**)&dt, tiles.size() * sizeof(PfTile)) != cudaSuccess ||
         cudaMalloc((void**)&db, bbytes) != cudaSuccess ||
-        cudaMalloc((void**)&de, ((size_t)nxt * kPfN + per * kPfM) * sizeof(int)) != cudaSuccess ||
+        cudaMalloc((void**)&de, (2 * ny + (size_t)nxt * kPfN + per * kPfM) * sizeof(int)) !=
+            cudaSuccess ||
         cudaFuncSetAttribute(k_prefit_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kPfSmem) != cudaSuccess) {
       cudaGetLastError();
@@ -412,19 +415,23 @@ struct SplitState {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    int *eb = de, *ea = de + (size_t)nxt * kPfN;
+    int *bal = de, *eY = de + ny, *eb = de + 2 * ny, *ea = eb + (size_t)nxt * kPfN;
     uint16_t* ad = (uint16_t*)ws;
     cudaError_t e = cudaMemcpyAsync(dt, tiles.data(), tiles.size() * sizeof(PfTile),
                                     cudaMemcpyHostToDevice, st);
     if (!e) e = cudaMemsetAsync(db, 0, bbytes, st);
+    if (!e) e = cudaMemsetAsync(eY, 0, ny * sizeof(int), st);
     if (!e) {
       Scope sc(this, 3, st);
-      k_pf_metric<<<cdiv_(naux, 8), 256, 0, st>>>(d_Linv, naux, nkt_all, eb, db);
-      (*launches)++;
+      k_pf_rowmax<<<dim3(cdiv_(naux, 8), cdiv_(nbf, 16)), 256, 0, st>>>(
+          d_B, dd_panel_off, dd_blk_of, dd_boff, dd_panelK, nbf, naux, (unsigned int*)eY);
+      k_pf_balance<<<nkt_all, dim3(32, 32), 0, st>>>(d_Linv, naux, (unsigned int*)eY, bal);
+      k_pf_metric<<<cdiv_(naux, 8), 256, 0, st>>>(d_Linv, bal, naux, nkt_all, eb, db);
+      *launches += 3;
       for (size_t t0 = 0; t0 < tiles.size(); t0 += per) {
         const int n = (int)std::min(per, tiles.size() - t0);
-        k_pf_colexp<<<n, dim3(128, 4), 0, st>>>(dt + t0, naux, ea);
-        k_pf_coldigits<<<dim3(n, 2 * nkt_all), 256, 0, st>>>(dt + t0, ea, naux, nkt_all, ad);
+        k_pf_colexp<<<n, dim3(128, 4), 0, st>>>(dt + t0, bal, naux, ea);
+        k_pf_coldigits<<<dim3(n, 2 * nkt_all), 256, 0, st>>>(dt + t0, ea, bal, naux, nkt_all, ad);
         k_prefit_gemm<<<std::min(n * nxt, nsm), kThreads, kPfSmem, st>>>(
             dt + t0, n * nxt, nxt, naux, nkt_all, ad, ea, db, eb, d_err, kSpinNs);
         *launches += 3;

@@ -1488,6 +1488,12 @@ gbjk_status gbjk_test_split_stall(gbjk_ctx* ctx, int item, double wait_ms) {
   return GBJK_OK;
 }
 
+gbjk_status gbjk_test_prefit_room(gbjk_ctx* ctx, long long bytes) {
+  if (!ctx) return GBJK_INVALID_ARG;
+  ctx->split.prefit_room = bytes < 0 ? ~size_t(0) : (size_t)bytes;
+  return GBJK_OK;
+}
+
 gbjk_status gbjk_set_occ_batch(gbjk_ctx* ctx, int cols) {
   if (!ctx || cols < 0) return GBJK_INVALID_ARG;
   if (cols != ctx->occ_req) ctx->epoch++;

@@ -200,17 +200,18 @@ __global__ void __launch_bounds__(256)
   store_digits8x8(x, bal, e[blockIdx.x * kPfM + r], o, kPfM * kPfK);
 }
 
-// Exponents and digits of the rows of L^-1 (entries right of the diagonal are
-// taken as zero).  grid ceil(naux / 8), block 256: the block's eight warps find
-// the exponents of its eight rows, then share their k-tiles.  Row X goes to
-// tile X / 48; rows of the last tile beyond naux stay as allocated (zero).
+// Exponents and digits of the rows of L^-1 from row0 on (a multiple of 48;
+// entries right of the diagonal are taken as zero).  grid ceil(rows / 8), block
+// 256: the block's eight warps find the exponents of its eight rows, then share
+// their k-tiles.  Row X goes to tile (X - row0) / 48; rows of the last tile beyond
+// naux stay as they are (zero).
 __global__ void __launch_bounds__(256)
-    k_pf_metric(const double* __restrict__ L, const int* __restrict__ b, int naux, int nkt,
-                int* __restrict__ e, uint16_t* __restrict__ dst) {
+    k_pf_metric(const double* __restrict__ L, const int* __restrict__ b, int naux, int row0,
+                int nkt, int* __restrict__ e, uint16_t* __restrict__ dst) {
   __shared__ int se[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   {
-    const int X = blockIdx.x * 8 + warp;
+    const int X = row0 + blockIdx.x * 8 + warp;
     int mx = kPfNone;
     if (X < naux)
       for (int Y = lane; Y <= X; Y += 32) {
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(256)
   }
   __syncthreads();
   const int rr = lane & 7, kc = lane >> 3;
-  const int X = blockIdx.x * 8 + rr;
+  const int X = row0 + blockIdx.x * 8 + rr;
   const int xt = (blockIdx.x * 8) / kPfN, g = blockIdx.x - xt * (kPfN / 8);
   for (int kt = warp; kt < nkt; kt += 8) {
     const int Y0 = kt * kPfK + kc * 8;
@@ -251,8 +252,8 @@ __device__ __forceinline__ double scale_exp2(double v, int e) {
   return ex > 0 && ex < 2047 ? __longlong_as_double(b + ((long long)e << 52)) : ldexp(v, e);
 }
 
-// Work item it: tensor tile it / nxt, X tile rotated by the tile so that every
-// CTA meets all k lengths whatever the grid size.
+// Work item it of a launch over nxt X tiles: tensor tile it / nxt, X tile rotated by
+// the tile so that every CTA meets all k lengths whatever the grid size.
 __device__ __forceinline__ void pf_item(int it, int nxt, int* tile, int* xt) {
   *tile = it / nxt;
   *xt = nxt - 1 - (it + *tile) % nxt;
@@ -261,8 +262,9 @@ __device__ __forceinline__ int pf_nkt(int xt, int naux) {
   return (min(naux, (xt + 1) * kPfN) + kPfK - 1) / kPfK;
 }
 
+// X tiles xt0 .. xt0 + nxt - 1, whose digits bdig holds.
 __global__ void __launch_bounds__(kThreads, 1)
-    k_prefit_gemm(const PfTile* __restrict__ tiles, int nitems, int nxt, int naux, int nkt_all,
+    k_prefit_gemm(const PfTile* __restrict__ tiles, int nitems, int nxt, int xt0, int naux, int nkt_all,
                   const uint16_t* __restrict__ adig, const int* __restrict__ ea,
                   const uint16_t* __restrict__ bdig, const int* __restrict__ eb,
                   int* __restrict__ err, unsigned long long spin_ns) {
@@ -308,7 +310,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
         int tile, xt;
         pf_item(it, nxt, &tile, &xt);
-        const int nkt = pf_nkt(xt, naux);
+        const int nkt = pf_nkt(xt0 + xt, naux);
         const unsigned char* ga = (const unsigned char*)adig + (long long)tile * nkt_all * kPfBytesA;
         const unsigned char* gb = (const unsigned char*)bdig + (long long)xt * nkt_all * kPfBytesB;
         for (int k = 0; k < nkt; ++k) {
@@ -339,7 +341,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
         int tile, xt;
         pf_item(it, nxt, &tile, &xt);
-        const int nkt = pf_nkt(xt, naux);
+        const int nkt = pf_nkt(xt0 + xt, naux);
         for (int k = 0; k < nkt; ++k) {
           const bool chunk_start = (k % kPfChunk) == 0;
           const bool chunk_end = ((k + 1) % kPfChunk) == 0 || k + 1 == nkt;
@@ -392,10 +394,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
       int tile, xt;
       pf_item(it, nxt, &tile, &xt);
-      const int nchunk = (pf_nkt(xt, naux) + kPfChunk - 1) / kPfChunk;
+      const int nchunk = (pf_nkt(xt0 + xt, naux) + kPfChunk - 1) / kPfChunk;
       const PfTile& t = tiles[tile];
       const int er = ea[tile * kPfM + row];
-      const int X0 = xt * kPfN + third * kPfCols;
+      const int X0 = (xt0 + xt) * kPfN + third * kPfCols;
       long long HI[kPfCols], LO[kPfCols];
 #pragma unroll
       for (int c = 0; c < kPfCols; ++c) HI[c] = LO[c] = 0;

@@ -107,6 +107,7 @@ struct SplitState {
   // test hook (gbjk_test_split_stall): the producer stops at this work item
   // of every split GEMM launch (-1: never), and the waits' time limit
   int stop_item = -1;
+  size_t prefit_room = ~size_t(0);  // most bytes of temporary digits in the prefit
   unsigned long long spin_ns = kSpinNs;
   double ms[4] = {0, 0, 0, 0};
   int64_t nl[4] = {0, 0, 0, 0};
@@ -304,8 +305,7 @@ struct SplitState {
 
   // --- once per tensor: Bfit = L^-1 B ----------------------------------------
   // On the FP64 pipe, each element the in-order fma chain of the oracle's
-  // prefit (the FP64 MP2 batch needs that order; the mixed path takes it where
-  // the tensor-core prefit finds no room).
+  // prefit (the FP64 MP2 batch needs that order).
   gbjk_status prefit_fp64(cudaStream_t st, const double* d_B, const double* d_Linv, double* d_Bfit,
                           int64_t* launches, std::string* err) {
     std::vector<GemmGroup> groups;
@@ -367,7 +367,10 @@ struct SplitState {
   // On the tensor cores (prefit_gemm.cuh).  ws: device memory that may be
   // overwritten, for the digits of as many tensor columns as it holds (at
   // most 1 GB of them at a time); a temporary buffer where it holds too few to
-  // occupy the SMs.
+  // occupy the SMs.  The digits of L^-1 (16 naux^2 bytes) have a buffer of their
+  // own, of fewer 48-row tiles at a time where there is no room for all; one
+  // tile of each, in ws, is the least.  The parts change no result: every output
+  // is one exact sum.
   gbjk_status prefit(cudaStream_t st, const double* d_B, const double* d_Linv, double* d_Bfit,
                      void* ws, size_t ws_bytes, int64_t* launches, std::string* err) {
     std::vector<PfTile> tiles;
@@ -378,70 +381,110 @@ struct SplitState {
     }
     if (tiles.empty()) return GBJK_OK;
     const int nkt_all = cdiv_(naux, kPfK), nxt = cdiv_(naux, kPfN);
-    const size_t tile_bytes = (size_t)nkt_all * kPfBytesA, bbytes = (size_t)nxt * nkt_all * kPfBytesB;
-    const size_t most =
-        std::min(tiles.size(), std::max<size_t>(1, (size_t(1) << 30) / tile_bytes));
-    size_t per = std::min(most, ws_bytes / tile_bytes);
-    void* own = nullptr;
-    if (per < most && per * nxt < 1024) {
-      if (cudaMalloc(&own, most * tile_bytes) == cudaSuccess) {
-        ws = own;
-        per = most;
-      } else {
-        cudaGetLastError();
-      }
-    }
+    const size_t abytes = (size_t)nkt_all * kPfBytesA, bbytes = (size_t)nkt_all * kPfBytesB;
+    const size_t most = std::min(tiles.size(), std::max<size_t>(1, (size_t(1) << 30) / abytes));
+    const size_t ny = (size_t)nkt_all * kPfK;
     PfTile* dt = nullptr;
-    uint16_t* db = nullptr;
     // balance and largest exponents of Y, exponents of the X rows and of the tensor columns
     int* de = nullptr;
-    const size_t ny = (size_t)nkt_all * kPfK;
+    void *own = nullptr, *db = nullptr;
     auto done = [&]() {
       cudaFree(own);
       cudaFree(dt);
       cudaFree(db);
       cudaFree(de);
     };
-    if (per == 0 || cudaMalloc((void**)&dt, tiles.size() * sizeof(PfTile)) != cudaSuccess ||
-        cudaMalloc((void**)&db, bbytes) != cudaSuccess ||
-        cudaMalloc((void**)&de, (2 * ny + (size_t)nxt * kPfN + per * kPfM) * sizeof(int)) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_prefit_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kPfSmem) != cudaSuccess) {
-      cudaGetLastError();
-      done();
-      return prefit_fp64(st, d_B, d_Linv, d_Bfit, launches, err);
+    size_t room = prefit_room;
+    // a buffer of n units, n the first of want, want / 2, .. that there is memory
+    // for, and more than `least`; 0 if none
+    auto grab = [&](void** p, size_t unit, size_t want, size_t least) {
+      for (size_t n = want; n > least; n /= 2) {
+        if (unit * n > room) continue;
+        if (cudaMalloc(p, unit * n) == cudaSuccess) {
+          room -= unit * n;
+          return n;
+        }
+        cudaGetLastError();
+      }
+      *p = nullptr;
+      return size_t(0);
+    };
+    bool ok = cudaMalloc((void**)&dt, tiles.size() * sizeof(PfTile)) == cudaSuccess &&
+              cudaMalloc((void**)&de, (2 * ny + (size_t)nxt * kPfN + most * kPfM) * sizeof(int)) ==
+                  cudaSuccess;
+    size_t nx = 0, per = 0;  // X tiles and tensor tiles at a time
+    if (ok) {
+      nx = grab(&db, bbytes, nxt, 0);
+      uint8_t* w = (uint8_t*)ws;
+      uint16_t* bd = (uint16_t*)db;
+      if (nx == 0 && ws_bytes >= bbytes) {
+        nx = 1;
+        bd = (uint16_t*)w;
+        w += bbytes;
+        ws_bytes -= bbytes;
+      }
+      per = std::min(most, ws_bytes / abytes);
+      if (per < most && per * nx < 1024)
+        if (const size_t n = grab(&own, abytes, most, per)) {
+          per = n;
+          w = (uint8_t*)own;
+        }
+      if (nx && per)
+        return prefit_parts(st, d_Linv, d_B, tiles, dt, de, bd, (int)nx, (uint16_t*)w, per,
+                            launches, err, done);
     }
+    cudaGetLastError();
+    done();
+    *err = "split path: out of memory for the prefit's operand digits";
+    return GBJK_OOM;
+  }
+  // ... with digit buffers bd and ad for nx tiles of L^-1 and `per` tiles of the
+  // tensor; done() frees what prefit() allocated
+  template <class Done>
+  gbjk_status prefit_parts(cudaStream_t st, const double* d_Linv, const double* d_B,
+                           const std::vector<PfTile>& tiles, PfTile* dt, int* de, uint16_t* bd,
+                           int nx, uint16_t* ad, size_t per, int64_t* launches, std::string* err,
+                           Done done) {
+    const int nkt_all = cdiv_(naux, kPfK), nxt = cdiv_(naux, kPfN);
+    const size_t bbytes = (size_t)nkt_all * kPfBytesB, ny = (size_t)nkt_all * kPfK;
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     int *bal = de, *eY = de + ny, *eb = de + 2 * ny, *ea = eb + (size_t)nxt * kPfN;
-    uint16_t* ad = (uint16_t*)ws;
-    cudaError_t e = cudaMemcpyAsync(dt, tiles.data(), tiles.size() * sizeof(PfTile),
-                                    cudaMemcpyHostToDevice, st);
-    if (!e) e = cudaMemsetAsync(db, 0, bbytes, st);
+    cudaError_t e = cudaFuncSetAttribute(
+        k_prefit_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem);
+    if (!e)
+      e = cudaMemcpyAsync(dt, tiles.data(), tiles.size() * sizeof(PfTile), cudaMemcpyHostToDevice,
+                          st);
     if (!e) e = cudaMemsetAsync(eY, 0, ny * sizeof(int), st);
     if (!e) {
       Scope sc(this, 3, st);
       k_pf_rowmax<<<dim3(cdiv_(naux, 8), cdiv_(nbf, 16)), 256, 0, st>>>(
           d_B, dd_panel_off, dd_blk_of, dd_boff, dd_panelK, nbf, naux, (unsigned int*)eY);
       k_pf_balance<<<nkt_all, dim3(32, 32), 0, st>>>(d_Linv, naux, (unsigned int*)eY, bal);
-      k_pf_metric<<<cdiv_(naux, 8), 256, 0, st>>>(d_Linv, bal, naux, nkt_all, eb, db);
-      *launches += 3;
-      for (size_t t0 = 0; t0 < tiles.size(); t0 += per) {
-        const int n = (int)std::min(per, tiles.size() - t0);
-        k_pf_colexp<<<n, dim3(128, 4), 0, st>>>(dt + t0, bal, naux, ea);
-        k_pf_coldigits<<<dim3(n, 2 * nkt_all), 256, 0, st>>>(dt + t0, ea, bal, naux, nkt_all, ad);
-        k_prefit_gemm<<<std::min(n * nxt, nsm), kThreads, kPfSmem, st>>>(
-            dt + t0, n * nxt, nxt, naux, nkt_all, ad, ea, db, eb, d_err, kSpinNs);
-        *launches += 3;
+      *launches += 2;
+      for (int x0 = 0; x0 < nxt && !e; x0 += nx) {
+        const int m = std::min(nx, nxt - x0), row0 = x0 * kPfN;
+        e = cudaMemsetAsync(bd, 0, (size_t)m * bbytes, st);
+        k_pf_metric<<<cdiv_(std::min(naux - row0, m * kPfN), 8), 256, 0, st>>>(
+            d_Linv, bal, naux, row0, nkt_all, eb, bd);
+        (*launches)++;
+        for (size_t t0 = 0; t0 < tiles.size(); t0 += per) {
+          const int n = (int)std::min(per, tiles.size() - t0);
+          k_pf_colexp<<<n, dim3(128, 4), 0, st>>>(dt + t0, bal, naux, ea);
+          k_pf_coldigits<<<dim3(n, 2 * nkt_all), 256, 0, st>>>(dt + t0, ea, bal, naux, nkt_all, ad);
+          k_prefit_gemm<<<std::min(n * m, nsm), kThreads, kPfSmem, st>>>(
+              dt + t0, n * m, m, x0, naux, nkt_all, ad, ea, bd, eb, d_err, kSpinNs);
+          *launches += 3;
+        }
       }
-      e = cudaGetLastError();
+      if (!e) e = cudaGetLastError();
     }
-    if (!e) e = cudaStreamSynchronize(st);
+    // on an error too: nothing in flight uses the buffers any more
+    const cudaError_t es = cudaStreamSynchronize(st);
     done();
-    if (e != cudaSuccess) {
-      *err = std::string("prefit: ") + cudaGetErrorString(e);
+    if (e || es) {
+      *err = std::string("prefit: ") + cudaGetErrorString(e ? e : es);
       return GBJK_CUDA_ERROR;
     }
     if (const int code = read_error()) {

@@ -73,6 +73,7 @@ def lib():
         L.gbjk_set_jmode.argtypes = [vp, C.c_int]
         L.gbjk_set_overlap.argtypes = [vp, C.c_int]
         L.gbjk_test_split_stall.argtypes = [vp, C.c_int, C.c_double]
+        L.gbjk_test_prefit_room.argtypes = [vp, C.c_longlong]
         L.gbjk_scf_begin.argtypes = [vp, dp, dp, dp, C.c_int, C.c_int]
         L.gbjk_scf_build.argtypes = [vp, C.c_int, dp, C.c_int, dp]
         L.gbjk_scf_extrapolate.argtypes = [vp, dp, dp]
@@ -338,6 +339,11 @@ class JKEngine:
         bounded waits run out and builds report TIMEOUT; -1 restores."""
         self._check(lib().gbjk_test_split_stall(self.h, int(item), float(wait_ms)),
                     "gbjk_test_split_stall")
+
+    def test_prefit_room(self, nbytes):
+        """Test hook (gbjk_test_prefit_room): the first mixed-path build of a
+        tensor allocates at most nbytes for its temporary digits; -1 restores."""
+        self._check(lib().gbjk_test_prefit_room(self.h, int(nbytes)), "gbjk_test_prefit_room")
 
     def set_occ_batch(self, cols):
         """FP64 K in occupied batches of `cols` orbitals (0: all at once)."""

@@ -154,6 +154,13 @@ gbjk_status gbjk_upload_b_eri3c(gbjk_ctx* ctx, const gbjk_shells* ao, const gbjk
  * item < 0 restores normal operation.  No counterpart in the reference. */
 gbjk_status gbjk_test_split_stall(gbjk_ctx* ctx, int item, double wait_ms);
 
+/* Test hook for a nearly full device: the prefit of a mixed-precision engine
+ * (its first build of a tensor) allocates at most `bytes` for its temporary
+ * operand digits, as if the device had no more.  It then works in smaller
+ * parts, with the same bits, or reports GBJK_OOM; bytes < 0 restores normal
+ * operation.  No counterpart in the reference. */
+gbjk_status gbjk_test_prefit_room(gbjk_ctx* ctx, long long bytes);
+
 /* Mixed-precision build: after the half transform the J column sums
  * (HBM-bound) may run on a second stream of the context beside the digit pass
  * and the exchange GEMM (tensor-bound).  sms > 0: they do, and the exchange

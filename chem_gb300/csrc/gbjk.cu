@@ -758,10 +758,9 @@ gbjk_status ensure_k_occ_batched(gbjk_ctx* ctx, int nocc) {
   return GBJK_OK;
 }
 
+// (plans and buffers: ensure_k_occ_batched)
 gbjk_status run_k_occ_batched(gbjk_ctx* ctx, int kmethod, const double* dC, int nocc,
                               double* dK) {
-  gbjk_status s;
-  if ((s = ensure_k_occ_batched(ctx, nocc))) return s;
   auto& ob = ctx->ob;
   const int nbf = ctx->nbf, nblk = ctx->nblk;
   const bool mo = kmethod == GBJK_K_DFMO;
@@ -805,9 +804,8 @@ gbjk_status run_k_occ_batched(gbjk_ctx* ctx, int kmethod, const double* dC, int 
   return filter(ctx, dK);
 }
 
+// (plans and buffers: ensure_k_batched)
 gbjk_status run_k_batched(gbjk_ctx* ctx, const double* dC, int nocc, double* dK) {
-  gbjk_status s;
-  if ((s = ensure_k_batched(ctx, nocc))) return s;
   auto& fb = ctx->fb;
   const int nbf = ctx->nbf;
   {
@@ -1851,6 +1849,29 @@ static gbjk_status prepare_split(gbjk_ctx* ctx, int nocc) {
   return ctx->split.prepare(ctx->stream, ctx->d_B, ctx->d_Linv, nocc, &ctx->launches, &ctx->err);
 }
 
+// Work forked to the side stream: whatever way the build returns, the context's
+// stream waits for it, so that the caller's next use of J, P or the J buffers on
+// that stream (or after a synchronisation with it) follows.
+struct SideFork {
+  gbjk_ctx* ctx;
+  bool on = false;
+  explicit SideFork(gbjk_ctx* c) : ctx(c) {}
+  // the side stream goes on from `from` (recorded on the context's stream)
+  cudaError_t fork(cudaEvent_t from) {
+    const cudaError_t e = cudaStreamWaitEvent(ctx->side, from, 0);
+    on = on || e == cudaSuccess;
+    return e;
+  }
+  cudaError_t join() {
+    on = false;
+    const cudaError_t e = cudaEventRecord(ctx->ev_join, ctx->side);
+    return e != cudaSuccess ? e : cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0);
+  }
+  ~SideFork() {
+    if (on && join() != cudaSuccess) cudaGetLastError();  // the build's own error stands
+  }
+};
+
 // Mixed-precision J + K.  The density rows of every panel ride along as
 // extra B-operand rows of the split half transform, whose epilogue emits
 // the partials of dt = L^-1 g; J = (L^-1 B)^T dt is one FP64 pass over the
@@ -1875,9 +1896,10 @@ static gbjk_status run_jk_split(gbjk_ctx* ctx, const double* dP, const double* d
   ctx->split.ev_ht = nullptr;
   ctx->split.k_grid = 0;
   if (s) return s;
+  SideFork side(ctx);
   if (fused) {
     cudaStream_t js = overlap ? ctx->side : ctx->stream;
-    if (overlap) CK(cudaStreamWaitEvent(js, ctx->ev_fork, 0));
+    if (overlap) CK(side.fork(ctx->ev_fork));
     CK(cudaMemsetAsync(dJ, 0, (size_t)nbf * nbf * sizeof(double), js));
     {
       PhaseScope ps(ctx, PH_J_REDUCE);
@@ -1897,10 +1919,9 @@ static gbjk_status run_jk_split(gbjk_ctx* ctx, const double* dP, const double* d
           dJ, ctx->nbf, ctx->d_boff, ctx->nblk, ctx->eps);
       CKL(PH_FILTER);
     }
-    if (overlap) CK(cudaEventRecord(ctx->ev_join, js));
   }
   if ((s = filter(ctx, dK))) return s;
-  if (overlap) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
+  if (overlap) CK(side.join());
   if (!dJ || fused) return GBJK_OK;
   return run_j(ctx, dP, dJ, ctx->stream);  // auxiliary-batched: FP64 J
 }
@@ -1919,28 +1940,30 @@ gbjk_status gbjk_compute_jk_dev(gbjk_ctx* ctx, int kmethod, const double* dP, co
       if ((s = prepare_split(ctx, nocc))) return s;
       return run_jk_split(ctx, dP, dC, nocc, dJ, dK);
     }
-    if (!fp64_batched(ctx) && !fp64_occ_batched(ctx, nocc) &&
-        (s = ensure_k_workspace(ctx, nocc)))
-      return s;
+    // every plan and buffer before J starts beside K
+    s = fp64_batched(ctx)             ? ensure_k_batched(ctx, nocc)
+        : fp64_occ_batched(ctx, nocc) ? ensure_k_occ_batched(ctx, nocc)
+                                      : ensure_k_workspace(ctx, nocc);
+    if (s) return s;
   }
   // J and K share nothing but the tensor: J runs on the side stream beside K
   // unless phases are asked for in order or timed (water: a dozen launches of a
   // few microseconds in two lines instead of one, 95 -> 70 us per call)
   const bool beside = dJ && dK && ctx->overlap_sms >= 0 && !ctx->profile;
   cudaStream_t js = beside ? ctx->side : ctx->stream;
+  SideFork side(ctx);
   if (beside) {
     CK(cudaEventRecord(ctx->ev_fork, ctx->stream));
-    CK(cudaStreamWaitEvent(js, ctx->ev_fork, 0));
+    CK(side.fork(ctx->ev_fork));
   }
   if (dJ && (s = run_j(ctx, dP, dJ, js))) return s;
-  if (beside) CK(cudaEventRecord(ctx->ev_join, js));
   if (dK) {
     s = fp64_batched(ctx)               ? run_k_batched(ctx, dC, nocc, dK)
         : fp64_occ_batched(ctx, nocc)   ? run_k_occ_batched(ctx, kmethod, dC, nocc, dK)
                                         : run_k(ctx, kmethod, dC, nocc, dK);
     if (s) return s;
   }
-  if (beside) CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0));
+  if (beside) CK(side.join());
   return GBJK_OK;
 }
 

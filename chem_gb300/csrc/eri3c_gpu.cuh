@@ -26,6 +26,7 @@
 #include <stdint.h>
 
 #include <cmath>
+#include <cstring>
 
 namespace gbjk {
 
@@ -124,8 +125,27 @@ inline void eri_boys_table(double* tab) {
   }
 }
 
+// T as the table takes it: an argument below zero, which only a negative exponent
+// gives, counts as zero; NaN stays.  (On the bits: an FP64 compare would cost as
+// much as a product.)
+__host__ __device__ __forceinline__ double eri_boys_arg(double T) {
+#ifdef __CUDA_ARCH__
+  const uint32_t hi = (uint32_t)__double2hiint(T);
+#else
+  uint64_t u;
+  std::memcpy(&u, &T, 8);
+  const uint32_t hi = (uint32_t)(u >> 32);
+#endif
+  return hi - 0x80000000u <= 0x7FF00000u ? 0.0 : T;
+}
+// Its table row, for 0 <= T <= kEriBoysTmax or NaN (row 0)
+__host__ __device__ __forceinline__ int eri_boys_row(double T) {
+  return (int)((float)T * (float)kEriBoysStep + 0.5f);
+}
+
 __device__ __forceinline__ void eri_boys(const double* __restrict__ tab, int nmax, double T,
                                          double* F) {
+  T = eri_boys_arg(T);
   if (T > kEriBoysTmax) {
     const double eT = exp(-T);
     F[0] = 0.5 * sqrt(3.14159265358979323846 / T) * erf(sqrt(T));
@@ -133,7 +153,7 @@ __device__ __forceinline__ void eri_boys(const double* __restrict__ tab, int nma
     for (int m = 0; m < nmax; ++m) F[m + 1] = ((2 * m + 1) * F[m] - eT) * inv2T;
     return;
   }
-  const int i = (int)((float)T * (float)kEriBoysStep + 0.5f);
+  const int i = eri_boys_row(T);
   const double x = (double)i * (1.0 / kEriBoysStep) - T;
   const double2* c = reinterpret_cast<const double2*>(tab + ((long long)nmax * kEriBoysRows + i) * 8);
   const double2 c0 = __ldg(c), c1 = __ldg(c + 1), c2 = __ldg(c + 2), c3 = __ldg(c + 3);

@@ -2467,7 +2467,7 @@ gbjk_status gbjk_mp2_release(gbjk_ctx* ctx) {
   if (!ctx) return GBJK_INVALID_ARG;
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
-  ctx->mp2.release_plan();
+  ctx->mp2.release();
   return GBJK_OK;
 }
 

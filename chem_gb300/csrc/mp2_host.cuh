@@ -41,7 +41,7 @@ struct Mp2State {
   double *d_H = nullptr, *d_W = nullptr, *d_Z = nullptr, *d_rsq = nullptr, *d_E = nullptr;
   long long cg_stride = 0, h_stride = 0, w_stride = 0;
   // FP64 path: L^-1 B in the oracle's summation order (kept over plans until
-  // the tensor or the metric changes)
+  // the batch is released or the tensor or the metric changes)
   double* d_Bfit64 = nullptr;
   size_t bfit_bytes = 0;
   // FP64 plan

@@ -1519,7 +1519,7 @@ gbjk_status gbjk_set_split_fuse(gbjk_ctx* ctx, int on) {
   }
   return GBJK_OK;
 }
-int gbjk_get_split_fuse(const gbjk_ctx* ctx) { return ctx ? (ctx->split.hfuse ? 1 : 0) : -1; }
+int gbjk_get_split_fuse(const gbjk_ctx* ctx) { return ctx ? (ctx->split.fuses() ? 1 : 0) : -1; }
 
 // --- launch configuration and autotuning -----------------------------------
 static gbjk_status check_ready(gbjk_ctx* ctx);

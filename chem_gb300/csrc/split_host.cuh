@@ -66,7 +66,9 @@ struct SplitState {
   // the per-nocc buffers).  Off by default: on GB300 the fused half
   // transform and segmented exchange together take longer than the FP64 H
   // round trip and digit pass they replace.
-  bool hfuse = false, hfuse_eff = false;
+  bool hfuse = false, hfuse_eff = false;  // asked for; what the current plan does
+  // what the builds do, as far as a plan has decided it
+  bool fuses() const { return hfuse && (nocc < 0 || hfuse_eff); }
   SplitJob* d_bjobs = nullptr;  // A-digit jobs, nbatch * nbf (one per (batch, mu))
   std::vector<long long> a_off, eA_off;
   std::vector<int> a_nrb, nkt;

@@ -361,11 +361,15 @@ class JKEngine:
 
     def set_split_fuse(self, on):
         """Mixed-path exchange digits: cut in the half-transform epilogue
-        with one exponent per (AO function, 32 auxiliary indices) (True), or
-        from an FP64 H with one exponent per AO function (False, default)."""
+        with one exponent per (AO function, 32 auxiliary indices) (True, as
+        long as a row's columns fit one 96-wide tile), or from the half
+        transform's integers with one exponent per AO function (False,
+        default)."""
         self._check(lib().gbjk_set_split_fuse(self.h, 1 if on else 0), "gbjk_set_split_fuse")
 
     def get_split_fuse(self):
+        """Whether the last build cut them in the epilogue; before a build,
+        the setting."""
         return bool(lib().gbjk_get_split_fuse(self.h))
 
     def set_jmode(self, jmode):

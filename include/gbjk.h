@@ -180,6 +180,8 @@ int gbjk_get_overlap(const gbjk_ctx* ctx);
  * within the split path's accuracy bound; their results differ in the last
  * bits.  No counterpart in the reference. */
 gbjk_status gbjk_set_split_fuse(gbjk_ctx* ctx, int on);
+/* 1 if the last build's plan cuts them in the epilogue; before a build (or
+ * after a change of settings or data) the setting. */
 int gbjk_get_split_fuse(const gbjk_ctx* ctx);
 
 /* jmode: GBJK_J_VINV (default, the reference route) or GBJK_J_CHOLESKY.

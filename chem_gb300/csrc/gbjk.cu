@@ -1476,6 +1476,16 @@ gbjk_status gbjk_download_b(gbjk_ctx* ctx, double* B) {
   return GBJK_OK;
 }
 
+gbjk_status gbjk_download_fitted(gbjk_ctx* ctx, double* B) {
+  if (!ctx || !B) return fail(ctx, GBJK_INVALID_ARG, "gbjk_download_fitted");
+  if (!ctx->split.b_ready)
+    return fail(ctx, GBJK_NOT_READY, "gbjk_download_fitted: no mixed-precision build yet");
+  CK(cudaSetDevice(ctx->device));
+  CK(cudaStreamSynchronize(ctx->stream));
+  CK(cudaMemcpy(B, ctx->split.Bfit, (size_t)ctx->nnz * sizeof(double), cudaMemcpyDeviceToHost));
+  return GBJK_OK;
+}
+
 gbjk_status gbjk_test_split_stall(gbjk_ctx* ctx, int item, double wait_ms) {
   if (!ctx) return GBJK_INVALID_ARG;
   if (item >= 0 && !(wait_ms >= 1.0 && wait_ms <= 2000.0))

@@ -89,6 +89,7 @@ def lib():
         L.gbjk_set_occ_batch.argtypes = [vp, C.c_int]
         L.gbjk_upload_b_synthetic.argtypes = [vp, C.c_ulonglong, C.c_double]
         L.gbjk_download_b.argtypes = [vp, dp]
+        L.gbjk_download_fitted.argtypes = [vp, dp]
         ip = C.POINTER(C.c_int)
         L.gbjk_upload_b_eri3c.argtypes = [vp, C.POINTER(GbjkShells), C.POINTER(GbjkShells), dp,
                                           ip, C.c_int, ip, C.c_int, ip, ip,
@@ -262,6 +263,12 @@ class JKEngine:
     def download_b(self):
         B = np.empty(self.layout.nnz)
         self._check(lib().gbjk_download_b(self.h, _dp(B)), "gbjk_download_b")
+        return B
+
+    def download_fitted(self):
+        """L^-1 B as the mixed-path builds use it (after the first of them)."""
+        B = np.empty(self.layout.nnz)
+        self._check(lib().gbjk_download_fitted(self.h, _dp(B)), "gbjk_download_fitted")
         return B
 
     def set_tunables(self, **tun):

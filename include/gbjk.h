@@ -119,6 +119,9 @@ gbjk_status gbjk_set_aux_batch(gbjk_ctx* ctx, int rows);
  * No counterpart in the reference. */
 gbjk_status gbjk_upload_b_synthetic(gbjk_ctx* ctx, unsigned long long seed, double decay);
 gbjk_status gbjk_download_b(gbjk_ctx* ctx, double* B);
+/* The prefitted tensor L^-1 B that the mixed-precision builds use, in the same
+ * panels (GBJK_NOT_READY before the first of them). */
+gbjk_status gbjk_download_fitted(gbjk_ctx* ctx, double* B);
 
 /* Shells of a basis, normalised as the host engine uses them (the output of
  * gbints_basis_shells): per shell l, primitive count, first basis function,

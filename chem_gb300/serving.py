@@ -69,13 +69,18 @@ class Request:
 
 def footprint_bytes(layout, nocc, precision="split"):
     """Device bytes a J/K engine will hold for this molecule (estimate used
-    for admission; the engine's own gbjk_device_bytes is recorded after)."""
+    for admission; the engine's own gbjk_device_bytes is recorded after).  The
+    mixed path's set-up temporaries come before the buffers of a build and take
+    less where there is less memory, so they are not charged."""
     nnz, nbf, naux = layout.nnz, layout.nbf, layout.naux
     b = 8 * nnz + 2 * 8 * naux * naux           # B, L^-1, V^-1
     b += 8 * (nbf * nbf * 4 + nbf * naux)       # P, J, K, partials
     if precision == "split":
         b += 8 * nnz + 11 * nnz                 # L^-1 B (FP64) + digit slices (padded)
-        b += 6.1 * nnz                          # J's compact copy (6 B, rows padded)
+        # J's compact copy, 6 B: blocks on and above the diagonal, as the tensor
+        # is symmetric
+        diag = naux * int(sum(int(n) ** 2 for n in layout.bsizes))
+        b += 6.1 * 0.5 * (nnz + diag)
         b += 8 * nbf * naux * (nocc + 1)        # fitted half transform
         b += 11 * nbf * naux * (nocc + 1)       # its digits
         b += 8 * nbf * nbf * 64                 # split-K partials (upper bound)

@@ -398,7 +398,9 @@ gbjk_status gbjk_compute_j_noalloc(const gbjk_desc* desc, const int* d_colmap, c
                                    const double* d_Vinv, const double* d_Ptot, double* d_J,
                                    void* stream, char* errbuf, size_t errlen);
 
-/* Device memory held by the context, in bytes. */
+/* Device memory held by the context, in bytes (what a call allocates and frees
+ * again is not in it: the first mixed-precision build takes up to
+ * 16 naux^2 bytes and 1 GB so, less where there is less). */
 size_t gbjk_device_bytes(const gbjk_ctx* ctx);
 /* Kernels launched by this context since creation (for launch accounting). */
 int64_t gbjk_kernel_launches(const gbjk_ctx* ctx);

@@ -153,15 +153,31 @@ __global__ void __launch_bounds__(512)
                 int* __restrict__ e) {
   __shared__ int sm[4][128];
   const PfTile t = tiles[blockIdx.x];
-  const int c = t.c0 + threadIdx.x;
+  const int c = t.c0 + threadIdx.x, lane = threadIdx.x & 31;
   int mx = kPfNone;
-  if (c < t.ncol) {
-    const int m = c / t.K, k = c - m * t.K;
+  {
+    const int cc = min(c, t.ncol - 1);
+    const int m = cc / t.K, k = cc - m * t.K;
     const double* p = t.src + (long long)m * naux * t.K + k;
-#pragma unroll 8
-    for (int Y = threadIdx.y; Y < naux; Y += 4) {
-      const int E = (int)(__double_as_longlong(__ldg(p + (long long)Y * t.K)) >> 52) & 0x7FF;
-      if (E) mx = max(mx, E + b[Y] - 1022);
+    // Bound by the latency of its loads: sixteen high words on their way, then
+    // the balances of their Y, which the lanes brought and pass on (six waters 62
+    // us; 148 with a load each beside the element's and eight on their way).
+    for (int Y0 = threadIdx.y; Y0 < naux; Y0 += 64) {
+      const int Yl = min(Y0 + 4 * (lane & 15), naux - 1);
+      const int bl = __ldg(b + Yl);
+      unsigned int h[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int Y = Y0 + 4 * j;
+        h[j] = Y < naux ? __ldg(reinterpret_cast<const unsigned int*>(p + (long long)Y * t.K) + 1)
+                        : 0u;
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int E = (int)(h[j] >> 20) & 0x7FF;
+        const int eb = __shfl_sync(0xffffffffu, bl, j) + E - 1022;
+        mx = max(mx, E ? eb : kPfNone);
+      }
     }
   }
   sm[threadIdx.y][threadIdx.x] = mx;
@@ -216,7 +232,8 @@ __global__ void __launch_bounds__(256)
     if (X < naux)
       for (int Y = lane; Y <= X; Y += 32) {
         const int E = (int)(__double_as_longlong(L[(long long)X * naux + Y]) >> 52) & 0x7FF;
-        if (E) mx = max(mx, E - b[Y] - 1022);
+        const int eb = E - __ldg(b + Y) - 1022;
+        mx = max(mx, E ? eb : kPfNone);
       }
     mx = __reduce_max_sync(0xffffffffu, mx);
     if (lane == 0) {

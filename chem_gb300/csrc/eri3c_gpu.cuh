@@ -10,17 +10,17 @@
 //   for a primitive pair (a_i, b_j): Hermite coefficients E^{ab}_{tuv}
 //   (Helgaker, Jorgensen, Olsen eq. 9.5.6-9.5.7), for every auxiliary
 //   primitive c_k the Hermite Coulomb integrals R_{tuv}(alpha, P - C)
-//   (eq. 9.9.18-9.9.20, Boys function by its series and downward recursion,
-//   or erf and upward recursion for large arguments), contracted with the
-//   single-centre expansion of c and its spherical transform into
-//   W[tuv][mc], then with E^{ab} into the cartesian (a, b) accumulators,
-//   and finally transformed to spherical (a, b).
-// Work: one block per AO shell pair (a in block I, b in block J, a <= b
-// when I == J) of a kept block pair; its 4 warps take the auxiliary shells
-// of the kept auxiliary blocks in turn.  Lanes split the Hermite indices of
-// the bra (W) and the cartesian pairs (accumulators); the R table of a
-// primitive triple lives in the warp's shared memory.  Supported: AO shells
-// up to d and auxiliary shells up to f (la + lb + lc <= 7); the host checks.
+//   (eq. 9.9.18-9.9.20, Boys function from a table of Taylor expansions and
+//   downward recursion, or erf and upward recursion for large arguments),
+//   contracted with the single-centre expansion of c and its spherical
+//   transform into W[tuv][mc], then with E^{ab} folded with both spherical
+//   transforms into the results.
+// Work: a block takes an AO shell pair (a in block I, b in block J, a <= b
+// when I == J) of a kept block pair and a range of auxiliary blocks; its 4
+// warps take the kept auxiliary shells of the range in turn (k_eri3c).  The R
+// table of a primitive triple lives in the warp's shared memory.  Supported:
+// AO shells up to d and auxiliary shells up to f (la + lb + lc <= 7); the host
+// checks.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -35,7 +35,6 @@ constexpr int kEriMaxL = 2 * kEriMaxLao + kEriMaxLaux;                          
 constexpr int kEriNR = (kEriMaxL + 1) * (kEriMaxL + 2) * (kEriMaxL + 3) / 6;     // 120
 constexpr int kEriLb = 2 * kEriMaxLao;                                           // 4
 constexpr int kEriNW = (kEriLb + 1) * (kEriLb + 2) * (kEriLb + 3) / 6;           // 35
-constexpr int kEriNcab = 36;  // (d cartesians)^2
 constexpr int kEriMaxSph = 7;
 constexpr int kEriWarps = 4;
 // Boys values (-2 alpha)^n F_n(T), n <= L, of up to kEriRnChunk (bra

@@ -36,11 +36,18 @@ using namespace gbjk;
 
 // SMs the mixed-path exchange GEMM leaves to the concurrent J column sums
 // unless gbjk_set_overlap says otherwise: 0, the exchange takes every SM and
-// the J blocks fill the registers and shared memory its CTAs leave free (five
-// waters, a build through the host call: 155 us against 166 in order)
+// the J blocks fill the registers and shared memory its CTAs leave free
 constexpr int kDefaultOverlapSms = 0;
-// ... as long as J's tensor copy is smaller than this
+// ... as long as J's tensor copy is smaller than this.  Builds through the host
+// call, beside against in order, by the size of the copy: 27 MB (five waters)
+// 129 / 147 us, 56 MB 158 / 178, 125 MB 260 / 269, 227 MB (C10H22) 375 / 386,
+// 358 MB 581 / 579, 433 MB 681 / 674, 516 MB 808 / 790, 702 MB 1121 / 1120,
+// 1159 MB (C20H42) 1913 / 1889.
 constexpr size_t kOverlapJBytes = size_t(384) << 20;
+
+// Auxiliary functions of an engine at most: a metric of 5 GB.  (The FP64 J sums once
+// kept a vector of naux in shared memory; larger ones have never been run.)
+constexpr int kMaxNaux = 25600;
 
 enum Phase {
   PH_GATHER = 0,
@@ -311,8 +318,9 @@ void add_tiles(std::vector<GemmTile>& tiles, int group, int M, int N, int k0, in
 }
 
 // Occupied counts up to this many use 64 x 16 tiles in the FP64 half
-// transform and fit (a 64 x 64 tile would be mostly padding); a GEMM phase
-// with at most kElemOutputs outputs runs one thread per output instead.
+// transform and fit (a 64 x 64 tile would be mostly padding); where these have at
+// most kElemOutputs outputs they run on 16 x 16 tiles, one thread per output, as
+// the exchange does at every size.
 constexpr int kNarrowN = 16;
 constexpr long long kElemOutputs = 1 << 20;
 
@@ -1012,7 +1020,7 @@ gbjk_status gbjk_create(gbjk_ctx** out, const gbjk_desc* d) {
   *out = nullptr;
   if (d->nbf <= 0 || d->naux <= 0 || d->nblk <= 0 || !d->blk_size || !d->panel_K || !d->colmap)
     return GBJK_INVALID_ARG;
-  if ((size_t)d->naux * sizeof(double) > 200 * 1024) return GBJK_INVALID_ARG;
+  if (d->naux > kMaxNaux) return GBJK_INVALID_ARG;
   auto* ctx = new (std::nothrow) gbjk_ctx;
   if (!ctx) return GBJK_OOM;
   ctx->device = d->device;
@@ -1884,8 +1892,9 @@ struct SideFork {
 
 // Mixed-precision J + K.  The density rows of every panel ride along as
 // extra B-operand rows of the split half transform, whose epilogue emits
-// the partials of dt = L^-1 g; J = (L^-1 B)^T dt is one FP64 pass over the
-// prefitted tensor.  Without dJ the density rows are zero.
+// the partials of dt = L^-1 g; J = (L^-1 B)^T dt is one pass over the compact
+// copy of the prefitted tensor (6 bytes an element, the upper block triangle where
+// it is symmetric), in FP32 pairs.  Without dJ the density rows are zero.
 static gbjk_status run_jk_split(gbjk_ctx* ctx, const double* dP, const double* dC, int nocc,
                                 double* dJ, double* dK) {
   const int nbf = ctx->nbf, naux = ctx->naux;
@@ -1894,8 +1903,7 @@ static gbjk_status run_jk_split(gbjk_ctx* ctx, const double* dP, const double* d
   // overlap on (and no per-phase timing, whose events sit on one stream) it
   // runs on the side stream beside the exchange.  Where J alone fills the
   // GPU's memory bandwidth the two only delay each other, and the phases run in
-  // order (C20H42, 1.1 GB: 1.93 ms against 1.96 side by side; C10H22, 0.2 GB:
-  // 0.414 against 0.413; five waters, 0.03 GB: 166 us against 155).
+  // order (kOverlapJBytes).
   const bool fused = dJ && ctx->split.fused_j();
   const bool overlap = fused && !ctx->profile &&
                        (ctx->overlap_sms > 0 ||

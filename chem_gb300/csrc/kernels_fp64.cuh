@@ -602,12 +602,13 @@ __global__ void __launch_bounds__(TN * 4)
   }
 }
 
-// Small problems: 16 x 16 tiles, one thread per output, each output the
-// in-order fma chain over the tile's k range.  A lower-triangular A stops at
-// k = m: the terms beyond are exact zeros, so every nonzero result equals the
-// tiled kernel's bit for bit.  For problems so small that 64-row tiles would
-// be mostly padding and the few tiles would leave most SMs' FP64 units idle.
-// Bound by latency: 64 k of both operands are staged in shared memory at a
+// 16 x 16 tiles, one thread per output, each output the in-order fma chain over
+// the tile's k range.  A lower-triangular A stops at k = m: the terms beyond
+// are exact zeros, so every nonzero result equals the tiled kernel's bit for
+// bit.  For the exchange and the SCF's square products, whose tiles follow the
+// diagonal and the edge closest (FP64 pipe), and for half transforms and fits so
+// small that 64-row tiles would be mostly padding and the few tiles would leave
+// most SMs' FP64 units idle.  The latter are bound by latency: 64 k of both operands are staged in shared memory at a
 // time, the next 64 in registers meanwhile, so the chain waits for memory
 // once per tile and not once per eight k.  The threads take the outputs that
 // the matrix has, in row order: an FP64 instruction of a warp costs 16 clocks

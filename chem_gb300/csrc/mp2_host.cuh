@@ -11,12 +11,13 @@
 //   Z    Z_t[X][Y]    = sum_{i,a} W_t[X][i][a] W_t[Y][i][a]
 //   e_t  = sum_{X,Y} Z_t[X][Y]^2 = tr(Z V^-1 Z V^-1) of the unfitted Z
 // Each of T1, T2 and Z is one launch over all points (a grouped FP64 GEMM,
-// or the split-precision tensor-core GEMM of split_gemm.cuh); the energy is
-// an ordered FP64 reduction.  Split path per build:
-//   gather Lo rows per panel -> their digits -> T1 (A digits of Bfit are the
-//   J/K engine's) -> column exponents of H -> H digits (rows (X,i), k = n)
-//   and Lv digits -> T2 (epilogue: per-X exponent maxima of W) -> W digits
-//   -> Z upper tiles, split over k -> ordered reduce -> row sums -> e_t.
+// or the split-precision tensor-core GEMM of split_gemm.cuh); the energy is an
+// FP64 reduction, in order on the FP64 path.  Split path per build:
+//   digits of the rows of Lo (through each panel's columns) and of Lv -> T1 (A
+//   digits of Bfit are the J/K engine's; the points' columns share tiles) -> H
+//   exponents and digits (rows (X,i), k = n) -> T2 (integers, per-X exponent
+//   maxima of W) -> W digits -> Z upper tiles, split over k -> ordered reduce ->
+//   row sums -> e_t.
 #pragma once
 #include <algorithm>
 #include <string>

@@ -484,7 +484,7 @@ struct PrepJob {
 // then its warps share the k-tiles and find the values in L1.  Gathering the
 // columns, the exponents and the digits were four launches: 20 -> 9 us of a
 // C10H22 build, 33 -> 19 us of a C20H42 one.
-// grid (most 8-row groups of a job + 1, njobs), block 256.
+// grid (most 8-row groups of a job, njobs), block 256.
 __global__ void __launch_bounds__(256)
     k_prep_rows(const PrepJob* __restrict__ jobs, const double* __restrict__ b0,
                 const double* __restrict__ b1) {

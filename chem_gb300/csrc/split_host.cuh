@@ -6,10 +6,10 @@
 //   row exponents and slice images (the A operands of the half transform).
 // Per nocc: buffers and the two work lists (half transform, exchange).
 // Per build (stream-ordered, no host sync):
-//   C digits (B operand of every panel) -> split GEMM Hfit = Bfit C (FP64,
-//   row exponents by atomicMax) -> H digits -> split GEMM
-//   Kpart = Hfit Hfit^T (upper tiles, split-K) -> ordered reduce
-//   K = -sum Kpart.
+//   rows of C and P -> digits (B operand of every panel) -> split GEMM
+//   Hfit = Bfit C (the product's integers, row exponents by atomicMax) -> H
+//   digits -> split GEMM Kpart = Hfit Hfit^T (upper tiles, split-K) -> ordered
+//   reduce K = -sum Kpart.
 // With hfuse the half-transform epilogue cuts the digits of Hfit itself
 // (one exponent per AO function and group of 32 auxiliary indices) and the
 // exchange is the segmented variant that applies those exponents.
@@ -43,8 +43,8 @@ struct SplitState {
   bool bfit_owned = false;
   double* Bfit = nullptr;
   // compact copy of Bfit for the mixed-path J (k_encode_f32i16: FP32 hi and
-  // a 16-bit remainder per element, 6 bytes), unbatched only; with jsym the
-  // upper block triangle alone
+  // a 16-bit remainder per element, 6 bytes), unbatched only; of a symmetric
+  // tensor the upper block triangle alone (prepare_j)
   float* d_Bhi = nullptr;
   uint16_t* d_Blo = nullptr;
   JPanel* d_jp = nullptr;
@@ -64,8 +64,8 @@ struct SplitState {
   int apitch = 0;
   // fused digit cut of H in the half transform (requested; in effect for
   // the per-nocc buffers).  Off by default: on GB300 the fused half
-  // transform and segmented exchange together take longer than the FP64 H
-  // round trip and digit pass they replace.
+  // transform and segmented exchange together take longer than the H round
+  // trip and digit pass they replace.
   bool hfuse = false, hfuse_eff = false;  // asked for; what the current plan does
   // what the builds do, as far as a plan has decided it
   bool fuses() const { return hfuse && (nocc < 0 || hfuse_eff); }
@@ -95,7 +95,6 @@ struct SplitState {
   std::vector<SplitIntJob> hjobs;  // digits of H, one per distinct batch size
   long long* d_eoff = nullptr;     // their exponent offsets per AO function
   int c_groups = 0;  // most 8-row groups of a job
-  long long h_threads = 0;
   int* d_err = nullptr;
   int nsm = 148;
   bool profile = false;
@@ -805,7 +804,7 @@ struct SplitState {
     es_ld = apitch / 32;  // auxiliary groups of a full batch
     const long long hk = (long long)pad32(xb) * hld;
     // exchange k-tiles of a batch: fused, one per (auxiliary group, orbital);
-    // unfused, the FP64 H row of pad32(xbc) * hld values in 32-value tiles
+    // unfused, the H row of pad32(xbc) * hld values in 32-value tiles
     auto xk_nkt = [&](int xbc) {
       return fuse ? (pad32(xbc) / 32) * nocc_ : cdiv_((long long)pad32(xbc) * hld, kTileK);
     };

@@ -5,7 +5,7 @@
 // row's exponent e (|x| < 2^e), X = rint(|x| 2^(63-e)), in eight balanced
 // base-256 digits, exact in BF16 (the top one in [0, 128]).  Before that the
 // contracted index is balanced: column Y of L^-1 is divided, row Y of B
-// multiplied, by the power of two that makes their largest elements alike
+// multiplied, by a power of two that takes the column's largest element to 1
 // (k_pf_balance), so that the scale of an auxiliary function does not matter.  The product keeps
 // the 36 digit pairs (s, t) with s + t <= 7; all eight diagonals d = s + t are
 // summed exactly: a digit product is at most 2^14, so 128 k of at most eight
@@ -16,9 +16,9 @@
 // the operands' rounding at 2^-63 of their rows' largest elements and the
 // dropped pairs: for a result (X, c) about 2^-56 max_Y |L^-1[X][Y]| max_Y
 // |B[Y][c]| of the balanced operands.  An in-order FP64 sum loses 2^-53 of its
-// partial sums.  Over a tensor the first is the smaller by far, but a
-// single result whose terms are all far below that product of maxima is further
-// off here; those who read the result take sums over X or k, where it drowns.
+// partial sums.  Over a column c the first is the smaller by far, but a
+// single result whose terms are all far below the column's is further off here;
+// those who read the tensor take sums over X, where it drowns.
 //
 // This is the set-up cost of every new molecule: naux nnz(B) / 2 products, on
 // GB300's FP64 pipe (6e11 fma/s) 162 ms for C12H26 and 740 ms for C20H42.
@@ -47,7 +47,7 @@ constexpr int kPfBytesA = kPfDigits * kPfM * kPfK * 2, kPfBytesB = kPfDigits * k
 constexpr int kPfSmem = kPfStages * (kPfBytesA + kPfBytesB) + 1024;
 constexpr int kPfCols = kPfN / 3;  // output columns per epilogue thread
 // exponent of a row without a nonzero element; those of balanced rows reach
-// from -2044 to 2048
+// from -9213 to 2048
 constexpr int kPfNone = -1000000;
 
 // 128 tensor columns: c = c0 .. c0 + 127 of the panel's ncol = b_I K_I columns
@@ -95,40 +95,18 @@ __device__ __forceinline__ void store_digits8x8(const double (&x)[8], const int 
   }
 }
 
-// The largest exponent field of row Y of the tensor over all panels, into EB[Y]
-// (zeroed).  A warp takes one Y of sixteen AO functions.  Bound by HBM: one more
-// pass over the tensor (C12H26, 0.9 GB: 0.14 ms of the 20 of a new molecule).
-// grid (ceil(naux / 8), ceil(nbf / 16)), block 256.
-__global__ void __launch_bounds__(256)
-    k_pf_rowmax(const double* __restrict__ B, const long long* __restrict__ panel_off,
-                const int* __restrict__ blk_of, const int* __restrict__ boff,
-                const int* __restrict__ panel_K, int nbf, int naux,
-                unsigned int* __restrict__ EB) {
-  const int Y = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (Y >= naux) return;
-  unsigned int mx = 0;
-  const int mu1 = min(nbf, (int)(blockIdx.y + 1) * 16);
-  for (int mu = blockIdx.y * 16; mu < mu1; ++mu) {
-    const int I = blk_of[mu], K = panel_K[I];
-    const double* p = B + panel_off[I] + ((long long)(mu - boff[I]) * naux + Y) * K;
-#pragma unroll 4
-    for (int k = lane; k < K; k += 32)
-      mx = max(mx, (unsigned int)(__double_as_longlong(__ldg(p + k)) >> 52) & 0x7FF);
-  }
-  mx = __reduce_max_sync(0xffffffffu, mx);
-  if (lane == 0 && mx) atomicMax(EB + Y, mx);
-}
-
-// b[Y]: half the distance between the exponents of the largest element of column
-// Y of L^-1 and of row Y of the tensor, rounded down; a function taken 2^s times
-// as large lowers it by s, which leaves every digit as it is.  (On C4H10 and
-// C8H18 in their fitting basis the error bound above is 0.6 times that of
-// unbalanced operands, and twice it where L^-1 alone is balanced.)  Column maxima
-// of the lower triangle: a block walks 32 columns, 32 rows at a time.
+// b[Y]: the exponent of the largest element of column Y of L^-1; a function taken
+// 2^s times as large lowers it by s, which leaves every digit as it is.  No
+// element of the balanced L^-1 is above 1, and in every column some are: the
+// error of a result (X, c) is bounded by the largest product |L^-1[X'][Y] B[Y][c]|
+// of its column c, whatever the other columns' scales are.  (Balancing against
+// the tensor's rows too halves the error of fitting bases, but takes a pass
+// over the tensor, and the largest columns then spoil the others.)  A column of
+// zeros takes its row of the tensor out of the sums.  A block walks 32 columns of
+// the lower triangle, 32 rows at a time: 11 us for C12H26.
 // grid ceil(naux / 32), block (32, 32).
 __global__ void __launch_bounds__(1024)
-    k_pf_balance(const double* __restrict__ L, int naux, const unsigned int* __restrict__ EB,
-                 int* __restrict__ b) {
+    k_pf_balance(const double* __restrict__ L, int naux, int* __restrict__ b) {
   __shared__ unsigned int sm[32][33];
   const int Y = blockIdx.x * 32 + threadIdx.x;
   unsigned int mx = 0;
@@ -141,9 +119,7 @@ __global__ void __launch_bounds__(1024)
   __syncthreads();
   // warp y holds column 32 blockIdx.x + y
   mx = __reduce_max_sync(0xffffffffu, sm[threadIdx.y][threadIdx.x]);
-  const int Yw = blockIdx.x * 32 + threadIdx.y;
-  if (threadIdx.x == 0)
-    b[Yw] = Yw < naux && mx && EB[Yw] ? ((int)mx - (int)EB[Yw]) >> 1 : 0;
+  if (threadIdx.x == 0) b[blockIdx.x * 32 + threadIdx.y] = mx ? (int)mx - 1023 : -8192;
 }
 
 // Exponents of a tile's 128 tensor columns (max over Y); grid ntiles, block

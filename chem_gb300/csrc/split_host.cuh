@@ -386,7 +386,7 @@ struct SplitState {
     const size_t most = std::min(tiles.size(), std::max<size_t>(1, (size_t(1) << 30) / abytes));
     const size_t ny = (size_t)nkt_all * kPfK;
     PfTile* dt = nullptr;
-    // balance and largest exponents of Y, exponents of the X rows and of the tensor columns
+    // balance of Y, exponents of the X rows and of the tensor columns
     int* de = nullptr;
     void *own = nullptr, *db = nullptr;
     auto done = [&]() {
@@ -411,7 +411,7 @@ struct SplitState {
       return size_t(0);
     };
     bool ok = cudaMalloc((void**)&dt, tiles.size() * sizeof(PfTile)) == cudaSuccess &&
-              cudaMalloc((void**)&de, (2 * ny + (size_t)nxt * kPfN + most * kPfM) * sizeof(int)) ==
+              cudaMalloc((void**)&de, (ny + (size_t)nxt * kPfN + most * kPfM) * sizeof(int)) ==
                   cudaSuccess;
     size_t nx = 0, per = 0;  // X tiles and tensor tiles at a time
     if (ok) {
@@ -431,7 +431,7 @@ struct SplitState {
           w = (uint8_t*)own;
         }
       if (nx && per)
-        return prefit_parts(st, d_Linv, d_B, tiles, dt, de, bd, (int)nx, (uint16_t*)w, per,
+        return prefit_parts(st, d_Linv, tiles, dt, de, bd, (int)nx, (uint16_t*)w, per,
                             launches, err, done);
     }
     cudaGetLastError();
@@ -442,7 +442,7 @@ struct SplitState {
   // ... with digit buffers bd and ad for nx tiles of L^-1 and `per` tiles of the
   // tensor; done() frees what prefit() allocated
   template <class Done>
-  gbjk_status prefit_parts(cudaStream_t st, const double* d_Linv, const double* d_B,
+  gbjk_status prefit_parts(cudaStream_t st, const double* d_Linv,
                            const std::vector<PfTile>& tiles, PfTile* dt, int* de, uint16_t* bd,
                            int nx, uint16_t* ad, size_t per, int64_t* launches, std::string* err,
                            Done done) {
@@ -451,19 +451,16 @@ struct SplitState {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    int *bal = de, *eY = de + ny, *eb = de + 2 * ny, *ea = eb + (size_t)nxt * kPfN;
+    int *bal = de, *eb = de + ny, *ea = eb + (size_t)nxt * kPfN;
     cudaError_t e = cudaFuncSetAttribute(
         k_prefit_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmem);
     if (!e)
       e = cudaMemcpyAsync(dt, tiles.data(), tiles.size() * sizeof(PfTile), cudaMemcpyHostToDevice,
                           st);
-    if (!e) e = cudaMemsetAsync(eY, 0, ny * sizeof(int), st);
     if (!e) {
       Scope sc(this, 3, st);
-      k_pf_rowmax<<<dim3(cdiv_(naux, 8), cdiv_(nbf, 16)), 256, 0, st>>>(
-          d_B, dd_panel_off, dd_blk_of, dd_boff, dd_panelK, nbf, naux, (unsigned int*)eY);
-      k_pf_balance<<<nkt_all, dim3(32, 32), 0, st>>>(d_Linv, naux, (unsigned int*)eY, bal);
-      *launches += 2;
+      k_pf_balance<<<nkt_all, dim3(32, 32), 0, st>>>(d_Linv, naux, bal);
+      (*launches)++;
       for (int x0 = 0; x0 < nxt && !e; x0 += nx) {
         const int m = std::min(nx, nxt - x0), row0 = x0 * kPfN;
         e = cudaMemsetAsync(bd, 0, (size_t)m * bbytes, st);

@@ -42,6 +42,29 @@ def _exponent(a, axis):
     return np.frexp(np.abs(a).max(axis))[1]
 
 
+def _check(eng, lay, L, D, dense_to_panels):
+    """Every element of the engine's prefitted tensor against L D."""
+    naux, n = D.shape[0], D.shape[1]
+    with pytest.raises(RuntimeError):
+        eng.download_fitted()
+    eng.compute_jk(None, np.eye(n)[:, :2].copy())
+    F = eng.download_fitted()
+    eng.close()
+    Dm = D.reshape(naux, n * n)
+    hi, lo = _dd_product(L, Dm)
+    hi, lo = (dense_to_panels(lay, x.reshape(naux, n, n))[0] for x in (hi, lo))
+    # exponents of the operands with the columns of L taken to 1
+    ey = _exponent(L, 0)
+    Ls, Ds = np.ldexp(L, -ey[None]), np.ldexp(Dm, ey[:, None])
+    ed = _exponent(Ds, 0)
+    E = np.where(np.abs(Dm).max(0) > 0, _exponent(Ls, 1)[:, None] + ed, -1000)
+    # per term: 2 operands rounded at half a unit of 2^-63 and the 7 dropped digit
+    # pairs of 2^-64 (6 of 2^-72, ..); one rounding of the result
+    bound = naux * 9.1 * np.ldexp(1.0, E - 64)
+    bound = dense_to_panels(lay, bound.reshape(naux, n, n))[0] + 2.0 ** -53 * np.abs(hi)
+    assert (np.abs((F - hi) - lo) <= bound).all()
+
+
 @pytest.mark.parametrize("kind", ["plain", "cancelling", "scaled"])
 @pytest.mark.parametrize("naux", [1, 32, 33, 48, 49, 128, 129, 257])
 def test_prefit_elements(naux, kind, dense_to_panels):
@@ -63,21 +86,26 @@ def test_prefit_elements(naux, kind, dense_to_panels):
         T, L = T * s[:, None, None], L / s
     B, D = dense_to_panels(lay, T)
     eng = JKEngine(lay, B, L, L.T @ L, precision="split")
-    with pytest.raises(RuntimeError):
-        eng.download_fitted()
-    eng.compute_jk(None, np.eye(n)[:, :2].copy())
-    F = eng.download_fitted()
-    eng.close()
-    Dm = D.reshape(naux, n * n)
-    hi, lo = _dd_product(L, Dm)
-    hi, lo = (dense_to_panels(lay, x.reshape(naux, n, n))[0] for x in (hi, lo))
-    # exponents of the balanced operands
-    ey = _exponent(L, 0) - _exponent(Dm, 1)
-    Ls, Ds = np.ldexp(L, -(ey >> 1)[None]), np.ldexp(Dm, (ey >> 1)[:, None])
-    ed = _exponent(Ds, 0)
-    E = np.where(np.abs(Dm).max(0) > 0, _exponent(Ls, 1)[:, None] + ed, -1000)
-    # per term: 2 operands rounded at half a unit of 2^-63 and the 7 dropped digit
-    # pairs of 2^-64 (6 of 2^-72, ..); one rounding of the result
-    bound = naux * 9.1 * np.ldexp(1.0, E - 64)
-    bound = dense_to_panels(lay, bound.reshape(naux, n, n))[0] + 2.0 ** -53 * np.abs(hi)
-    assert (np.abs((F - hi) - lo) <= bound).all()
+    _check(eng, lay, L, D, dense_to_panels)
+
+
+@pytest.mark.parametrize("spread", [20, 60])
+@pytest.mark.parametrize("naux", [33, 130])
+def test_columns_keep_their_own_scale(naux, spread, dense_to_panels):
+    """AO and auxiliary functions scaled over many powers of two and integrals that
+    vanish for some of them: the bound holds in every column."""
+    rng = np.random.default_rng(naux + spread)
+    lay = build_layout([3, 9, 4], [naux], lambda i, j: np.array([True]))
+    n = lay.nbf
+    T = rng.standard_normal((naux, n, n))
+    T[rng.random((naux, n, n)) < 0.5] = 0.0
+    T = T + T.transpose(0, 2, 1)
+    T[:5, :4] = 0.0
+    T[:5, :, :4] = 0.0  # auxiliary functions without the first AO functions
+    T[7] = 0.0          # .. without any
+    a = 2.0 ** rng.integers(-spread, 1, n)
+    s = 2.0 ** rng.integers(-spread, spread + 1, naux)
+    L = np.tril(rng.standard_normal((naux, naux))) / s
+    B, D = dense_to_panels(lay, T * (s[:, None, None] * a[:, None] * a[None]))
+    eng = JKEngine(lay, B, L, L.T @ L, precision="split")
+    _check(eng, lay, L, D, dense_to_panels)

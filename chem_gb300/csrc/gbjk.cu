@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -48,6 +49,43 @@ constexpr size_t kOverlapJBytes = size_t(384) << 20;
 // Auxiliary functions of an engine at most: a metric of 5 GB.  (The FP64 J sums once
 // kept a vector of naux in shared memory; larger ones have never been run.)
 constexpr int kMaxNaux = 25600;
+
+// The engines' host copies of their error flags, one int each: a page-locked page
+// that stays for the process, its slots taken and given back under a lock.  (A
+// page-locked allocation per engine took 300 us of its life, as long as all else
+// of a small one.)  More engines than slots take pageable ints; those of a page
+// whose lock was lost (a device reset) are no more than that.
+class FlagPool {
+  static constexpr int kSlots = 1024;
+  std::mutex m_;
+  int* page_ = nullptr;
+  std::vector<int*> free_;
+
+ public:
+  int* take() {
+    std::lock_guard<std::mutex> l(m_);
+    if (!page_ && (page_ = (int*)std::aligned_alloc(4096, kSlots * sizeof(int)))) {
+      if (cudaHostRegister(page_, kSlots * sizeof(int), cudaHostRegisterPortable) != cudaSuccess)
+        cudaGetLastError();  // works pageable
+      for (int i = kSlots; i-- > 0;) free_.push_back(page_ + i);
+    }
+    if (free_.empty()) return (int*)std::malloc(sizeof(int));
+    int* p = free_.back();
+    free_.pop_back();
+    return p;
+  }
+  void give(int* p) {
+    std::lock_guard<std::mutex> l(m_);
+    if (page_ && p >= page_ && p < page_ + kSlots)
+      free_.push_back(p);
+    else
+      std::free(p);
+  }
+};
+FlagPool& flag_pool() {
+  static FlagPool* p = new FlagPool;  // never destroyed: engines may outlive statics
+  return *p;
+}
 
 enum Phase {
   PH_GATHER = 0,
@@ -97,7 +135,7 @@ struct gbjk_ctx {
   // co-resident; -1: no second stream, the phases in order).
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  int* h_err = nullptr;  // page-locked copy of the split path's error flag
+  int* h_err = nullptr;  // page-locked copy of the split path's error flag (flag_pool)
   int overlap_sms = kDefaultOverlapSms;
   // FP64 K of a pre-fitted tensor in auxiliary batches (gbjk_set_aux_batch):
   // per batch b the half transform of rows [b*xb, b*xb + xbc) (one group per
@@ -1075,10 +1113,13 @@ gbjk_status gbjk_create(gbjk_ctx** out, const gbjk_desc* d) {
   }
   if (cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess ||
-      cudaHostAlloc((void**)&ctx->h_err, sizeof(int), cudaHostAllocPortable) != cudaSuccess) {
+      cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming) != cudaSuccess) {
     gbjk_destroy(ctx);
     return GBJK_CUDA_ERROR;
+  }
+  if (!(ctx->h_err = flag_pool().take())) {
+    gbjk_destroy(ctx);
+    return GBJK_OOM;
   }
   gbjk_status s;
   auto up = [&](auto** dptr, const auto& vec) -> gbjk_status {
@@ -1136,7 +1177,7 @@ void gbjk_destroy(gbjk_ctx* ctx) {
   if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
   if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
-  if (ctx->h_err) cudaFreeHost(ctx->h_err);
+  if (ctx->h_err) flag_pool().give(ctx->h_err);
   delete ctx;
 }
 

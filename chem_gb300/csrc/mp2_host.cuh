@@ -63,8 +63,13 @@ struct Mp2State {
   long long *d_cofs = nullptr, *d_eoff = nullptr;
   std::vector<SplitIntJob> wjobs;
   int c_groups = 0, lv_groups = 0;
-  // page-locked: factors on their way in, then the energies on theirs out
+  // page-locked: factors on their way in, then the energies on theirs out.  From
+  // the second upload on (getting it and giving it back takes 300 us, as long as
+  // a small batch: not for one that is used once), kept over plans.
   double *h_stage = nullptr, *h_E = nullptr;
+  size_t stage_cap = 0;
+  int uploads = 0;
+  bool stage_zero = false;  // of this plan's padding
   // profiling
   bool profile = false;
   double ms[kNumPh] = {};
@@ -90,6 +95,10 @@ struct Mp2State {
     release_plan();
     free_(&d_Bfit64);
     bfit_bytes = bytes = 0;
+    if (h_stage) cudaFreeHost(h_stage);
+    h_stage = nullptr;
+    stage_cap = 0;
+    uploads = 0;
   }
   void release_plan() {
     free_(&d_Lo);
@@ -116,8 +125,8 @@ struct Mp2State {
     free_(&d_pjobs);
     free_(&d_cofs);
     free_(&d_eoff);
-    if (h_stage) cudaFreeHost(h_stage);
-    h_stage = h_E = nullptr;
+    h_E = nullptr;
+    stage_zero = false;
     resolve();
     bytes = bfit_bytes;
     npts = 0;
@@ -232,14 +241,6 @@ struct Mp2State {
       *err = "MP2 batch: out of device memory for the transforms";
       return GBJK_OOM;
     }
-    const size_t nst = (size_t)npts * nbf * (hld + vld) + npts;
-    if (cudaHostAlloc((void**)&h_stage, nst * 8, cudaHostAllocPortable) != cudaSuccess) {
-      cudaGetLastError();  // the copies go through pageable memory
-      h_stage = nullptr;
-    } else {
-      std::fill(h_stage, h_stage + nst, 0.0);  // the padding stays zero
-    }
-    h_E = h_stage ? h_stage + nst - npts : nullptr;
     precision = prec;
     gbjk_status s = prec == GBJK_SPLIT_BF16
                         ? plan_split(st, nbf, naux, nblk, bsize, boff, panelK, cmoff, sp, err)
@@ -600,12 +601,25 @@ struct Mp2State {
   // ordered on the stream after any evaluation still in flight.
   gbjk_status upload(cudaStream_t st, int nbf, const double* const* Lo, const double* const* Lv,
                      std::string* err) {
-    // Through page-locked memory kept with the plan, the copy of Lo under the
+    // Through page-locked memory where there is some, the copy of Lo under the
     // packing of Lv.  (A fresh buffer per call, zeroed and packed by rows, took 270
     // us for eight points of C8H18; this 100, and the wait for its copies.)
     const size_t nlo = (size_t)npts * nbf * hld, nlv = (size_t)npts * nbf * vld;
+    const size_t nst = nlo + nlv + npts;
+    if (uploads++ > 0 && stage_cap < nst) {
+      if (h_stage) cudaFreeHost(h_stage);
+      stage_cap = nst;
+      if (cudaHostAlloc((void**)&h_stage, nst * 8, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();  // the copies go through pageable memory
+        h_stage = nullptr;
+        stage_cap = 0;
+      }
+    }
+    double* lo = stage_cap >= nst ? h_stage : nullptr;
+    h_E = lo ? lo + nlo + nlv : nullptr;
+    if (lo && !stage_zero) std::fill(lo, lo + nst, 0.0);  // the padding stays zero
+    stage_zero = lo != nullptr;
     std::vector<double> pageable;
-    double* lo = h_stage;
     if (!lo) {
       pageable.assign(nlo + nlv, 0.0);
       lo = pageable.data();

@@ -385,13 +385,12 @@ struct SplitState {
     const size_t abytes = (size_t)nkt_all * kPfBytesA, bbytes = (size_t)nkt_all * kPfBytesB;
     const size_t most = std::min(tiles.size(), std::max<size_t>(1, (size_t(1) << 30) / abytes));
     const size_t ny = (size_t)nkt_all * kPfK;
-    PfTile* dt = nullptr;
-    // balance of Y, exponents of the X rows and of the tensor columns
+    // balance of Y, exponents of the X rows and of the tensor columns; the tiles
+    const size_t nint = (ny + (size_t)nxt * kPfN + most * kPfM + 63) & ~size_t(63);
     int* de = nullptr;
     void *own = nullptr, *db = nullptr;
     auto done = [&]() {
       cudaFree(own);
-      cudaFree(dt);
       cudaFree(db);
       cudaFree(de);
     };
@@ -410,9 +409,8 @@ struct SplitState {
       *p = nullptr;
       return size_t(0);
     };
-    bool ok = cudaMalloc((void**)&dt, tiles.size() * sizeof(PfTile)) == cudaSuccess &&
-              cudaMalloc((void**)&de, (ny + (size_t)nxt * kPfN + most * kPfM) * sizeof(int)) ==
-                  cudaSuccess;
+    const bool ok = cudaMalloc((void**)&de, nint * sizeof(int) + tiles.size() * sizeof(PfTile)) ==
+                    cudaSuccess;
     size_t nx = 0, per = 0;  // X tiles and tensor tiles at a time
     if (ok) {
       nx = grab(&db, bbytes, nxt, 0);
@@ -431,8 +429,8 @@ struct SplitState {
           w = (uint8_t*)own;
         }
       if (nx && per)
-        return prefit_parts(st, d_Linv, tiles, dt, de, bd, (int)nx, (uint16_t*)w, per,
-                            launches, err, done);
+        return prefit_parts(st, d_Linv, tiles, (PfTile*)(de + nint), de, bd, (int)nx,
+                            (uint16_t*)w, per, launches, err, done);
     }
     cudaGetLastError();
     done();
